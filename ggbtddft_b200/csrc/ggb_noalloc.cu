@@ -6,8 +6,8 @@
 // CUDA graph after its set-up, or a process that has reserved all device memory up front.  This
 // entry point computes the same per-(l, orbital) dipole and acceleration sums and per-orbital norm
 // that the time step records (dipoleMoment.cuh / dipoleAcceleration.cuh plus the norm), from
-// caller-provided device-accessible buffers only.  The partial sums over radius tiles, which the
-// context keeps in buffers it allocates, live here in a file-scope __device__ array of fixed size.
+// caller-provided device-accessible buffers only.  The norm's partial sums over l live in a file-scope
+// __device__ array of fixed size.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -17,86 +17,91 @@
 
 namespace ggb {
 
-// Capacity of the shared scratch: n_orb * N_l * ceil(N_r / 32) partial sums (each two double4,
-// 64 bytes: 4 MiB in all) and n_orb * ceil(N_r / 32) norm partials (dd, 16 bytes: 256 KiB).
+// Limits of a call: n_orb * N_l * ceil(N_r / 32) and n_orb * ceil(N_r / 32).
 constexpr int NA_MAX_PARTIALS = 65536;
 constexpr int NA_MAX_NORM = 16384;
 constexpr int NA_MAX_NL = 256;
 
-static __device__ __align__(256) double4 g_obs_scratch[2 * NA_MAX_PARTIALS];
-static __device__ __align__(256) double2 g_norm_scratch[NA_MAX_NORM];
+// Norm partials (dd), one per (orbital, l): n_orb * N_l <= NA_MAX_PARTIALS (1 MiB).
+static __device__ __align__(256) double2 g_norm_scratch[NA_MAX_PARTIALS];
 
-constexpr int NA_WARPS = 8;
+// One block per (l, orbital) row.  The rows l - 1, l and l + 1 of the orbital come straight from L2
+// (each is read three times: 25 MB of L2 traffic for nine orbitals on 600 radii, 97 l), a thread
+// sums its radii in double-double, and one reduction over the block ends the row: no partial sums
+// per tile of radii, no second pass over them, and one reduction per row where the tile form
+// (a warp reduction of every row for every 32 radii) made ceil(N_r / 32).  128 threads: a row of
+// 600 radii is five loads per thread, all rows of a call are resident at once.  Bound by the latency
+// of one load, the five sums and the reduction; N_r 600, N_l 97, nine orbitals: 12.3 us a
+// call with the norm kernel, 44.7 us as tiles and a reduction kernel.
+constexpr int NA_THREADS = 128;
 
-// One CTA per (orbital, 32-radius tile): the tile of every l in shared memory, then the same
-// per-l dipole/acceleration partials as the time step (observables_tile) and a compensated norm
-// partial.
-__global__ void __launch_bounds__(NA_WARPS * 32)
-k_obs_partials(const double2* __restrict__ x, const double* __restrict__ r, const double* __restrict__ coef,
-               const int* __restrict__ m_of, int n_l, int n_orb, int n_r, int n_tiles, double4* __restrict__ obs,
-               double2* __restrict__ norm_part) {
-  extern __shared__ double2 xs[];  // [N_l][32]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = blockIdx.x / n_tiles, tile = blockIdx.x - k * n_tiles;
-  const int rr_i = tile * TR + lane;
-  const bool rv = rr_i < n_r;
-  for (int l = warp; l < n_l; l += NA_WARPS)
-    xs[l * TR + lane] = rv ? x[((size_t)l * n_orb + k) * n_r + rr_i] : make_double2(0.0, 0.0);
-  __syncthreads();
-  GroupArgs g{};
-  g.n_l = n_l;
-  g.n_m = NA_MAX_NL;      // the coefficient rows are laid out for m = 0 .. NA_MAX_NL-1
-  g.n_tiles = n_tiles;
-  g.obs_seg = TR;
-  g.coef = coef;
-  g.obs = obs;
+__global__ void __launch_bounds__(NA_THREADS)
+k_obs_rows(const double2* __restrict__ x, const double* __restrict__ r, const double* __restrict__ coef,
+           const int* __restrict__ m_of, int n_l, int n_orb, int n_r, double2* __restrict__ dip,
+           double2* __restrict__ acc, double2* __restrict__ norm_part) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int l = blockIdx.x / n_orb, k = blockIdx.x - l * n_orb;
   int m = m_of[k];
   if (m < 0 || m > n_l) m = n_l;   // an invalid m contributes nothing (no l satisfies l >= m)
-  const double rr = rv ? r[rr_i] : 1.0;
-  const double fr2 = rv ? pow(rr, -2.0) : 0.0;
-  // the coefficient rows of this m, NA_MAX_NL long whatever the call's N_l
-  const int mr = m < NA_MAX_NL ? m : NA_MAX_NL - 1;
-  const double* cu_row = coef + ((size_t)CF_CU * NA_MAX_NL + mr) * NA_MAX_NL;
-  const double* cd_row = coef + ((size_t)CF_CD * NA_MAX_NL + mr) * NA_MAX_NL;
-  observables_tile(g, xs, k, m, tile * TR, lane, warp, NA_WARPS, rr, fr2, TR, cu_row, cd_row);
-  if (warp == 0) {
-    dd s{0.0, 0.0};
-    for (int l = m; l < n_l; ++l) {
-      const double2 v = xs[l * TR + lane];
-      s = dd_add(s, dd{v.x * v.x + v.y * v.y, 0.0});
-    }
+  // dipole (re, im), acceleration (re, im), norm
+  dd s[5];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = dd_add(s, dd{__shfl_xor_sync(0xffffffffu, s.hi, o),
-                                                       __shfl_xor_sync(0xffffffffu, s.lo, o)});
-    if (lane == 0) norm_part[(size_t)k * n_tiles + tile] = make_double2(s.hi, s.lo);
+  for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
+  if (l >= m) {   // here m < NA_MAX_NL
+    // the first row has no lower, the last no upper neighbour (dipoleMoment.cuh:19-43)
+    const bool up = l + 1 < n_l, down = l > m;
+    const double c_u = (l == m || l != n_l - 1) ? coef[((size_t)CF_CU * NA_MAX_NL + m) * NA_MAX_NL + l] : 0.0;
+    const double c_d = down ? coef[((size_t)CF_CD * NA_MAX_NL + m) * NA_MAX_NL + l] : 0.0;
+    const size_t ls = (size_t)n_orb * n_r;
+    const double2* row = x + (size_t)l * ls + (size_t)k * n_r;
+    for (int i = threadIdx.x; i < n_r; i += NA_THREADS) {
+      const double2 xl = row[i];
+      const double2 xu = up ? row[ls + i] : make_double2(0.0, 0.0);
+      const double2 xd = down ? (row - ls)[i] : make_double2(0.0, 0.0);
+      const double rr = r[i], fr2 = 1.0 / (rr * rr);
+      const double zx = c_u * xu.x + c_d * xd.x, zy = c_u * xu.y + c_d * xd.y;
+      // conj(x_l) . z
+      const double px = xl.x * zx + xl.y * zy, py = xl.x * zy - xl.y * zx;
+      s[0] = dd_add(s[0], dd{rr * px, 0.0});
+      s[1] = dd_add(s[1], dd{rr * py, 0.0});
+      s[2] = dd_add(s[2], dd{fr2 * px, 0.0});
+      s[3] = dd_add(s[3], dd{fr2 * py, 0.0});
+      s[4] = dd_add(s[4], dd{xl.x * xl.x + xl.y * xl.y, 0.0});
+    }
+  }
+  __shared__ dd part[NA_THREADS / 32][5];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+      s[q] = dd_add(s[q], dd{__shfl_xor_sync(0xffffffffu, s[q].hi, o), __shfl_xor_sync(0xffffffffu, s[q].lo, o)});
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < 5; ++q) part[threadIdx.x >> 5][q] = s[q];
+  __syncthreads();
+  if (threadIdx.x < 5) {
+    dd t = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < NA_THREADS / 32; ++w) t = dd_add(t, part[w][threadIdx.x]);
+    const size_t o = (size_t)l * n_orb + k;
+    if (threadIdx.x < 2) reinterpret_cast<double*>(dip + o)[threadIdx.x] = t.hi + t.lo;
+    else if (threadIdx.x < 4) reinterpret_cast<double*>(acc + o)[threadIdx.x - 2] = t.hi + t.lo;
+    else norm_part[(size_t)k * n_l + l] = make_double2(t.hi, t.lo);
   }
 }
 
-// One thread per (l, orbital) sums the tiles; one thread per orbital sums the norm partials.
-__global__ void k_obs_reduce(const double4* __restrict__ obs, const double2* __restrict__ norm_part, int n_l,
-                             int n_orb, int n_tiles, double2* __restrict__ dip, double2* __restrict__ acc,
-                             double* __restrict__ norm) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n_l * n_orb) {
-    const int l = i / n_orb, k = i - l * n_orb;
-    const double4* p = obs + 2 * (((size_t)k * n_l + l) * n_tiles);
-    dd sx{0.0, 0.0}, sy{0.0, 0.0}, sz{0.0, 0.0}, sw{0.0, 0.0};
-    for (int t = 0; t < n_tiles; ++t) {
-      const double4 h = p[2 * t], lo = p[2 * t + 1];
-      sx = dd_add(sx, dd{h.x, lo.x}); sy = dd_add(sy, dd{h.y, lo.y});
-      sz = dd_add(sz, dd{h.z, lo.z}); sw = dd_add(sw, dd{h.w, lo.w});
-    }
-    dip[(size_t)l * n_orb + k] = make_double2(sx.hi + sx.lo, sy.hi + sy.lo);
-    acc[(size_t)l * n_orb + k] = make_double2(sz.hi + sz.lo, sw.hi + sw.lo);
-  }
-  if (i < n_orb) {
-    dd s{0.0, 0.0};
-    for (int t = 0; t < n_tiles; ++t) {
-      const double2 v = norm_part[(size_t)i * n_tiles + t];
-      s = dd_add(s, dd{v.x, v.y});
-    }
-    norm[i] = s.hi + s.lo;
-  }
+// One warp per orbital sums the norm partials of its l.  Launched as a programmatic dependent of
+// k_obs_rows: its launch overlaps that kernel, it reads after the wait.
+__global__ void __launch_bounds__(32)
+k_obs_norm(const double2* norm_part, int n_l, double* __restrict__ norm) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const double2* p = norm_part + (size_t)blockIdx.x * n_l;
+  dd s{0.0, 0.0};
+  for (int l = threadIdx.x; l < n_l; l += 32) s = dd_add(s, dd{p[l].x, p[l].y});
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    s = dd_add(s, dd{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
+  if (threadIdx.x == 0) norm[blockIdx.x] = s.hi + s.lo;
 }
 
 // Angular coefficient rows c_u, c_d (l, m < NA_MAX_NL) of the observables, [coef][m][l] with rows
@@ -120,7 +125,6 @@ __global__ void k_fill_coef(double* coef) {
 // Per-device addresses of the file-scope arrays, resolved on a device's first call.
 struct NoallocDevice {
   bool ready = false;
-  double4* obs = nullptr;
   double2* norm = nullptr;
   double* coef = nullptr;
 };
@@ -133,12 +137,8 @@ static int noalloc_setup(int dev) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
   NoallocDevice& d = g_dev[dev];
   if (d.ready) return GGB_OK;
-  if (cudaGetSymbolAddress((void**)&d.obs, g_obs_scratch) != cudaSuccess) return GGB_ERR_CUDA;
   if (cudaGetSymbolAddress((void**)&d.norm, g_norm_scratch) != cudaSuccess) return GGB_ERR_CUDA;
   if (cudaGetSymbolAddress((void**)&d.coef, g_coef) != cudaSuccess) return GGB_ERR_CUDA;
-  if (cudaFuncSetAttribute(k_obs_partials, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           NA_MAX_NL * TR * (int)sizeof(double2)) != cudaSuccess)
-    return GGB_ERR_CUDA;
   k_fill_coef<<<(NA_MAX_NL * NA_MAX_NL + 255) / 256, 256>>>(d.coef);
   if (cudaStreamSynchronize(0) != cudaSuccess) return GGB_ERR_CUDA;
   d.ready = true;
@@ -161,10 +161,17 @@ extern "C" int ggb_observables_noalloc(const double* x, const double* r, const i
   if (rc) return rc;
   const NoallocDevice& d = g_dev[dev];
   cudaStream_t s = (cudaStream_t)stream;
-  k_obs_partials<<<n_orb * n_tiles, NA_WARPS * 32, (size_t)n_l * TR * sizeof(double2), s>>>(
-      reinterpret_cast<const double2*>(x), r, d.coef, m, n_l, n_orb, n_r, n_tiles, d.obs, d.norm);
-  const int nt = n_l * n_orb > n_orb ? n_l * n_orb : n_orb;
-  k_obs_reduce<<<(nt + 127) / 128, 128, 0, s>>>(d.obs, d.norm, n_l, n_orb, n_tiles, reinterpret_cast<double2*>(dip),
-                                                 reinterpret_cast<double2*>(acc), norm);
+  k_obs_rows<<<n_l * n_orb, NA_THREADS, 0, s>>>(reinterpret_cast<const double2*>(x), r, d.coef, m, n_l, n_orb, n_r,
+                                                 reinterpret_cast<double2*>(dip), reinterpret_cast<double2*>(acc), d.norm);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute after{};
+  after.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  after.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(n_orb);
+  cfg.blockDim = dim3(32);
+  cfg.stream = s;
+  cfg.attrs = &after;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_obs_norm, (const double2*)d.norm, n_l, norm);
   return cudaGetLastError() == cudaSuccess ? GGB_OK : GGB_ERR_CUDA;
 }

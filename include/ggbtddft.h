@@ -197,8 +197,9 @@ void ggb_destroy(ggb_ctx* ctx);
    device-accessible (device memory or mapped host memory); nothing is copied, and no cudaMalloc,
    cudaFree or allocating library routine is called.
    Limits: N_l <= 256, N_kso * N_l * ceil(N_r / 32) <= 65536 and N_kso * ceil(N_r / 32) <= 16384;
-   larger sizes return GGB_ERR_ARG.  The partial sums live in fixed arrays inside the library
-   (5.25 MiB, held on every device that loads the library until the process exits) that all calls
+   larger sizes return GGB_ERR_ARG.  The norm's partial sums live in a fixed array inside the library
+   (1 MiB, and 1 MiB of coefficients, held on every device that loads the library until the process
+   exits) that all calls
    share: calls that overlap on the GPU (other streams or threads) race, so serialise them.  Each
    call writes every partial it reads, so nothing has to start at zero.  The first call on a device
    looks up the arrays' device addresses (cudaGetSymbolAddress) with that device current and fills
