@@ -11,12 +11,12 @@
 //                  (hartreePotentialDensity.cuh:1-181, dipoleMoment.cuh:1-75,
 //                  dipoleAcceleration.cuh:1-71), so the orbitals are read once per half-step.
 //  k_radial_fp64   x_l <- A_l x_l for every l with A_l(a,b) = W[l][b][a]: the batched ZGEMM of
-//                  h_propagationH0 (h_timePropagation.cuh:1-30), out of place.  Persistent, two CTAs
-//                  per SM; a producer warp streams the W rows and x segments of each 16-wide k chunk
-//                  into a 3-stage shared-memory ring with cp.async.bulk (mbarrier transaction
-//                  counts), so that ~200 KB per SM are in flight whatever the occupancy; four
-//                  consumer warps (one output radius per thread, TC orbital columns in registers)
-//                  run the FP64 FMAs from shared memory.
+//                  h_propagationH0 (h_timePropagation.cuh:1-30), out of place.  More than nine
+//                  columns: persistent, two CTAs per SM; a producer warp streams the W rows and x
+//                  segments of each 16-wide k chunk into a 3-stage shared-memory ring with
+//                  cp.async.bulk (mbarrier transaction counts), so that ~200 KB per SM are in flight
+//                  whatever the occupancy; four consumer warps run the product on the FP64 tensor
+//                  cores.  Up to nine columns (one run): k_radial_fp64_rows.
 //  k_finalize      per run: observables of the step from the partials, density multipoles
 //                  (occupation-weighted sum over orbitals), Hartree potentials by compensated
 //                  prefix scans (h_calculateHartreePotential.cuh:1-136), LDA exchange
@@ -438,26 +438,200 @@ static constexpr size_t radial_fp64_smem() {
   return (size_t)RAD_STAGES * (RAD_KC * RAD_TI + TC * RAD_KC) * sizeof(double2);
 }
 
+// Few orbital columns (up to RF_MAX_COLS): one block per (l, 32 output radii), k split over the block's
+// warps.  A warp streams its k slice of W straight into registers (per k step of 4: four loads, each
+// 4 k x 8 radii = four 128-byte segments, RF_D steps ahead of the products), the x values of RF_KC k at
+// a time come by cp.async into a double buffer of its own, so that no warp waits for another before
+// the slices' sums are added, in slice order, at the end.  Groups of four columns run on the FP64
+// tensor pipe as in the tile form above; the columns left over (one of nine) as plain FMAs on the same
+// fragments, each lane over its own k: an 8-column MMA tile would pad nine columns (18 real) to 24,
+// and the two units share one peak.  The many small blocks keep every SM supplied to the end, where
+// tiles of 128 radii leave the last wave a third full (485 tiles on 296 resident blocks).
+// Bound by HBM (W, 16 N_r^2 N_l bytes) and, at nine columns, as much by the FP64 pipe.  Tile form ->
+// this form: N_r 200, N_l 33, one column 16.9 -> 8.5 us; 400/65/1 35.5 -> 29.0 us (5.7 TB/s of W);
+// 253/49/3 22.8 -> 11.5 us; 600/97/9 164 -> 131 us (4.3 TB/s of W, 19 TFLOP/s).
+constexpr int RF_MAX_COLS = 9;
+constexpr int RF_KC = 16;                 // k per x chunk
+constexpr int RF_LDX = RF_KC + 4;         // row of a chunk: four columns' four k fall on 256 different bytes
+
+__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+
+// The first RF_KEEP bytes of W stay in L2 from step to step (normal priority), the rest streams
+// through it (evict first), so that W does not push itself out of L2 before it comes round again.
+// The helium step (166 MB of W) takes 156.9 us with none kept, 154.6 with 48 MB, 166.5 with 96 MB.
+constexpr size_t RF_KEEP = 48u << 20;
+
+template <int TC, int RF_WARPS, bool KEEP>
+__device__ __forceinline__ void radial_rows_block(int n_r, const double2* __restrict__ W,
+                                                  const double2* __restrict__ xin, double2* __restrict__ xout,
+                                                  double2* sm) {
+  // MMA tiles of four columns and FMA columns (three left over: one padded tile, for its registers)
+  constexpr int NT = (TC + 1) / 4, NF = TC > 4 * NT ? TC - 4 * NT : 0;
+  // k steps of W in flight: four where the registers allow it (three columns: 14.5 -> 11.5 us)
+  constexpr int RF_D = TC == 3 || TC == 4 ? 4 : 2;
+  constexpr int XC = 4 * NT > TC ? 4 * NT : TC;     // columns of the x buffers (a padded tile's last: unused)
+  constexpr int XW = 2 * XC * RF_LDX;               // x buffers of a warp
+  constexpr int PL = TC | 1, PW = PL * 32;          // partial sums of a warp, [32 radii][PL]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gid = lane >> 2, q = lane & 3;
+  const int n_it = (n_r + 31) / 32;
+  const int l = blockIdx.x / n_it, i0 = (blockIdx.x - l * n_it) * 32;
+  const int ks = (n_r + 4 * RF_WARPS - 1) / (4 * RF_WARPS) * 4;
+  const int k0 = min(n_r, warp * ks), k1 = min(n_r, k0 + ks);
+  double2* xs = sm + warp * XW;
+  const double2* Xl = xin + (size_t)l * TC * n_r;
+  auto load_x = [&](int kc, int buf) {
+    for (int e = lane; e < TC * RF_KC; e += 32) {
+      const int c = e / RF_KC, kk = e - c * RF_KC, k = kc + kk;
+      const bool v = k < k1;
+      cp_async16_zfill(xs + buf * XC * RF_LDX + c * RF_LDX + kk, Xl + (size_t)c * n_r + (v ? k : 0), v);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // W[l][k + q][i0 + 8 mt + gid] of the next k step, zero past the slice and past the last radius
+  const double2* wp = W + ((size_t)l * n_r + k0 + q) * n_r + i0 + gid;
+  const size_t wstep = 4 * (size_t)n_r;
+  int kw = k0 + q;
+  const int rows_left = n_r - i0 - gid;
+  auto load_w = [&](double2 (&w)[4]) {
+    const bool kv = kw < k1;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      w[mt] = make_double2(0.0, 0.0);
+      if (kv && 8 * mt < rows_left) w[mt] = KEEP ? __ldg(wp + 8 * mt) : __ldcs(wp + 8 * mt);
+    }
+    wp += wstep;
+    kw += 4;
+  };
+  double acc[4][NT > 0 ? NT : 1][2];
+  double2 accf[4][NF > 0 ? NF : 1];
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) accf[mt][f] = make_double2(0.0, 0.0);
+  }
+  double2 w[RF_D][4];
+#pragma unroll
+  for (int d = 0; d < RF_D; ++d) load_w(w[d]);
+  load_x(k0, 0);
+  int buf = 0;
+#pragma unroll 1
+  for (int kc = k0; kc < k1; kc += RF_KC, buf ^= 1) {
+    load_x(kc + RF_KC, buf ^ 1);          // past the slice: zeros, never read
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const double2* xb = xs + buf * XC * RF_LDX + q;
+#pragma unroll
+    for (int st = 0; st < RF_KC / 4; ++st) {
+      double2 (&ww)[4] = w[st % RF_D];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int c = 4 * nt + (gid >> 1);
+        const double2 x = (4 * NT <= TC || c < TC) ? xb[c * RF_LDX + 4 * st] : make_double2(0.0, 0.0);
+        const double bp = (gid & 1) ? x.y : x.x, bq = (gid & 1) ? x.x : -x.y;
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) mma_f64_8x8x4(acc[mt][nt][0], acc[mt][nt][1], ww[mt].x, bp);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) mma_f64_8x8x4(acc[mt][nt][0], acc[mt][nt][1], ww[mt].y, bq);
+      }
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const double2 x = xb[(4 * NT + f) * RF_LDX + 4 * st];
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) {
+          accf[mt][f].x = fma(ww[mt].x, x.x, accf[mt][f].x);
+          accf[mt][f].y = fma(ww[mt].x, x.y, accf[mt][f].y);
+          accf[mt][f].x = fma(-ww[mt].y, x.y, accf[mt][f].x);
+          accf[mt][f].y = fma(ww[mt].y, x.x, accf[mt][f].y);
+        }
+      }
+      load_w(ww);
+    }
+    __syncwarp();                         // the buffer is refilled in the next round
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                        // every warp is done with its x buffers
+  double2* part = sm + warp * PW;
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+      if (4 * NT <= TC || 4 * nt + q < TC) part[(8 * mt + gid) * PL + 4 * nt + q] = make_double2(acc[mt][nt][0], acc[mt][nt][1]);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      double2 v = accf[mt][f];
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+      }
+      if (q == mt) part[(8 * mt + gid) * PL + 4 * NT + f] = v;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < TC * 32; e += RF_WARPS * 32) {
+    const int c = e >> 5, rl = e & 31, r = i0 + rl;
+    double2 s = sm[rl * PL + c];
+#pragma unroll
+    for (int p = 1; p < RF_WARPS; ++p) {
+      const double2 v = sm[p * PW + rl * PL + c];
+      s.x += v.x;
+      s.y += v.y;
+    }
+    if (r < n_r) xout[((size_t)l * TC + c) * n_r + r] = s;
+  }
+}
+
+template <int TC>
+constexpr int rf_smem(int warps) {    // double2: x buffers or partial sums
+  constexpr int xc = (TC + 1) / 4 * 4 > TC ? (TC + 1) / 4 * 4 : TC;
+  return warps * (2 * xc * RF_LDX > (TC | 1) * 32 ? 2 * xc * RF_LDX : (TC | 1) * 32);
+}
+
+template <int TC, int RF_WARPS>
+__global__ void __launch_bounds__(RF_WARPS * 32, (TC == 1 ? 24 : 16) / RF_WARPS)
+k_radial_fp64_rows(int n_r, int l_keep, const double2* __restrict__ W, const double2* __restrict__ xin,
+                   double2* __restrict__ xout) {
+  __shared__ __align__(16) double2 sm[rf_smem<TC>(RF_WARPS)];
+  if ((int)blockIdx.x / ((n_r + 31) / 32) < l_keep) radial_rows_block<TC, RF_WARPS, true>(n_r, W, xin, xout, sm);
+  else radial_rows_block<TC, RF_WARPS, false>(n_r, W, xin, xout, sm);
+}
+
 static int g_radial_sms = 0;
 
 void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin, double2* xout, cudaStream_t s) {
   const int nc = g.n_cols;
-  int tc = nc >= 16 ? 16 : nc;
-  static const int opts[] = {1, 2, 3, 4, 6, 8, 9, 12, 16};
-  for (int o : opts)
-    if (o >= tc) { tc = o; break; }
+  if (nc <= RF_MAX_COLS) {
+    const int blocks = g.n_l * ((g.n_r + 31) / 32);
+    const int l_keep = (int)(RF_KEEP / (sizeof(double2) * g.n_r * g.n_r));
+    // eight warps a block until four blocks an SM are there, then four (fewer k slices to start and
+    // to add: 138 -> 133 us at 600/97/9; below, the smaller blocks leave the SMs emptier)
+    const bool wide = blocks < 4 * g_radial_sms;
+#define GGB_RF_CASE(C)                                                                       \
+  case C:                                                                                    \
+    if (wide) k_radial_fp64_rows<C, 8><<<blocks, 256, 0, s>>>(g.n_r, l_keep, W, xin, xout);  \
+    else k_radial_fp64_rows<C, 4><<<blocks, 128, 0, s>>>(g.n_r, l_keep, W, xin, xout);       \
+    break;
+    switch (nc) {
+      GGB_RF_CASE(1) GGB_RF_CASE(2) GGB_RF_CASE(3) GGB_RF_CASE(4) GGB_RF_CASE(5)
+      GGB_RF_CASE(6) GGB_RF_CASE(7) GGB_RF_CASE(8) GGB_RF_CASE(9)
+      default: break;
+    }
+#undef GGB_RF_CASE
+    return;
+  }
+  const int tc = nc <= 12 ? 12 : 16;
   const int tiles = ((g.n_r + RAD_TI - 1) / RAD_TI) * ((nc + tc - 1) / tc) * g.n_l;
   const int ctas = std::min(tiles, 2 * g_radial_sms);
-#define GGB_RAD_CASE(C)                                                                                     \
-  case C:                                                                                                   \
-    k_radial_fp64<C><<<ctas, RAD_THREADS, radial_fp64_smem<C>(), s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status); \
-    break;
-  switch (tc) {
-    GGB_RAD_CASE(1) GGB_RAD_CASE(2) GGB_RAD_CASE(3) GGB_RAD_CASE(4) GGB_RAD_CASE(6)
-    GGB_RAD_CASE(8) GGB_RAD_CASE(9) GGB_RAD_CASE(12) GGB_RAD_CASE(16)
-    default: break;
-  }
-#undef GGB_RAD_CASE
+  if (tc == 12)
+    k_radial_fp64<12><<<ctas, RAD_THREADS, radial_fp64_smem<12>(), s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status);
+  else
+    k_radial_fp64<16><<<ctas, RAD_THREADS, radial_fp64_smem<16>(), s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status);
 }
 
 static cudaError_t configure_radial_fp64() {
@@ -466,14 +640,11 @@ static cudaError_t configure_radial_fp64() {
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&g_radial_sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-#define GGB_RAD_ATTR(C)                                                                                   \
-  e = cudaFuncSetAttribute((const void*)k_radial_fp64<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                           (int)radial_fp64_smem<C>());                                                   \
+  e = cudaFuncSetAttribute((const void*)k_radial_fp64<12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)radial_fp64_smem<12>());
   if (e != cudaSuccess) return e;
-  GGB_RAD_ATTR(1) GGB_RAD_ATTR(2) GGB_RAD_ATTR(3) GGB_RAD_ATTR(4) GGB_RAD_ATTR(6)
-  GGB_RAD_ATTR(8) GGB_RAD_ATTR(9) GGB_RAD_ATTR(12) GGB_RAD_ATTR(16)
-#undef GGB_RAD_ATTR
-  return cudaSuccess;
+  return cudaFuncSetAttribute((const void*)k_radial_fp64<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)radial_fp64_smem<16>());
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,0 +1,70 @@
+"""The FP64 kernels at the edges of their tiles, against NumPy in FP64.
+
+Tolerances: a sum of n products in FP64 is off by at most n eps of the sum of the terms' magnitudes;
+the vectors are normalised, so 1e-12 covers n <= 1000 with the angular chain's V V^T on both sides.
+"""
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+
+from ggbtddft_b200 import problems as P
+from ggbtddft_b200.engine import TimePropagation, load_library
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+@pytest.mark.parametrize("n_r,cols", [(5, 1), (31, 2), (32, 3), (33, 4), (37, 5), (64, 6), (65, 7), (100, 8), (129, 9),
+                                      (70, 10), (33, 13), (45, 17)])
+def test_fp64_radial_product_at_every_column_count(n_r, cols):
+    """E = 0 and no Hartree: one step is x <- A x.  Column counts on both sides of the row form's limit,
+    radii at the edges of its 32-radius blocks, k slices and 16-wide chunks (down to empty slices)."""
+    base = P.reference_like(n_r, 6, 2, "H", r_mask=10.0).with_field(np.zeros(2))
+    rng = np.random.default_rng(cols)
+    runs = []
+    for _ in range(cols):
+        x = rng.standard_normal((6, 1, n_r)) + 1j * rng.standard_normal((6, 1, n_r))
+        runs.append(dataclasses.replace(base, x0=x / np.linalg.norm(x)))
+    tp = TimePropagation(runs, precision="fp64", groups=[list(range(cols))])
+    tp.step(1)
+    got = [tp.orbitals(i) for i in range(cols)]
+    tp.close()
+    for r, g in zip(runs, got):
+        want = np.einsum("lba,lkb->lka", base.W, r.x0)
+        assert np.linalg.norm(g - want) < TOL * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n_l,n_orb,n_r", [(2, 1, 1), (5, 2, 127), (9, 3, 128), (17, 1, 129), (33, 4, 600)])
+def test_observables_noalloc_at_the_edges(n_l, n_orb, n_r):
+    """Rows of fewer radii than threads, of one more than a multiple, m from 0 to N_l - 1 and an m
+    outside 0 .. N_l - 1, which contributes nothing."""
+    import torch
+    rng = np.random.default_rng(n_r)
+    x = rng.standard_normal((n_l, n_orb, n_r)) + 1j * rng.standard_normal((n_l, n_orb, n_r))
+    r = np.sort(rng.uniform(0.1, 50.0, n_r))
+    m = np.array(([0, n_l - 1, -1, n_l + 3] * 2)[:n_orb], dtype=np.int32)
+    l = np.arange(n_l)[:, None]
+    keep = (l >= m[None]) & (m >= 0)[None] & (m < n_l)[None]
+    for k in range(n_orb):
+        x[~keep[:, k], k] = 0.0
+    mf = np.clip(m, 0, n_l - 1)[None].astype(float)
+    c = np.sqrt(np.where(l >= mf, ((l + 1.0) ** 2 - mf ** 2) / ((2 * l + 1.0) * (2 * l + 3.0)), 0.0))[..., None]
+    z = np.zeros_like(x)
+    z[:-1] += c[:-1] * x[1:]
+    z[1:] += c[:-1] * x[:-1]
+    p = x.conj() * z
+    dev = torch.device("cuda", 0)
+    xd, rd, md = torch.from_numpy(x).to(dev), torch.from_numpy(r).to(dev), torch.from_numpy(m).to(dev)
+    dip = torch.full((n_l, n_orb), float("nan"), dtype=torch.complex128, device=dev)
+    acc, norm = torch.full_like(dip, float("nan")), torch.full((n_orb,), float("nan"), dtype=torch.float64, device=dev)
+    rc = load_library().ggb_observables_noalloc(xd.data_ptr(), rd.data_ptr(), md.data_ptr(), n_l, n_orb, n_r, dip.data_ptr(),
+                                                acc.data_ptr(), norm.data_ptr(), ctypes.c_void_p(None))
+    assert rc == 0
+    torch.cuda.synchronize()
+    for got, q in ((dip, r), (acc, r ** -2.0)):
+        scale = (np.abs(x) * np.abs(z) * q).sum(-1).max() + 1e-300
+        assert np.abs(got.cpu().numpy() - (p * q).sum(-1)).max() <= TOL * scale
+    assert np.allclose(norm.cpu().numpy(), (np.abs(x) ** 2).sum(axis=(0, 2)), rtol=TOL, atol=0)
