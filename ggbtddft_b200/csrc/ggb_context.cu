@@ -34,6 +34,7 @@ struct GroupHost {
   // device
   double *r_d = nullptr, *drdx_d = nullptr, *P_d = nullptr;
   double2* W_d = nullptr;        // FP64 form
+  double *frag_d = nullptr;
   double *mats_d = nullptr, *dph_d = nullptr, *coef_d = nullptr;
   double2 *x_d = nullptr, *y_d = nullptr;     // FP64 orbitals
   int *col_run_d = nullptr, *col_m_d = nullptr, *col_occ_d = nullptr, *runs_d = nullptr;
@@ -351,6 +352,14 @@ static int prepare_theta_tables(ggb_ctx* ctx, GroupHost& g, int n_mp) {
   return GGB_OK;
 }
 
+// The orbitals that k_finalize takes the observables from (the forms whose second half runs on the FP64
+// angular kernel), or null: it adds the second half's partials.
+static const double2* obs_source(const ggb_ctx* ctx, const GroupHost& g) {
+  const bool fp64_angular = ctx->dims.precision == GGB_FP64 ||
+                            (ctx->dims.precision == GGB_SPLIT_INT8 && g.mixed.angular_fp64);
+  return fp64_angular ? g.x_d : nullptr;
+}
+
 static int prepare(ggb_ctx* ctx) {
   if (ctx->prepared) return GGB_OK;
   int n_l_max = 0, n_r_max = 0;
@@ -380,6 +389,26 @@ static int prepare(ggb_ctx* ctx) {
     int rc;
     if ((rc = dalloc(ctx, &g.mats_d, mats.size()))) return rc;
     CK(cudaMemcpy(g.mats_d, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (ctx->dims.precision != GGB_SPLIT_BF16) {
+      // FP64 MMA fragments: lane (gid, q) of row tile rt holds S[l][8 rt + gid] at l = 8 kp + 4 e + q,
+      // e = 0, 1, of k-step pair kp; rows l < m and beyond N_l are zero
+      const int n8 = (n_l + 7) / 8;
+      std::vector<double> frag((size_t)n_mats * n_m * n8 * n8 * 64, 0.0);
+      size_t o = 0;
+      for (int mm = 0; mm < n_mats * n_m; ++mm) {
+        const double* S = mats.data() + (size_t)mm * n_l * ldS;
+        const int m = mm % n_m;
+        for (int rt = 0; rt < n8; ++rt)
+          for (int kp = 0; kp < n8; ++kp)
+            for (int lane = 0; lane < 32; ++lane)
+              for (int e = 0; e < 2; ++e, ++o) {
+                const int j = 8 * rt + lane / 4, l = 8 * kp + 4 * e + lane % 4;
+                if (j < n_l && l < n_l && l >= m) frag[o] = S[(size_t)l * ldS + j];
+              }
+      }
+      if ((rc = dalloc(ctx, &g.frag_d, frag.size()))) return rc;
+      CK(cudaMemcpy(g.frag_d, frag.data(), frag.size() * sizeof(double), cudaMemcpyHostToDevice));
+    }
     std::vector<double> dph((size_t)4 * n_m * ldS, 0.0);
     for (int c = 0; c < 4; ++c)
       for (int m = 0; m < n_m; ++m)
@@ -422,11 +451,17 @@ static int prepare(ggb_ctx* ctx) {
     const int n_g = g.d.n_r + 1;
     a.n_g_fac = (double)(n_g * (n_g + 1)) / 2.0;
     a.r = g.r_d; a.drdx = g.drdx_d; a.P = g.P_d;
-    a.mats = g.mats_d; a.dph = g.dph_d; a.coef = g.coef_d;
+    a.mats = g.mats_d; a.frag = g.frag_d; a.dph = g.dph_d; a.coef = g.coef_d;
     a.col_run = g.col_run_d; a.col_m = g.col_m_d; a.col_occ = g.col_occ_d; a.runs_of_group = g.runs_d;
     a.runs = ctx->runs_dev;
     a.dens = g.dens_d; a.obs = g.obs_d; a.step = g.step_d; a.status = ctx->status_d; a.done = g.done_d;
     a.fin_cnt = g.fin_cnt_d; a.fin_scr = g.fin_scr_d;
+    int max_orb = 0;
+    for (int ri : g.runs) max_orb = std::max(max_orb, ctx->runs[ri].d.n_orb);
+    a.fin_ob = obs_source(ctx, g) ? std::min(FIN_OB_ROWS, (n_l * max_orb + 7) / 8) : FIN_OB;
+    // the int8 form's initial density is summed over the lane groups of its own tiles (4 of 32 radii,
+    // 8 of 16), so that its potentials do not depend on the FP64 kernel's tile
+    a.den_groups = ctx->dims.precision == GGB_SPLIT_INT8 ? 128 / g.obs_seg : 0;
     a.chain[0] = c0; a.chain[1] = c1;
     a.chain[2] = c2;
     if (ctx->dims.precision != GGB_FP64) {
@@ -454,12 +489,12 @@ static void launch_group_step(ggb_ctx* ctx, GroupHost& g, cudaStream_t s) {
   if (ctx->dims.precision == GGB_FP64) {
     launch_angular_fp64(a, 0, g.x_d, g.y_d, 0, s);
     launch_radial_fp64(a, g.W_d, g.y_d, g.x_d, s);
-    launch_angular_fp64(a, 1, g.x_d, g.x_d, 1, s);
+    launch_angular_fp64(a, 1, g.x_d, g.x_d, a.n_den > 0, s);
   } else {
     mixed_step(g.mixed, a, s);
   }
   if (a.theta_tab) launch_theta_potentials(a, g.theta_args, g.x_d, s);
-  launch_finalize(a, 1, s);
+  launch_finalize(a, obs_source(ctx, g), 1, s);
 }
 
 // n steps of every group.  With several groups, each group's steps go to its own stream, forked
@@ -493,11 +528,11 @@ static int launch_steps(ggb_ctx* ctx, cudaStream_t s, int n) {
 static int launch_init(ggb_ctx* ctx, GroupHost& g, cudaStream_t s) {
   const GroupArgs& a = g.args;
   if (ctx->dims.precision == GGB_FP64) {
-    launch_angular_fp64(a, 2, g.x_d, g.x_d, 1, s);   // empty chain: partials of the initial orbitals
+    launch_angular_fp64(a, 2, g.x_d, nullptr, a.n_den > 0, s);   // empty chain: the initial orbitals' density
   } else {
     mixed_init(g.mixed, a, g.x_d, s);
   }
-  launch_finalize(a, 0, s);
+  launch_finalize(a, obs_source(ctx, g), 0, s);
   if (a.theta_tab) launch_theta_potentials(a, g.theta_args, g.x_d, s);
   CK(cudaGetLastError());
   g.needs_init = false;
@@ -535,13 +570,9 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
     g.V.assign(4, std::vector<std::vector<double>>(g.d.n_m));
     g.D.assign(4, std::vector<std::vector<double>>(g.d.n_m));
     g.ang_set.assign(4, std::vector<bool>(g.d.n_m, false));
-    // observables partials: one per CTA tile of radii.  The angular kernels take 32 radii per CTA
-    // (each CTA streams the chain matrices once per product: fewer radii per CTA cost more of that
-    // traffic than the extra CTAs gain, measured for the FP64 form), the int8 form 16 when N_l > 128
-    // (two M tiles of channels)
-    // radii per observables partial = the angular tile: 16 for the FP64 form and for the int8 form
-    // with two channel tiles (N_l > 128), 32 otherwise
-    g.obs_seg = (dims->precision == GGB_FP64 || (dims->precision == GGB_SPLIT_INT8 && g.d.n_l > 128)) ? 16 : TR;
+    // radii per observables partial = the angular tile: 16 for the int8 form with two channel tiles
+    // (N_l > 128), 32 otherwise (the FP64 angular kernel leaves the observables to k_finalize)
+    g.obs_seg = (dims->precision == GGB_SPLIT_INT8 && g.d.n_l > 128) ? 16 : TR;
     g.n_tiles = (g.d.n_r + g.obs_seg - 1) / g.obs_seg;
     g.ldS = ((g.d.n_l + 7) / 8) * 8;
   }
@@ -571,9 +602,9 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
     if (g.runs.empty()) return bad(GGB_ERR_ARG, "empty group");
     const size_t nr = g.d.n_r, nl = g.d.n_l, nc = g.n_cols;
     if ((rc = dalloc(ctx, &g.r_d, nr)) || (rc = dalloc(ctx, &g.drdx_d, nr)) || (rc = dalloc(ctx, &g.P_d, nr)) ||
-        (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles)) ||
+        (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (dims->precision != GGB_FP64 && (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles))) ||
         (rc = dalloc(ctx, &g.step_d, 1)) || (rc = dalloc(ctx, &g.done_d, 1)) ||
-        (rc = dalloc(ctx, &g.fin_cnt_d, g.runs.size())) || (rc = dalloc(ctx, &g.fin_scr_d, nc * FIN_OB * 8)) ||
+        (rc = dalloc(ctx, &g.fin_cnt_d, g.runs.size())) || (rc = dalloc(ctx, &g.fin_scr_d, nc * std::max<size_t>(FIN_OB * 8, nl * 10))) ||
         (rc = dalloc(ctx, &g.col_run_d, nc)) || (rc = dalloc(ctx, &g.col_m_d, nc)) ||
         (rc = dalloc(ctx, &g.col_occ_d, nc)) || (rc = dalloc(ctx, &g.runs_d, g.runs.size())))
       return bad(rc, "alloc");
@@ -783,13 +814,13 @@ int ggb_launch_phase(ggb_ctx* ctx, int phase, void* stream) {
     if (ctx->dims.precision == GGB_FP64) {
       if (phase == 0) launch_angular_fp64(a, 0, g.x_d, g.y_d, 0, s);
       if (phase == 1) launch_radial_fp64(a, g.W_d, g.y_d, g.x_d, s);
-      if (phase == 2) launch_angular_fp64(a, 1, g.x_d, g.x_d, 1, s);
+      if (phase == 2) launch_angular_fp64(a, 1, g.x_d, g.x_d, a.n_den > 0, s);
     } else {
       mixed_phase(g.mixed, a, phase, s);
     }
     if (phase == 3) {
       if (a.theta_tab) launch_theta_potentials(a, g.theta_args, g.x_d, s);
-      launch_finalize(a, 2, s);
+      launch_finalize(a, obs_source(ctx, g), 2, s);
     }
   }
   CK(cudaGetLastError());

@@ -7,6 +7,7 @@
 //   W        radial propagators, FP64 form: double2 [N_l][N_r][N_r] = propagatorL%03d.bin.
 //   mats     angular chain matrices, [n_mats][N_m][N_l][ldS] doubles, stored so that the kernel's
 //            product is y[j] = sum_l S[l][j] x[l]  (S = A^T of the left multiplier A).
+//   frag     the same matrices as FP64 MMA fragments, [n_mats][N_m][row tile][k-step pair][lane][2].
 //   dph      angular eigenvalues D[c][m][j], [4][N_m][ldS].
 //   coef     angular coefficient tables [COEF_N][N_m][N_l] (cu, cd, p, qu, qd, p3lm, f3lm).
 //   dens     density partials per column [n_cols][4][N_r] (not yet occupation weighted).
@@ -22,7 +23,8 @@ constexpr int TR = 32;            // radii per angular tile (one warp-width, coa
 constexpr int ANG_WARPS = 8;      // warps per angular CTA
 constexpr int MAX_NL = 220;       // largest N_l: two [N_l][32] complex128 tiles fit in 227 KB of shared memory
 constexpr int MAX_NR = 8192;      // largest N_r: three [N_r] FP64 rows of the potentials kernel
-constexpr int FIN_OB = 32;         // observables blocks per run in k_finalize (slices of l)
+constexpr int FIN_OB = 32;         // observables blocks per run in k_finalize: slices of l, from partials
+constexpr int FIN_OB_ROWS = 148;   // ... at most, from the orbitals (8 rows (l, orbital) per block and round)
 constexpr int N_DEN = 4;          // density multipoles carried per column (L = 0..3)
 
 // status bits (sticky, OR-ed on the device)
@@ -92,6 +94,7 @@ struct GroupArgs {
   const double* drdx;
   const double* P;
   const double* mats;
+  const double* frag;       // the chain matrices in fragment order of the FP64 angular kernel
   const double* dph;
   const double* coef;
   const int* col_run;   // [n_cols] run index within ctx
@@ -104,8 +107,10 @@ struct GroupArgs {
   int* step;                // ctx-wide step counter
   unsigned* status;
   unsigned* done;           // block counter for the last-block step increment
+  int fin_ob;               // observables blocks per run
+  int den_groups;           // lane groups of the FP64 angular kernel's density sums (0: as many as fit)
   unsigned* fin_cnt;        // [n_runs] finished observables blocks of the step (last-block totals)
-  double* fin_scr;          // [n_cols][FIN_OB][8] slice totals of the observables (double-double)
+  double* fin_scr;          // [n_cols][FIN_OB][8] slice or [n_cols][N_l][10] row totals of the observables (double-double)
   Chain chain[3];   // first half, second half, empty (initial partials)
 };
 
@@ -149,11 +154,11 @@ __device__ __forceinline__ dd dd_shfl_up(dd a, int d) {
 }
 
 // launchers (ggb_kernels_fp64.cu)
-void launch_angular_fp64(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_obs,
-                         cudaStream_t s);
+void launch_angular_fp64(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s);
 void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin, double2* xout,
                         cudaStream_t s);
-void launch_finalize(const GroupArgs& g, int mode, cudaStream_t s);
+// x: the orbitals the observables are taken from, or null: from the angular kernel's partials (g.obs)
+void launch_finalize(const GroupArgs& g, const double2* x, int mode, cudaStream_t s);
 size_t angular_smem_fp64(int n_l);
 cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max);
 cudaError_t set_max_dynamic_smem(const void* fn, int optin);

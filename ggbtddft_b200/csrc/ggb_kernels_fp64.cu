@@ -1,15 +1,14 @@
 // FP64 (parity form) kernels of the split-operator step.
 //
-//  k_angular_fp64  one half of the angular step for a tile of 16 radii of one orbital column:
-//                  the whole l-vector of every radius is held in shared memory while the chain
+//  k_angular_fp64  one half of the angular step for a tile of radii of one orbital column: the
+//                  whole l-vector of every radius is held in shared memory while the chain
 //                  (rotate -> phase -> [pre-multiplied rotate pair] -> phase ... -> rotate back,
 //                  plus the l-diagonal S phase) is applied, each product on the FP64 tensor cores
 //                  (mma.sync m8n8k4).  Replaces, per half-step, the 3 launches of each of
 //                  h_couplingFF/FP/D/P (couplingP.cuh:108-125, couplingD.cuh, couplingF.cuh) and
 //                  h_couplingS (couplingS.cuh:43-57).  The second half also produces the
-//                  density-multipole and dipole/acceleration partial sums of the new orbitals
-//                  (hartreePotentialDensity.cuh:1-181, dipoleMoment.cuh:1-75,
-//                  dipoleAcceleration.cuh:1-71), so the orbitals are read once per half-step.
+//                  density-multipole partial sums of the new orbitals
+//                  (hartreePotentialDensity.cuh:1-181).
 //  k_radial_fp64   x_l <- A_l x_l for every l with A_l(a,b) = W[l][b][a]: the batched ZGEMM of
 //                  h_propagationH0 (h_timePropagation.cuh:1-30), out of place.  More than nine
 //                  columns: persistent, two CTAs per SM; a producer warp streams the W rows and x
@@ -34,27 +33,29 @@ namespace ggb {
 // angular chain
 // ---------------------------------------------------------------------------------------------
 
-// A tile is RT radii of one orbital column (RT = the group's observables segment: 16 for the FP64
-// form, 16 or 32 for the initial partials of the int8 form): the whole l-vector of each radius sits
-// in shared memory as a [rows][2 RT + 8] FP64 matrix (column 2 rad + 0/1 = real/imaginary part of
-// radius rad; rows N_l rounded up to 8, zero beyond N_l), and every product of the chain
-// y_j = sum_l S[l][j] x_l is a small real GEMM  Y (N_l x 2 RT) = S^T (N_l x N_l) X (N_l x 2 RT)  on
-// the FP64 tensor cores: mma.sync m8n8k4 (8 channels x 8 columns x 4 l per instruction).  Each warp
-// owns pairs of 8-channel tiles (16 j) over all 2 RT columns; its S fragments come from L2
-// (read-only path), prefetched one chunk of AM_KU k-steps ahead; its X fragments from shared
-// memory.  The phases are applied to the accumulators in registers (each thread holds whole complex
-// numbers: the real and imaginary column of one radius), then written to the other buffer for the
-// next product.
-constexpr int AM_WARPS = 4;
-constexpr int AM_KU = 4;                    // k-steps (4 l each) per prefetch chunk
-// row stride in doubles: +8 puts the 4 rows of an X fragment on alternating bank halves
-__host__ __device__ constexpr int angular_ldx(int rt) { return 2 * rt + 8; }
-
-__host__ __device__ constexpr int angular_rows_mma(int n_l) {
-  // N_l rounded up to 8 (the channel tiles), and at least 16 rows: the free buffer holds the
-  // AM_NSUB x N_DEN x AM_RT density partials of the epilogue
-  return ((n_l + 7) / 8 * 8) > 16 ? (n_l + 7) / 8 * 8 : 16;
-}
+// A tile is P radii of one orbital column.  Its l-vectors sit in shared memory as a [rows][2 P + 4]
+// FP64 matrix (column 2 p + 0/1 = real/imaginary part of radius p; rows N_l rounded up to 8, zero beyond
+// N_l; the odd multiple of four doubles puts the fragment loads' 4 rows on different banks), and every
+// product of the chain y_j = sum_l S[l][j] x_l is a small real GEMM  Y (N_l x 2 P) = S^T X  on the FP64
+// tensor cores: mma.sync m8n8k4 (8 channels x 8 columns x 4 l per instruction).  The warps form 8 row
+// groups x WN column groups; a warp owns the 8-channel tiles rt = group, group + 8, ... (R of them) over
+// NT 8-column tiles, all of whose accumulators it holds, so that the product goes back in place: one
+// copy of the tile in shared memory.  Each S element is used by one row group, so it comes straight
+// from L2 into registers, laid out in fragment order (a warp's two k steps are 512 contiguous bytes),
+// AM_D pairs of k steps ahead of the products; the first product's are requested before the orbitals.
+// The phases are a pass over the tile by all threads (sincos per element), since the row tiles do not
+// divide evenly over the warps.
+//
+// P follows the number of tiles (angular_points): the smallest tile while all fit on the SMs at once
+// (one column on 200 radii: 50 blocks of 4 radii, where 16-radius tiles made 13 blocks), up to 40 radii
+// when that fills the SMs exactly once (nine columns on 600 radii: 135 blocks; at 16 radii 342 blocks,
+// 2.3 per SM, left a third of them waiting).  FP64-tensor bound at the large end (2 products x 4 N_l^2
+// flop per radius and column), latency bound at the small one.
+constexpr int AM_ROW_GROUPS = 8;
+__host__ __device__ constexpr int angular_ldx(int points) { return 2 * points + 4; }
+__host__ __device__ constexpr int angular_rows(int n_l) { return (n_l + 7) / 8 * 8; }
+// lane groups of the density's partial sums
+__host__ __device__ constexpr int angular_den_groups(int threads, int points) { return threads / points; }
 
 __device__ __forceinline__ void mma_f64_8x8x4(double& c0, double& c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -62,48 +63,90 @@ __device__ __forceinline__ void mma_f64_8x8x4(double& c0, double& c1, double a, 
                : "d"(a), "d"(b));
 }
 
-// One half of the angular step (or, with the empty chain of half 2, only the epilogue): replaces,
-// per half-step, the 3 launches of each of h_couplingFF/FP/D/P (couplingP.cuh:108-125,
-// couplingD.cuh, couplingF.cuh) and h_couplingS (couplingS.cuh:43-57); the second half also
-// produces the density-multipole and dipole/acceleration partial sums of the new orbitals
-// (hartreePotentialDensity.cuh:1-181, dipoleMoment.cuh:1-75, dipoleAcceleration.cuh:1-71).
-template <int RT>
-__global__ void __launch_bounds__(AM_WARPS * 32)
-k_angular_fp64(GroupArgs g, int half, const double2* __restrict__ xin, double2* xout, int do_obs) {
-  constexpr int AM_RT = RT;
-  constexpr int AM_LDX = angular_ldx(RT);
-  constexpr int AM_NT = 2 * RT / 8;                  // 8-column tiles per row
-  constexpr int AM_NSUB = AM_WARPS * 32 / RT;        // lane groups of RT threads (epilogue)
-  extern __shared__ double smd[];
-  __shared__ double s_rr[RT], s_rE[RT], s_v1[RT], s_v2[RT], s_v3[RT], s_sb[RT];
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const int gid = lane >> 2;      // fragment row group
-  const int q = lane & 3;         // fragment thread in group
-  const int n_l = g.n_l;
-  const int rows = angular_rows_mma(n_l);
-  const int tilesN = (g.n_r + AM_RT - 1) / AM_RT;
+// Density multipoles L = 0 .. n_den - 1 at one radius over l in [l0, l1) (rows of this m, l0 >= m),
+// every product x_l.x_(l+d) taken once: c_u(l) serves the terms (l, l+1) and (l+1, l) of the literal
+// sums, c_d(l+1) being c_u(l), and likewise for the other couplings.  For N_l >= m + 7 the literal l
+// ranges cover every l once, but for l = N_l - 4 of the octupole, counted twice without its upper
+// coupling (the reference's tail loop restarts there, hartreePotentialDensity.cuh:150).
+template <int STRIDE>
+__device__ __forceinline__ void density_window(int n_den, int n_l, const double2* xs, const double* rows, size_t rs,
+                                               int l0, int l1, double (&d)[N_DEN]) {
+  const double *cu = rows + CF_CU * rs, *pp = rows + CF_P * rs, *qu = rows + CF_QU * rs, *p3 = rows + CF_P3 * rs,
+               *f3 = rows + CF_F3 * rs;
+  auto at = [&](int l) { return l < n_l ? xs[(size_t)l * STRIDE] : make_double2(0.0, 0.0); };
+  auto dot = [](double2 a, double2 b) { return a.x * b.x + a.y * b.y; };
+  double2 x0 = at(l0), x1 = at(l0 + 1), x2 = at(l0 + 2);
+  for (int l = l0; l < l1; ++l) {
+    const double2 x3 = at(l + 3);
+    const double d0 = dot(x0, x0);
+    d[0] += d0;
+    if (n_den > 1) {
+      const double d1 = dot(x0, x1);
+      d[1] += 2.0 * cu[l] * d1;
+      if (n_den > 2) d[2] += pp[l] * d0 + 2.0 * qu[l] * dot(x0, x2);
+      if (n_den > 3) {
+        d[3] += 2.0 * (p3[l] * d1 + f3[l] * dot(x0, x3));
+        if (l == n_l - 4)
+          d[3] += f3[l - 3] * dot(xs[(size_t)(l - 3) * STRIDE], x0) + p3[l - 1] * dot(xs[(size_t)(l - 1) * STRIDE], x0) +
+                  p3[l] * d1;
+      }
+    }
+    x0 = x1;
+    x1 = x2;
+    x2 = x3;
+  }
+}
+
+// One half of the angular step (or, with the empty chain of half 2, only the density): replaces, per
+// half-step, the 3 launches of each of h_couplingFF/FP/D/P (couplingP.cuh:108-125, couplingD.cuh,
+// couplingF.cuh) and h_couplingS (couplingS.cuh:43-57); the second half also produces the
+// density-multipole partial sums of the new orbitals (hartreePotentialDensity.cuh:1-181).
+template <int NT, int WN, int R>
+__global__ void __launch_bounds__(AM_ROW_GROUPS * WN * 32)
+k_angular_fp64(GroupArgs g, int half, const double2* __restrict__ xin, double2* xout, int do_den) {
+  constexpr int P = 4 * NT * WN;
+  constexpr int LD = angular_ldx(P);
+  constexpr int THREADS = AM_ROW_GROUPS * WN * 32;
+  constexpr int AM_D = R * NT <= 2 ? 4 : 2;
+  extern __shared__ __align__(16) double xs[];
+  __shared__ double s_rE[P], s_v1[P], s_v2[P], s_v3[P], s_sb[P];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gid = lane >> 2, q = lane & 3;      // fragment row group, thread in group
+  const int wr = warp % AM_ROW_GROUPS, wn = warp / AM_ROW_GROUPS;
+  const int n_l = g.n_l, n8 = (n_l + 7) / 8;
+  const int tilesN = (g.n_r + P - 1) / P;
   const int col = blockIdx.x / tilesN;
-  const int tile = blockIdx.x - col * tilesN;
-  const int r0 = tile * AM_RT;
-  double* xs = smd;
-  double* ys = smd + (size_t)rows * AM_LDX;
+  const int r0 = (blockIdx.x - col * tilesN) * P;
   const int m = g.col_m[col];
+  const Chain& ch = g.chain[half];
+
+  // S^T fragments of row tile rt, k steps 2 kp and 2 kp + 1 (rows l < m are zero, as the reference's
+  // couplings start at l = m)
+  double2 fa[AM_D][R];
+  const double2* Sm = reinterpret_cast<const double2*>(g.frag) + (size_t)m * n8 * n8 * 32 + lane;
+  const size_t mat_stride = (size_t)g.n_m * n8 * n8 * 32;
+  auto load_a = [&](const double2* S, int kp, double2 (&dst)[R]) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int rt = wr + AM_ROW_GROUPS * i;
+      if (rt < n8 && kp < n8) dst[i] = __ldg(S + ((size_t)rt * n8 + kp) * 32);
+    }
+  };
+  if (ch.n_ops > 0)
+#pragma unroll
+    for (int d = 0; d < AM_D; ++d) load_a(Sm + ch.ops[0].mat * mat_stride, d, fa[d]);
+
   const RunDev run = g.runs[g.col_run[col]];
   int step = *g.step;
   if (step >= run.n_t) step = run.n_t - 1;  // overflow is flagged by k_finalize
-
-  // the tile's orbitals (zero beyond N_l and beyond N_r), zero padding rows in both buffers
-  for (int i = tid; i < rows * AM_RT; i += blockDim.x) {
-    const int l = i / AM_RT, rad = i - l * AM_RT, r = r0 + rad;
-    const double2 v = (l < n_l && r < g.n_r) ? xin[((size_t)l * g.n_cols + col) * g.n_r + r]
-                                             : make_double2(0.0, 0.0);
-    *reinterpret_cast<double2*>(xs + (size_t)l * AM_LDX + 2 * rad) = v;
-    if (l >= n_l) *reinterpret_cast<double2*>(ys + (size_t)l * AM_LDX + 2 * rad) = make_double2(0.0, 0.0);
+  // the tile's orbitals (zero beyond N_l and beyond N_r)
+  for (int i = tid; i < 8 * n8 * P; i += THREADS) {
+    const int l = i / P, p = i - l * P, r = r0 + p;
+    const double2 v = (l < n_l && r < g.n_r) ? xin[((size_t)l * g.n_cols + col) * g.n_r + r] : make_double2(0.0, 0.0);
+    *reinterpret_cast<double2*>(xs + (size_t)l * LD + 2 * p) = v;
   }
   // per-radius potentials
-  if (tid < AM_RT) {
+  if (tid < P) {
     const int r = r0 + tid;
     const bool rv = r < g.n_r;
     const int rc = rv ? r : 0;
@@ -116,7 +159,6 @@ k_angular_fp64(GroupArgs g, int half, const double2* __restrict__ xin, double2* 
       // couplingS.cuh:20-21, evaluated left to right
       sbase = run.v[rc] - run.v0[rc] + run.vexc[rc] - run.vexc0[rc];
     }
-    s_rr[tid] = rr;
     s_rE[tid] = rr * run.E[step];
     s_v1[tid] = v1;
     s_v2[tid] = v2;
@@ -127,154 +169,210 @@ k_angular_fp64(GroupArgs g, int half, const double2* __restrict__ xin, double2* 
   const double* pco = g.coef + ((size_t)CF_P * g.n_m + m) * n_l;
   __syncthreads();
 
-  const Chain& ch = g.chain[half];
   if (ch.pre_s) {
-    for (int i = tid; i < n_l * AM_RT; i += blockDim.x) {
-      const int l = i / AM_RT, rad = i - l * AM_RT;
-      double eta = s_sb[rad] + pco[l] * s_v2[rad];
+    for (int i = tid; i < n_l * P; i += THREADS) {
+      const int l = i / P, p = i - l * P;
+      double eta = s_sb[p] + pco[l] * s_v2[p];
       eta *= hdt;
-      double2* p = reinterpret_cast<double2*>(xs + (size_t)l * AM_LDX + 2 * rad);
-      *p = cmul_conj_phase(*p, eta);
+      double2* x = reinterpret_cast<double2*>(xs + (size_t)l * LD + 2 * p);
+      *x = cmul_conj_phase(*x, eta);
     }
     __syncthreads();
   }
 
-  const int k_steps = (n_l + 3) / 4;
-  const int n_pairs = ((n_l + 7) / 8 + 1) / 2;
   for (int o = 0; o < ch.n_ops; ++o) {
     const ChainOp op = ch.ops[o];
-    const double* S = g.mats + ((size_t)op.mat * g.n_m + m) * (size_t)n_l * g.ldS;
+    const double2* S = Sm + op.mat * mat_stride;
     const bool last = (o == ch.n_ops - 1);
-    const double* Dv = g.dph + ((size_t)op.coupling * g.n_m + m) * g.ldS;
-    for (int pr = warp; pr < n_pairs; pr += AM_WARPS) {
-      const int ja = pr * 16 + gid, jb = ja + 8;
-      const bool va = ja < n_l, vb = jb < n_l;
-      double acc[2][AM_NT][2];
+    double acc[R][NT][2];
 #pragma unroll
-      for (int t = 0; t < 2; ++t)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int nt = 0; nt < AM_NT; ++nt) acc[t][nt][0] = acc[t][nt][1] = 0.0;
-      // S fragments (A = S^T: row j, column l) of AM_KU k-steps; rows l < m are skipped, as the
-      // reference's couplings start at l = m
-      double fa[AM_KU][2], fn[AM_KU][2];
-      auto load_a = [&](int ks0, double (&dst)[AM_KU][2]) {
+      for (int nt = 0; nt < NT; ++nt) acc[i][nt][0] = acc[i][nt][1] = 0.0;
+    const double* xb = xs + (size_t)q * LD + wn * NT * 8 + gid;
+    for (int kp0 = 0; kp0 < n8; kp0 += AM_D) {
 #pragma unroll
-        for (int u = 0; u < AM_KU; ++u) {
-          const int l = (ks0 + u) * 4 + q;
-          const bool lv = l >= m && l < n_l;
-          dst[u][0] = (lv && va) ? __ldg(S + (size_t)l * g.ldS + ja) : 0.0;
-          dst[u][1] = (lv && vb) ? __ldg(S + (size_t)l * g.ldS + jb) : 0.0;
-        }
-      };
-      load_a(0, fa);
-      for (int ks0 = 0; ks0 < k_steps; ks0 += AM_KU) {
-        load_a(ks0 + AM_KU, fn);   // past the last k-step it loads nothing (l >= N_l)
+      for (int d = 0; d < AM_D; ++d) {
+        if (kp0 + d < n8 && wr < n8) {
+          const double* xr = xb + (size_t)(kp0 + d) * 8 * LD;
+          double fb[2][NT];
 #pragma unroll
-        for (int u = 0; u < AM_KU; ++u) {
-          if (ks0 + u < k_steps) {
-            const double* xr = xs + (size_t)((ks0 + u) * 4 + q) * AM_LDX + gid;
-            double fb[AM_NT];
+          for (int e = 0; e < 2; ++e)
 #pragma unroll
-            for (int nt = 0; nt < AM_NT; ++nt) fb[nt] = xr[nt * 8];
+            for (int nt = 0; nt < NT; ++nt) fb[e][nt] = xr[e * 4 * LD + nt * 8];
 #pragma unroll
-            for (int nt = 0; nt < AM_NT; ++nt) {
-              mma_f64_8x8x4(acc[0][nt][0], acc[0][nt][1], fa[u][0], fb[nt]);
-              mma_f64_8x8x4(acc[1][nt][0], acc[1][nt][1], fa[u][1], fb[nt]);
-            }
-          }
-        }
+          for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int u = 0; u < AM_KU; ++u) { fa[u][0] = fn[u][0]; fa[u][1] = fn[u][1]; }
-      }
-      // phases on the accumulators: thread (gid, q) holds channel j = pair base + 8 t + gid, radius
-      // 4 nt + q, real and imaginary part (couplingP.cuh:61-106 and twins)
+            for (int i = 0; i < R; ++i)
+              if (i == 0 || wr + AM_ROW_GROUPS * i < n8)
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int j = pr * 16 + 8 * t + gid;
-        if (j >= n_l) continue;
-        const double dj = Dv[j];
-#pragma unroll
-        for (int nt = 0; nt < AM_NT; ++nt) {
-          const int rad = 4 * nt + q;
-          double2 y = make_double2(acc[t][nt][0], acc[t][nt][1]);
-          if (op.phase == PH_THETA && j >= m) {
-            // the theta form: the whole angular potential at node x_j
-            double eta = (s_rE[rad] + s_v1[rad]) * dj + s_v2[rad] * legendre_p2(dj) +
-                         s_v3[rad] * legendre_p3(dj) + s_sb[rad];
-            // n_har > 4: the multipoles L >= 1 at this node come from the exact-quadrature table
-            if (g.theta_tab && r0 + rad < g.n_r) eta += run.htab[((size_t)m * n_l + j) * g.n_r + r0 + rad];
-            eta *= hdt;
-            y = cmul_conj_phase(y, eta);
-          } else if (op.phase != PH_NONE && j >= m) {
-            double eta;
-            if (op.phase == PH_P) eta = g.p_hartree ? (s_rE[rad] + s_v1[rad]) : s_rE[rad];
-            else if (op.phase == PH_D) eta = s_v2[rad];
-            else eta = s_v3[rad];   // FP and FF
-            eta *= hdt * dj;
-            y = cmul_conj_phase(y, eta);
-          }
-          if (last && ch.post_s) {
-            double eta = s_sb[rad] + pco[j] * s_v2[rad];
-            eta *= hdt;
-            y = cmul_conj_phase(y, eta);
-          }
-          *reinterpret_cast<double2*>(ys + (size_t)j * AM_LDX + 2 * rad) = y;
+                for (int nt = 0; nt < NT; ++nt)
+                  mma_f64_8x8x4(acc[i][nt][0], acc[i][nt][1], e ? fa[d][i].y : fa[d][i].x, fb[e][nt]);
+          load_a(S, kp0 + d + AM_D, fa[d]);
         }
       }
     }
+    if (!last)   // the next product's first fragments, under the phase pass
+#pragma unroll
+      for (int d = 0; d < AM_D; ++d) load_a(Sm + ch.ops[o + 1].mat * mat_stride, d, fa[d]);
+    // thread (gid, q) holds channel 8 rt + gid of radius 4 (wn NT + nt) + q: real and imaginary part
+    const bool direct = last && !ch.post_s;
+    const bool keep = !direct || do_den;
+    if (keep) __syncthreads();          // every warp has read the tile
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int j = 8 * (wr + AM_ROW_GROUPS * i) + gid;
+      if (j >= n_l) continue;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int p = 4 * (wn * NT + nt) + q;
+        const double2 y = make_double2(acc[i][nt][0], acc[i][nt][1]);
+        if (keep) *reinterpret_cast<double2*>(xs + (size_t)j * LD + 2 * p) = y;
+        if (direct && xout && r0 + p < g.n_r) xout[((size_t)j * g.n_cols + col) * g.n_r + r0 + p] = y;
+      }
+    }
+    if (keep) __syncthreads();
+    if (direct) break;
+    // phases (couplingP.cuh:61-106 and twins); the last product's is the S phase
+    const double* Dv = g.dph + ((size_t)op.coupling * g.n_m + m) * g.ldS;
+    for (int i = tid; i < n_l * P; i += THREADS) {
+      const int j = i / P, p = i - j * P;
+      double2* x = reinterpret_cast<double2*>(xs + (size_t)j * LD + 2 * p);
+      double2 y = *x;
+      if (op.phase == PH_THETA && j >= m) {
+        // the theta form: the whole angular potential at node x_j
+        const double dj = Dv[j];
+        double eta = (s_rE[p] + s_v1[p]) * dj + s_v2[p] * legendre_p2(dj) + s_v3[p] * legendre_p3(dj) + s_sb[p];
+        // n_har > 4: the multipoles L >= 1 at this node come from the exact-quadrature table
+        if (g.theta_tab && r0 + p < g.n_r) eta += run.htab[((size_t)m * n_l + j) * g.n_r + r0 + p];
+        eta *= hdt;
+        y = cmul_conj_phase(y, eta);
+      } else if (op.phase != PH_NONE && j >= m) {
+        double eta;
+        if (op.phase == PH_P) eta = g.p_hartree ? (s_rE[p] + s_v1[p]) : s_rE[p];
+        else if (op.phase == PH_D) eta = s_v2[p];
+        else eta = s_v3[p];   // FP and FF
+        eta *= hdt * Dv[j];
+        y = cmul_conj_phase(y, eta);
+      }
+      if (last) {
+        double eta = s_sb[p] + pco[j] * s_v2[p];
+        eta *= hdt;
+        y = cmul_conj_phase(y, eta);
+        if (xout && r0 + p < g.n_r) xout[((size_t)j * g.n_cols + col) * g.n_r + r0 + p] = y;
+      }
+      *x = y;
+    }
     __syncthreads();
-    double* t = xs; xs = ys; ys = t;
   }
 
-  const double2* x2 = reinterpret_cast<const double2*>(xs);
-  if (xout)
-    for (int i = tid; i < n_l * AM_RT; i += blockDim.x) {
-      const int l = i / AM_RT, rad = i - l * AM_RT, r = r0 + rad;
-      if (r < g.n_r) xout[((size_t)l * g.n_cols + col) * g.n_r + r] = x2[(size_t)l * (AM_LDX / 2) + rad];
-    }
-
-  if (do_obs) {
-    // lane groups of AM_RT threads, one radius per thread
-    const int lr = lane % AM_RT, sub = warp * (32 / AM_RT) + lane / AM_RT;
-    const double rr = s_rr[lr];
-    const double fr2 = (r0 + lr < g.n_r) ? pow(rr, -2.0) : 0.0;
-    observables_tile<double2, AM_LDX / 2>(g, x2, col, m, r0, lr, sub, AM_NSUB, rr, fr2);
-    // density multipoles: the literal l loops strided over the lane groups, then the groups summed
-    // in order (the free buffer holds the AM_NSUB x N_DEN x AM_RT partials)
+  if (do_den) {
+    // density multipoles: lane groups of P threads, one radius per thread, a range of l per group,
+    // then the groups summed in order (the tile's memory holds the groups' partials)
+    const double2* x2 = reinterpret_cast<const double2*>(xs);
     const int n_den = g.n_den > 0 ? g.n_den : 1;  // L = 0 is always needed for the norm
+    const int n_sub = g.den_groups > 0 ? g.den_groups : angular_den_groups(THREADS, P);
+    const int sub = tid / P, p = tid - sub * P;
     double d[N_DEN] = {0.0, 0.0, 0.0, 0.0};
-    density_partials<double2, AM_LDX / 2>(n_den, m, n_l, x2, lr, g.coef + (size_t)m * n_l, sub, AM_NSUB, d,
-                                          g.n_m * n_l);
-#pragma unroll
-    for (int L = 0; L < N_DEN; ++L) ys[(sub * N_DEN + L) * AM_RT + lr] = d[L];
+    if (sub < n_sub) {
+      if (g.den_groups > 0 || n_l < m + 7) {
+        // the literal l loops strided over the groups
+        density_partials<double2, LD / 2>(n_den, m, n_l, x2, p, g.coef + (size_t)m * n_l, sub, n_sub, d, g.n_m * n_l);
+      } else {
+        const int per = (n_l - m + n_sub - 1) / n_sub, l0 = m + sub * per;
+        density_window<LD / 2>(n_den, n_l, x2 + p, g.coef + (size_t)m * n_l, (size_t)g.n_m * n_l, l0, min(n_l, l0 + per), d);
+      }
+    }
     __syncthreads();
-    if (tid < n_den * AM_RT) {
-      const int L = tid / AM_RT, p = tid - L * AM_RT, rl = r0 + p;
+    if (sub < n_sub)
+#pragma unroll
+      for (int L = 0; L < N_DEN; ++L) xs[(sub * N_DEN + L) * P + p] = d[L];
+    __syncthreads();
+    for (int i = tid; i < n_den * P; i += THREADS) {
+      const int L = i / P, pp = i - L * P, rl = r0 + pp;
       double sum = 0.0;
-      for (int w = 0; w < AM_NSUB; ++w) sum += ys[(w * N_DEN + L) * AM_RT + p];
+      for (int w = 0; w < n_sub; ++w) sum += xs[(w * N_DEN + L) * P + pp];
       if (rl < g.n_r) g.dens[((size_t)col * N_DEN + L) * g.n_r + rl] = sum;
     }
   }
 }
 
-static size_t angular_smem_rt(int n_l, int rt) {
-  return 2 * (size_t)angular_rows_mma(n_l) * angular_ldx(rt) * sizeof(double);
+static int g_angular_sms = 0;
+static constexpr int ANGULAR_POINTS[] = {4, 8, 16, 24, 32, 40};
+
+static int angular_warps_n(int points) { return points == 4 ? 1 : 2; }
+static size_t angular_smem_points(int n_l, int points) {
+  const int threads = AM_ROW_GROUPS * angular_warps_n(points) * 32;
+  return std::max((size_t)angular_rows(n_l) * angular_ldx(points),
+                  (size_t)angular_den_groups(threads, points) * N_DEN * points) * sizeof(double);
 }
-// the largest launch for groups of up to n_l channels: 32-radius tiles only for N_l <= 128 (the int8
-// form's initial partials), 16-radius tiles otherwise
+// accumulators of a warp's row tiles and column tiles, in registers (512 threads: 128 each)
+static bool angular_points_ok(int n_l, int points) {
+  const int r = ((n_l + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS;
+  return r <= 2 || (r == 3 && points <= 32) || points <= 24;
+}
 size_t angular_smem_fp64(int n_l) {
-  return std::max(angular_smem_rt(std::min(n_l, 128), TR), angular_smem_rt(n_l, 16));
+  size_t most = 0;
+  for (int p : ANGULAR_POINTS)
+    if (angular_points_ok(n_l, p)) most = std::max(most, angular_smem_points(n_l, p));
+  return most;
 }
 
-void launch_angular_fp64(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_obs,
-                         cudaStream_t s) {
-  if (g.obs_seg == 16) {
-    const int tiles = g.n_cols * ((g.n_r + 15) / 16);
-    k_angular_fp64<16><<<tiles, AM_WARPS * 32, angular_smem_rt(g.n_l, 16), s>>>(g, half, xin, xout, do_obs);
-  } else {
-    const int tiles = g.n_cols * ((g.n_r + TR - 1) / TR);
-    k_angular_fp64<TR><<<tiles, AM_WARPS * 32, angular_smem_rt(g.n_l, TR), s>>>(g, half, xin, xout, do_obs);
+// Radii per block: the least rounds over the SMs x (radii + the time of a block that does not depend
+// on them, about that of 12 radii).
+static int angular_points(const GroupArgs& g) {
+  int best = 4;
+  long best_cost = -1;
+  for (int p : ANGULAR_POINTS) {
+    if (!angular_points_ok(g.n_l, p)) continue;
+    const long tiles = (long)g.n_cols * ((g.n_r + p - 1) / p);
+    const long cost = (tiles + g_angular_sms - 1) / g_angular_sms * (p + 12);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = p;
+    }
   }
+  return best;
+}
+
+template <int NT, int WN, int R>
+static void launch_angular_tile(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
+  constexpr int P = 4 * NT * WN;
+  const int tiles = g.n_cols * ((g.n_r + P - 1) / P);
+  k_angular_fp64<NT, WN, R><<<tiles, AM_ROW_GROUPS * WN * 32, angular_smem_points(g.n_l, P), s>>>(g, half, xin, xout, do_den);
+}
+template <int R>
+static void launch_angular_rows(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
+  switch (angular_points(g)) {
+    case 4: launch_angular_tile<1, 1, R>(g, half, xin, xout, do_den, s); break;
+    case 8: launch_angular_tile<1, 2, R>(g, half, xin, xout, do_den, s); break;
+    case 16: launch_angular_tile<2, 2, R>(g, half, xin, xout, do_den, s); break;
+    case 24: launch_angular_tile<3, 2, R>(g, half, xin, xout, do_den, s); break;
+    case 32: if constexpr (R <= 3) launch_angular_tile<4, 2, R>(g, half, xin, xout, do_den, s); break;
+    default: if constexpr (R <= 2) launch_angular_tile<5, 2, R>(g, half, xin, xout, do_den, s); break;
+  }
+}
+
+void launch_angular_fp64(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
+  switch (((g.n_l + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS) {
+    case 1: launch_angular_rows<1>(g, half, xin, xout, do_den, s); break;
+    case 2: launch_angular_rows<2>(g, half, xin, xout, do_den, s); break;
+    case 3: launch_angular_rows<3>(g, half, xin, xout, do_den, s); break;
+    default: launch_angular_rows<4>(g, half, xin, xout, do_den, s); break;
+  }
+}
+
+template <int R>
+static cudaError_t configure_angular_rows(int optin) {
+  cudaError_t e = set_max_dynamic_smem((const void*)k_angular_fp64<1, 1, R>, optin);
+  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<1, 2, R>, optin);
+  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<2, 2, R>, optin);
+  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<3, 2, R>, optin);
+  if constexpr (R <= 3)
+    if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<4, 2, R>, optin);
+  if constexpr (R <= 2)
+    if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<5, 2, R>, optin);
+  return e;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -720,20 +818,58 @@ __device__ __forceinline__ double ipow(double x, int L) {
   return p;
 }
 
+// Dipole, acceleration and norm of orbital row (l, column col) by one warp, the lanes striding over
+// the radii, in double-double: <x_l | r (c_u x_(l+1) + c_d x_(l-1))>, the same with r^-2, and |x_l|^2
+// (dipoleMoment.cuh:19-43, dipoleAcceleration.cuh:17-41 and their cublasZdotc).  Every lane gets the sums.
+__device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x, int col, int l, int lane, dd (&s)[5]) {
+#pragma unroll
+  for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
+  const int n_l = g.n_l, n_r = g.n_r, m = g.col_m[col];
+  if (l < m) return;
+  // the first row has no lower, the last no upper neighbour
+  const bool up = l + 1 < n_l, down = l > m;
+  const double c_u = up ? g.coef[((size_t)CF_CU * g.n_m + m) * n_l + l] : 0.0;
+  const double c_d = down ? g.coef[((size_t)CF_CD * g.n_m + m) * n_l + l] : 0.0;
+  const size_t ls = (size_t)g.n_cols * n_r;
+  const double2* row = x + (size_t)l * ls + (size_t)col * n_r;
+#pragma unroll 2
+  for (int i = lane; i < n_r; i += 32) {
+    const double2 xl = row[i];
+    const double2 xu = up ? row[ls + i] : make_double2(0.0, 0.0);
+    const double2 xd = down ? (row - ls)[i] : make_double2(0.0, 0.0);
+    const double rr = g.r[i], fr2 = 1.0 / (rr * rr);
+    const double zx = c_u * xu.x + c_d * xd.x, zy = c_u * xu.y + c_d * xd.y;
+    const double px = xl.x * zx + xl.y * zy, py = xl.x * zy - xl.y * zx;   // conj(x_l) . z
+    s[0] = dd_add(s[0], dd{rr * px, 0.0});
+    s[1] = dd_add(s[1], dd{rr * py, 0.0});
+    s[2] = dd_add(s[2], dd{fr2 * px, 0.0});
+    s[3] = dd_add(s[3], dd{fr2 * py, 0.0});
+    s[4] = dd_add(s[4], dd{xl.x * xl.x + xl.y * xl.y, 0.0});
+  }
+#pragma unroll
+  for (int q = 0; q < 5; ++q) s[q] = warp_sum_dd2(s[q]);
+}
+
 // Blocks: for each run of the group, n_den Hartree blocks (L = 0..n_den-1; block L = 0 also does
-// the exchange potential) + FIN_OB observables blocks.  mode 0 = initial potentials (no observables,
+// the exchange potential) + g.fin_ob observables blocks.  mode 0 = initial potentials (no observables,
 // no step increment), mode 1 = end of step, mode 2 = end of step without the step increment and the
 // watchdog checks (the per-phase timing).
 //
-// Observables: observables block ob sums the partials of a slice of l (one warp per orbital, lanes
-// striding over the tiles, double-double), writes the per-l series and its slice's totals to a
-// scratch row; the last of the run's FIN_OB blocks to finish (a per-run counter) adds the slices in
-// order, writes the totals and the norm and runs the NaN / norm-growth watchdog.
-__global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, int mode) {
+// Observables, from the orbitals (ROWS: the FP64 angular kernel): one warp per (l, orbital) row of the
+// run, straight from L2 where the orbitals of a run still are (the angular kernel's tiles summed them
+// before: a double-double warp reduction of every row for every 16 radii, 8 us of its second half for
+// one column on 200 radii and 25 us for nine on 600).  From the partials of the int8 and BF16 angular
+// kernels: observables block ob sums the partials of a slice of l (one warp per orbital, lanes
+// striding over the tiles, double-double).  Either way the per-l series are written, the rows' or
+// slices' totals go to a scratch row, and the last of the run's blocks to finish (a per-run counter)
+// adds them, writes the totals and the norm and runs the NaN / norm-growth watchdog.
+// ROWS: the observables come from the orbitals x (the partial sums' kernel needs half its registers).
+template <bool ROWS>
+__global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
   extern __shared__ double fsm[];  // [3][N_r]
   __shared__ dd wsum[FIN_THREADS / 32];
   __shared__ int s_last;
-  const int nb = g.n_den + FIN_OB;
+  const int nb = g.n_den + g.fin_ob;
   const int ri = blockIdx.x / nb;
   const int role = blockIdx.x - ri * nb;  // < n_den: Hartree L = role; >= n_den: observables slice
   const int run_idx = g.runs_of_group[ri];
@@ -744,12 +880,27 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, int mode)
   const bool obs_block = role >= g.n_den;
   const int ob = role - g.n_den;
 
-  if (obs_block && mode != 0) {
-    if (step >= run.n_t) {
-      if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);
+  if (obs_block && mode != 0 && step >= run.n_t) {
+    if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);
+  } else if (obs_block && (mode != 0 || ROWS)) {
+    const int n_orb = run.n_orb;
+    if constexpr (ROWS) {
+      for (int i = ob * (FIN_THREADS / 32) + warp; i < n_l * n_orb; i += g.fin_ob * (FIN_THREADS / 32)) {
+        const int l = i / n_orb, k = i - l * n_orb;
+        dd s[5];
+        observe_row(g, x, run.col0 + k, l, lane, s);
+        if (lane == 0) {
+          if (mode != 0 && g.per_l) {
+            run.dip[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
+            run.acc[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
+          }
+          double2* o = reinterpret_cast<double2*>(g.fin_scr) + ((size_t)(run.col0 + k) * n_l + l) * 5;
+#pragma unroll
+          for (int q = 0; q < 5; ++q) o[q] = make_double2(s[q].hi, s[q].lo);
+        }
+      }
     } else {
-      const int n_orb = run.n_orb;
-      const int l0 = ob * n_l / FIN_OB, l1 = (ob + 1) * n_l / FIN_OB;
+      const int l0 = ob * n_l / g.fin_ob, l1 = (ob + 1) * n_l / g.fin_ob;
       for (int k = warp; k < n_orb; k += FIN_THREADS / 32) {
         dd tx{0.0, 0.0}, ty{0.0, 0.0}, tz{0.0, 0.0}, tw{0.0, 0.0};
         for (int l = l0; l < l1; ++l) {
@@ -773,39 +924,53 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, int mode)
           o[4] = tz.hi; o[5] = tz.lo; o[6] = tw.hi; o[7] = tw.lo;
         }
       }
-      __syncthreads();
-      if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(g.fin_cnt + ri, 1u) == (unsigned)(FIN_OB - 1);
-      }
-      __syncthreads();
-      if (s_last) {
-        __threadfence();
-        // totals over l (the slices in order), the norm; one warp per orbital
-        for (int k = warp; k < n_orb; k += FIN_THREADS / 32) {
-          dd sx{0.0, 0.0}, sy{0.0, 0.0}, sz{0.0, 0.0}, sw{0.0, 0.0};
-          for (int b = 0; b < FIN_OB; ++b) {
+    }
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      s_last = atomicAdd(g.fin_cnt + ri, 1u) == (unsigned)(g.fin_ob - 1);
+    }
+    __syncthreads();
+    if (s_last) {
+      __threadfence();
+      // totals over l, the norm; one warp per orbital
+      for (int k = warp; k < n_orb; k += FIN_THREADS / 32) {
+        dd s[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
+        if constexpr (ROWS) {
+          const double2* o = reinterpret_cast<const double2*>(g.fin_scr) + (size_t)(run.col0 + k) * n_l * 5;
+          for (int l = lane; l < n_l; l += 32)
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+              const double2 v = __ldcg(o + (size_t)l * 5 + q);
+              s[q] = dd_add(s[q], dd{v.x, v.y});
+            }
+#pragma unroll
+          for (int q = 0; q < 5; ++q) s[q] = warp_sum_dd2(s[q]);
+        } else {
+          for (int b = 0; b < g.fin_ob; ++b) {      // the slices in order
             const double* o = g.fin_scr + ((size_t)(run.col0 + k) * FIN_OB + b) * 8;
-            sx = dd_add(sx, dd{__ldcg(o + 0), __ldcg(o + 1)}); sy = dd_add(sy, dd{__ldcg(o + 2), __ldcg(o + 3)});
-            sz = dd_add(sz, dd{__ldcg(o + 4), __ldcg(o + 5)}); sw = dd_add(sw, dd{__ldcg(o + 6), __ldcg(o + 7)});
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q] = dd_add(s[q], dd{__ldcg(o + 2 * q), __ldcg(o + 2 * q + 1)});
           }
           const double* dn = g.dens + (size_t)(run.col0 + k) * N_DEN * n_r;  // L = 0 row
-          dd nd{0.0, 0.0};
-          for (int q = lane; q < n_r; q += 32) nd = dd_add(nd, dd{dn[q], 0.0});
-          nd = warp_sum_dd2(nd);
-          const double nrm = nd.hi + nd.lo;
-          if (lane == 0) {
-            run.dip_tot[(size_t)k * run.n_t + step] = make_double2(sx.hi + sx.lo, sy.hi + sy.lo);
-            run.acc_tot[(size_t)k * run.n_t + step] = make_double2(sz.hi + sz.lo, sw.hi + sw.lo);
-            run.norm[(size_t)k * run.n_t + step] = nrm;
-            if (mode == 1) {
-              if (!(nrm == nrm) || isinf(nrm) || !(sx.hi == sx.hi) || !(sz.hi == sz.hi)) atomicOr(g.status, ST_NAN);
-              if (nrm > run.norm0[k] * (1.0 + g.norm_tol) + 1e-300) atomicOr(g.status, ST_NORM_GROWTH);
-            }
+          for (int q = lane; q < n_r; q += 32) s[4] = dd_add(s[4], dd{dn[q], 0.0});
+          s[4] = warp_sum_dd2(s[4]);
+        }
+        const double nrm = s[4].hi + s[4].lo;
+        if (lane == 0 && mode == 0) run.norm0[k] = nrm;   // for the growth watchdog
+        if (lane == 0 && mode != 0) {
+          run.dip_tot[(size_t)k * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
+          run.acc_tot[(size_t)k * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
+          run.norm[(size_t)k * run.n_t + step] = nrm;
+          if (mode == 1) {
+            if (!(nrm == nrm) || isinf(nrm) || !(s[0].hi == s[0].hi) || !(s[2].hi == s[2].hi)) atomicOr(g.status, ST_NAN);
+            if (nrm > run.norm0[k] * (1.0 + g.norm_tol) + 1e-300) atomicOr(g.status, ST_NORM_GROWTH);
           }
         }
-        if (tid == 0) g.fin_cnt[ri] = 0u;   // for the next launch (stream-ordered after this one)
       }
+      if (tid == 0) g.fin_cnt[ri] = 0u;   // for the next launch (stream-ordered after this one)
     }
   } else if (obs_block && mode == 0 && ob == 0) {
     // initial norm for the growth watchdog
@@ -849,7 +1014,8 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, int mode)
   }
 
   // exchange (block L = 0, or the first observables block when Hartree is off)
-  const bool xc_block = (g.n_den > 0) ? (role == 0) : (ob == 0);
+  // without Hartree the density is the frozen one: the potential stays what mode 0 wrote
+  const bool xc_block = (g.n_den > 0) ? (role == 0) : (ob == 0 && mode == 0);
   if (xc_block) {
     const bool pw92 = (run.flags & RUN_FLAG_PW92) != 0;
     for (int q = tid; q < n_r; q += FIN_THREADS) {
@@ -908,10 +1074,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, int mode)
   }
 }
 
-void launch_finalize(const GroupArgs& g, int mode, cudaStream_t s) {
-  const dim3 grid(g.n_runs * (g.n_den + FIN_OB)), block(FIN_THREADS);
+void launch_finalize(const GroupArgs& g, const double2* x, int mode, cudaStream_t s) {
+  const dim3 grid(g.n_runs * (g.n_den + g.fin_ob)), block(FIN_THREADS);
   const size_t smem = 3 * (size_t)g.n_r * sizeof(double);
-  k_finalize<<<grid, block, smem, s>>>(g, mode);
+  if (x) k_finalize<true><<<grid, block, smem, s>>>(g, x, mode);
+  else k_finalize<false><<<grid, block, smem, s>>>(g, x, mode);
 }
 
 // Allow a kernel the largest dynamic shared memory the device offers beyond its static part.
@@ -932,13 +1099,19 @@ cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max) {
   if (e != cudaSuccess) return e;
   if (angular_smem_fp64(n_l_max) > (size_t)optin || 3 * (size_t)n_r_max * sizeof(double) > (size_t)optin)
     return cudaErrorInvalidValue;
-  e = set_max_dynamic_smem((const void*)k_angular_fp64<16>, optin);
+  e = cudaDeviceGetAttribute(&g_angular_sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  e = set_max_dynamic_smem((const void*)k_angular_fp64<TR>, optin);
-  if (e != cudaSuccess) return e;
+  switch (((n_l_max + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS) {   // groups of fewer row tiles too
+    default: e = configure_angular_rows<4>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
+    case 3: e = configure_angular_rows<3>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
+    case 2: e = configure_angular_rows<2>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
+    case 1: e = configure_angular_rows<1>(optin); if (e != cudaSuccess) return e;
+  }
   e = configure_radial_fp64();
   if (e != cudaSuccess) return e;
-  return set_max_dynamic_smem((const void*)k_finalize, optin);
+  e = set_max_dynamic_smem((const void*)k_finalize<true>, optin);
+  if (e != cudaSuccess) return e;
+  return set_max_dynamic_smem((const void*)k_finalize<false>, optin);
 }
 
 }  // namespace ggb

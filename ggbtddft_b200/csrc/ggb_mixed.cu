@@ -797,7 +797,7 @@ static void angular_half(MixedGroup& m, const GroupArgs& a, int half, cudaStream
       int8_slice_x(m, a, m.Xd, s);
     } else {
       // also the density and dipole partial sums
-      if (m.angular_fp64) launch_angular_fp64(a, 1, m.Yd, m.Xd, 1, s);
+      if (m.angular_fp64) launch_angular_fp64(a, 1, m.Yd, m.Xd, a.n_den > 0, s);
       else int8_angular(m, a, 1, m.Yd, m.Xd, s);
     }
     return;
