@@ -458,7 +458,8 @@ static int prepare(ggb_ctx* ctx) {
     a.fin_cnt = g.fin_cnt_d; a.fin_scr = g.fin_scr_d;
     int max_orb = 0;
     for (int ri : g.runs) max_orb = std::max(max_orb, ctx->runs[ri].d.n_orb);
-    a.fin_ob = obs_source(ctx, g) ? std::min(FIN_OB_ROWS, (n_l * max_orb + 7) / 8) : FIN_OB;
+    a.fin_ob = std::min(FIN_OB, ((n_l + 1) * max_orb + 7) / 8);
+    a.obs_parts = ctx->dims.precision == GGB_SPLIT_INT8 ? 1 : 2;
     // the int8 form's initial density is summed over the lane groups of its own tiles (4 of 32 radii,
     // 8 of 16), so that its potentials do not depend on the FP64 kernel's tile
     a.den_groups = ctx->dims.precision == GGB_SPLIT_INT8 ? 128 / g.obs_seg : 0;
@@ -604,7 +605,7 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
     if ((rc = dalloc(ctx, &g.r_d, nr)) || (rc = dalloc(ctx, &g.drdx_d, nr)) || (rc = dalloc(ctx, &g.P_d, nr)) ||
         (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (dims->precision != GGB_FP64 && (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles))) ||
         (rc = dalloc(ctx, &g.step_d, 1)) || (rc = dalloc(ctx, &g.done_d, 1)) ||
-        (rc = dalloc(ctx, &g.fin_cnt_d, g.runs.size())) || (rc = dalloc(ctx, &g.fin_scr_d, nc * std::max<size_t>(FIN_OB * 8, nl * 10))) ||
+        (rc = dalloc(ctx, &g.fin_cnt_d, g.runs.size())) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
         (rc = dalloc(ctx, &g.col_run_d, nc)) || (rc = dalloc(ctx, &g.col_m_d, nc)) ||
         (rc = dalloc(ctx, &g.col_occ_d, nc)) || (rc = dalloc(ctx, &g.runs_d, g.runs.size())))
       return bad(rc, "alloc");

@@ -870,9 +870,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
             sw += xl.x * z2.y - xl.y * z2.x;
           }
         }
-        double4* o = g.obs + 2 * (((size_t)col * n_l + l) * g.n_tiles + r0 / NP);
-        o[0] = make_double4(sx, sy, sz, sw);
-        o[1] = make_double4(0.0, 0.0, 0.0, 0.0);
+        g.obs[((size_t)col * n_l + l) * g.n_tiles + r0 / NP] = make_double4(sx, sy, sz, sw);
       }
       // density multipoles: every lane works (point lane % NP), the literal l loops strided over the
       // NG lane groups, then the groups summed in order

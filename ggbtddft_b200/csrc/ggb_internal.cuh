@@ -11,8 +11,8 @@
 //   dph      angular eigenvalues D[c][m][j], [4][N_m][ldS].
 //   coef     angular coefficient tables [COEF_N][N_m][N_l] (cu, cd, p, qu, qd, p3lm, f3lm).
 //   dens     density partials per column [n_cols][4][N_r] (not yet occupation weighted).
-//   obs      dipole/acceleration partials per column, l and r-tile [n_cols][N_l][n_tiles][2] double4
-//            (double-double: high parts, then low parts).
+//   obs      dipole/acceleration partials per column, l and r-tile [n_cols][N_l][n_tiles][obs_parts] double4
+//            (obs_parts = 2: high parts, then low parts).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -23,8 +23,7 @@ constexpr int TR = 32;            // radii per angular tile (one warp-width, coa
 constexpr int ANG_WARPS = 8;      // warps per angular CTA
 constexpr int MAX_NL = 220;       // largest N_l: two [N_l][32] complex128 tiles fit in 227 KB of shared memory
 constexpr int MAX_NR = 8192;      // largest N_r: three [N_r] FP64 rows of the potentials kernel
-constexpr int FIN_OB = 32;         // observables blocks per run in k_finalize: slices of l, from partials
-constexpr int FIN_OB_ROWS = 148;   // ... at most, from the orbitals (8 rows (l, orbital) per block and round)
+constexpr int FIN_OB = 148;        // observables blocks per run in k_finalize, at most (8 rows (l, orbital) each)
 constexpr int N_DEN = 4;          // density multipoles carried per column (L = 0..3)
 
 // status bits (sticky, OR-ed on the device)
@@ -90,6 +89,7 @@ struct GroupArgs {
   double n_g_fac;   // N_g (N_g + 1) / 2
   double norm_tol;
   int obs_seg;      // radii per observables partial sum (32; 16 for the int8 form when N_l > 128)  // relative growth of an orbital norm above its initial value that raises ST_NORM_GROWTH
+  int obs_parts;    // entries of g.obs per partial: 1, or 2 (high and low parts)
   const double* r;
   const double* drdx;
   const double* P;
@@ -110,7 +110,7 @@ struct GroupArgs {
   int fin_ob;               // observables blocks per run
   int den_groups;           // lane groups of the FP64 angular kernel's density sums (0: as many as fit)
   unsigned* fin_cnt;        // [n_runs] finished observables blocks of the step (last-block totals)
-  double* fin_scr;          // [n_cols][FIN_OB][8] slice or [n_cols][N_l][10] row totals of the observables (double-double)
+  double* fin_scr;          // [n_cols][N_l + 1][5] row sums of the observables (hi, lo); row N_l: the norm
   Chain chain[3];   // first half, second half, empty (initial partials)
 };
 
@@ -148,6 +148,23 @@ __device__ __forceinline__ dd dd_add(dd a, dd b) {
   e += a.lo + b.lo;
   double h = s + e;
   return dd{h, e - (h - s)};
+}
+// Cascaded summation (Ogita, Rump and Oishi's Sum2): hi is the plain sum, lo collects its exact rounding
+// errors.  As accurate as the normalised pair above for sums of a few thousand terms, with one addition
+// per term on the dependency chain instead of seven.
+__device__ __forceinline__ void sum2_add(dd& a, double b) {
+  const double s = a.hi + b, bp = s - a.hi;
+  a.lo += (a.hi - (s - bp)) + (b - bp);
+  a.hi = s;
+}
+__device__ __forceinline__ void sum2_add(dd& a, dd b) {
+  sum2_add(a, b.hi);
+  a.lo += b.lo;
+}
+__device__ __forceinline__ void sum2_warp(dd& a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    sum2_add(a, dd{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
 }
 __device__ __forceinline__ dd dd_shfl_up(dd a, int d) {
   return dd{__shfl_up_sync(0xffffffffu, a.hi, d), __shfl_up_sync(0xffffffffu, a.lo, d)};

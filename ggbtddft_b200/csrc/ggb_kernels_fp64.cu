@@ -803,15 +803,6 @@ __device__ void block_scan_dd(const double* t, double* out, int n, bool backward
   __syncthreads();
 }
 
-__device__ __forceinline__ dd warp_sum_dd2(dd a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const dd b{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-    a = dd_add(a, b);
-  }
-  return a;
-}
-
 __device__ __forceinline__ double ipow(double x, int L) {
   double p = 1.0;
   for (int i = 0; i < L; ++i) p *= x;
@@ -832,7 +823,7 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
   const double c_d = down ? g.coef[((size_t)CF_CD * g.n_m + m) * n_l + l] : 0.0;
   const size_t ls = (size_t)g.n_cols * n_r;
   const double2* row = x + (size_t)l * ls + (size_t)col * n_r;
-#pragma unroll 2
+#pragma unroll 4
   for (int i = lane; i < n_r; i += 32) {
     const double2 xl = row[i];
     const double2 xu = up ? row[ls + i] : make_double2(0.0, 0.0);
@@ -840,14 +831,14 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
     const double rr = g.r[i], fr2 = 1.0 / (rr * rr);
     const double zx = c_u * xu.x + c_d * xd.x, zy = c_u * xu.y + c_d * xd.y;
     const double px = xl.x * zx + xl.y * zy, py = xl.x * zy - xl.y * zx;   // conj(x_l) . z
-    s[0] = dd_add(s[0], dd{rr * px, 0.0});
-    s[1] = dd_add(s[1], dd{rr * py, 0.0});
-    s[2] = dd_add(s[2], dd{fr2 * px, 0.0});
-    s[3] = dd_add(s[3], dd{fr2 * py, 0.0});
-    s[4] = dd_add(s[4], dd{xl.x * xl.x + xl.y * xl.y, 0.0});
+    sum2_add(s[0], rr * px);
+    sum2_add(s[1], rr * py);
+    sum2_add(s[2], fr2 * px);
+    sum2_add(s[3], fr2 * py);
+    sum2_add(s[4], xl.x * xl.x + xl.y * xl.y);
   }
 #pragma unroll
-  for (int q = 0; q < 5; ++q) s[q] = warp_sum_dd2(s[q]);
+  for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
 }
 
 // Blocks: for each run of the group, n_den Hartree blocks (L = 0..n_den-1; block L = 0 also does
@@ -855,14 +846,16 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
 // no step increment), mode 1 = end of step, mode 2 = end of step without the step increment and the
 // watchdog checks (the per-phase timing).
 //
-// Observables, from the orbitals (ROWS: the FP64 angular kernel): one warp per (l, orbital) row of the
-// run, straight from L2 where the orbitals of a run still are (the angular kernel's tiles summed them
+// Observables: one warp per row (l, orbital) of the run.  ROWS (the FP64 angular kernel): from the
+// orbitals, straight from L2 where those of a run still are (the angular kernel's tiles summed them
 // before: a double-double warp reduction of every row for every 16 radii, 8 us of its second half for
-// one column on 200 radii and 25 us for nine on 600).  From the partials of the int8 and BF16 angular
-// kernels: observables block ob sums the partials of a slice of l (one warp per orbital, lanes
-// striding over the tiles, double-double).  Either way the per-l series are written, the rows' or
-// slices' totals go to a scratch row, and the last of the run's blocks to finish (a per-run counter)
-// adds them, writes the totals and the norm and runs the NaN / norm-growth watchdog.
+// one column on 200 radii and 25 us for nine on 600).  Otherwise from the partial sums per tile of
+// radii that the int8 and BF16 angular kernels leave (an eighth of the orbitals' bytes: the orbitals
+// of an ensemble are not in L2), with one more row per orbital for the norm, from the density.  The
+// rows' sums go to a scratch array, and the last of the run's blocks to finish (a per-run counter) adds
+// them over l, writes the totals and runs the NaN / norm-growth watchdog.  (Blocks that took a slice of
+// l with one warp per orbital walked its rows one after another: 27 us for nine orbitals, N_l 97, and
+// 88 us for 21 such runs at N_l 161, now 14 and 47 us.)
 // ROWS: the observables come from the orbitals x (the partial sums' kernel needs half its registers).
 template <bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
@@ -882,47 +875,43 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
 
   if (obs_block && mode != 0 && step >= run.n_t) {
     if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);
-  } else if (obs_block && (mode != 0 || ROWS)) {
+  } else if (obs_block) {
     const int n_orb = run.n_orb;
-    if constexpr (ROWS) {
-      for (int i = ob * (FIN_THREADS / 32) + warp; i < n_l * n_orb; i += g.fin_ob * (FIN_THREADS / 32)) {
-        const int l = i / n_orb, k = i - l * n_orb;
-        dd s[5];
+    double2* scr = reinterpret_cast<double2*>(g.fin_scr);     // [col][N_l + 1][5]; row N_l: the norm
+    const int rows = n_l * n_orb + (ROWS ? 0 : n_orb);
+    for (int i = ob * (FIN_THREADS / 32) + warp; i < rows; i += g.fin_ob * (FIN_THREADS / 32)) {
+      const int l = i / n_orb, k = i - l * n_orb;
+      dd s[5];
+      if constexpr (ROWS) {
         observe_row(g, x, run.col0 + k, l, lane, s);
-        if (lane == 0) {
-          if (mode != 0 && g.per_l) {
-            run.dip[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
-            run.acc[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
-          }
-          double2* o = reinterpret_cast<double2*>(g.fin_scr) + ((size_t)(run.col0 + k) * n_l + l) * 5;
+      } else {
 #pragma unroll
-          for (int q = 0; q < 5; ++q) o[q] = make_double2(s[q].hi, s[q].lo);
+        for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
+        if (l == n_l) {
+          const double* dn = g.dens + (size_t)(run.col0 + k) * N_DEN * n_r;  // L = 0 row
+          for (int q = lane; q < n_r; q += 32) sum2_add(s[4], dn[q]);
+          sum2_warp(s[4]);
+        } else {
+          const double4* p = g.obs + ((size_t)(run.col0 + k) * n_l + l) * g.n_tiles * g.obs_parts;
+          for (int t = lane; t < g.n_tiles * g.obs_parts; t += 32) {   // low parts are terms like the others
+            const double4 h = p[t];
+            sum2_add(s[0], h.x);
+            sum2_add(s[1], h.y);
+            sum2_add(s[2], h.z);
+            sum2_add(s[3], h.w);
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum2_warp(s[q]);
         }
       }
-    } else {
-      const int l0 = ob * n_l / g.fin_ob, l1 = (ob + 1) * n_l / g.fin_ob;
-      for (int k = warp; k < n_orb; k += FIN_THREADS / 32) {
-        dd tx{0.0, 0.0}, ty{0.0, 0.0}, tz{0.0, 0.0}, tw{0.0, 0.0};
-        for (int l = l0; l < l1; ++l) {
-          const double4* p = g.obs + 2 * (((size_t)(run.col0 + k) * n_l + l) * g.n_tiles);
-          dd sx{0.0, 0.0}, sy{0.0, 0.0}, sz{0.0, 0.0}, sw{0.0, 0.0};
-          for (int t = lane; t < g.n_tiles; t += 32) {
-            const double4 h = p[2 * t], lo = p[2 * t + 1];
-            sx = dd_add(sx, dd{h.x, lo.x}); sy = dd_add(sy, dd{h.y, lo.y});
-            sz = dd_add(sz, dd{h.z, lo.z}); sw = dd_add(sw, dd{h.w, lo.w});
-          }
-          sx = warp_sum_dd2(sx); sy = warp_sum_dd2(sy); sz = warp_sum_dd2(sz); sw = warp_sum_dd2(sw);
-          if (lane == 0 && g.per_l) {
-            run.dip[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(sx.hi + sx.lo, sy.hi + sy.lo);
-            run.acc[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(sz.hi + sz.lo, sw.hi + sw.lo);
-          }
-          tx = dd_add(tx, sx); ty = dd_add(ty, sy); tz = dd_add(tz, sz); tw = dd_add(tw, sw);
+      if (lane == 0) {
+        if (mode != 0 && g.per_l && l < n_l) {
+          run.dip[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
+          run.acc[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
         }
-        if (lane == 0) {
-          double* o = g.fin_scr + ((size_t)(run.col0 + k) * FIN_OB + ob) * 8;
-          o[0] = tx.hi; o[1] = tx.lo; o[2] = ty.hi; o[3] = ty.lo;
-          o[4] = tz.hi; o[5] = tz.lo; o[6] = tw.hi; o[7] = tw.lo;
-        }
+        double2* o = scr + ((size_t)(run.col0 + k) * (n_l + 1) + l) * 5;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) o[q] = make_double2(s[q].hi, s[q].lo);
       }
     }
     __syncthreads();
@@ -938,26 +927,15 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
         dd s[5];
 #pragma unroll
         for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
-        if constexpr (ROWS) {
-          const double2* o = reinterpret_cast<const double2*>(g.fin_scr) + (size_t)(run.col0 + k) * n_l * 5;
-          for (int l = lane; l < n_l; l += 32)
+        const double2* o = scr + (size_t)(run.col0 + k) * (n_l + 1) * 5;
+        for (int l = lane; l < n_l + (ROWS ? 0 : 1); l += 32)
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
-              const double2 v = __ldcg(o + (size_t)l * 5 + q);
-              s[q] = dd_add(s[q], dd{v.x, v.y});
-            }
-#pragma unroll
-          for (int q = 0; q < 5; ++q) s[q] = warp_sum_dd2(s[q]);
-        } else {
-          for (int b = 0; b < g.fin_ob; ++b) {      // the slices in order
-            const double* o = g.fin_scr + ((size_t)(run.col0 + k) * FIN_OB + b) * 8;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) s[q] = dd_add(s[q], dd{__ldcg(o + 2 * q), __ldcg(o + 2 * q + 1)});
+          for (int q = 0; q < 5; ++q) {
+            const double2 v = __ldcg(o + (size_t)l * 5 + q);
+            sum2_add(s[q], dd{v.x, v.y});
           }
-          const double* dn = g.dens + (size_t)(run.col0 + k) * N_DEN * n_r;  // L = 0 row
-          for (int q = lane; q < n_r; q += 32) s[4] = dd_add(s[4], dd{dn[q], 0.0});
-          s[4] = warp_sum_dd2(s[4]);
-        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
         const double nrm = s[4].hi + s[4].lo;
         if (lane == 0 && mode == 0) run.norm0[k] = nrm;   // for the growth watchdog
         if (lane == 0 && mode != 0) {
@@ -971,15 +949,6 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
         }
       }
       if (tid == 0) g.fin_cnt[ri] = 0u;   // for the next launch (stream-ordered after this one)
-    }
-  } else if (obs_block && mode == 0 && ob == 0) {
-    // initial norm for the growth watchdog
-    for (int k = warp; k < run.n_orb; k += FIN_THREADS / 32) {
-      const double* dn = g.dens + (size_t)(run.col0 + k) * N_DEN * n_r;
-      dd nd{0.0, 0.0};
-      for (int q = lane; q < n_r; q += 32) nd = dd_add(nd, dd{dn[q], 0.0});
-      nd = warp_sum_dd2(nd);
-      if (lane == 0) run.norm0[k] = nd.hi + nd.lo;
     }
   }
 
