@@ -47,6 +47,8 @@ struct GroupHost {
   bool needs_init = true;
   GroupArgs args{};
   ThetaArgs theta_args{};        // theta form with n_har > 4 (ggb_theta.cu)
+  cudaStream_t branch = nullptr; // its second branch of a step, forked from and joined to the group's stream
+  cudaEvent_t branch_ev[2] = {nullptr, nullptr};
   MixedGroup mixed;              // split-precision form (ggb_mixed.cu)
   // flags shared by the runs of the group
   int n_har = 0, use_hartree = 0, target_id = 0, theta = 0;
@@ -289,9 +291,9 @@ static int prepare_theta_tables(ggb_ctx* ctx, GroupHost& g, int n_mp) {
       long double c2 = 0.5L;
       for (int k = 1; k <= m; ++k) c2 *= (2.0L * k + 1.0L) * (2.0L * k) / (4.0L * k * k);
       long double tm1 = 0.0L, t0 = std::sqrt(c2) * std::pow(1.0L - z * z, 0.5L * m);
-      double* row = T.data() + ((size_t)m * nq + q) * n_l;
+      double* node = T.data() + (size_t)m * n_l * nq + q;
       for (int l = m; l < n_l; ++l) {
-        row[l] = (double)t0;
+        node[(size_t)l * nq] = (double)t0;
         if (l + 1 < n_l) {
           const long double t1 = (z * t0 - (l > m ? (long double)h_cd(l, m) * tm1 : 0.0L)) / (long double)h_cu(l, m);
           tm1 = t0;
@@ -303,7 +305,7 @@ static int prepare_theta_tables(ggb_ctx* ctx, GroupHost& g, int n_mp) {
     long double p0 = 1.0L, p1 = xq[q];
     for (int L = 0; L < n_mp; ++L) {
       const long double pl = L == 0 ? 1.0L : p1;
-      wP[(size_t)L * nq + q] = (double)(wq[q] * pl);
+      wP[(size_t)q * n_mp + L] = (double)(wq[q] * pl);
       if (L >= 1) {
         const long double p2 = ((2.0L * L + 1.0L) * xq[q] * p1 - L * p0) / (L + 1.0L);
         p0 = p1;
@@ -333,18 +335,18 @@ static int prepare_theta_tables(ggb_ctx* ctx, GroupHost& g, int n_mp) {
   ThetaArgs& t = g.theta_args;
   t.n_mp = n_mp;
   t.nq = nq;
-  double *Td, *wPd, *PLd, *rqd, *fine, *rho, *vmp;
+  double *Td, *wPd, *PLd, *rqd, *rho, *vmp;
   int rc;
   const size_t nrun = g.runs.size();
   if ((rc = dalloc(ctx, &Td, T.size())) || (rc = dalloc(ctx, &wPd, wP.size())) || (rc = dalloc(ctx, &PLd, PLj.size())) ||
-      (rc = dalloc(ctx, &rqd, rq.size())) || (rc = dalloc(ctx, &fine, nrun * 2 * nq * n_r)) ||
+      (rc = dalloc(ctx, &rqd, rq.size())) ||
       (rc = dalloc(ctx, &rho, nrun * n_mp * n_r)) || (rc = dalloc(ctx, &vmp, nrun * n_mp * n_r)))
     return rc;
   CK(cudaMemcpy(Td, T.data(), T.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(wPd, wP.data(), wP.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(PLd, PLj.data(), PLj.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(rqd, rq.data(), rq.size() * sizeof(double), cudaMemcpyHostToDevice));
-  t.T = Td; t.wP = wPd; t.PLj = PLd; t.rq = rqd; t.fine = fine; t.rho = rho; t.vmp = vmp;
+  t.T = Td; t.wP = wPd; t.PLj = PLd; t.rq = rqd; t.rho = rho; t.vmp = vmp;
   for (int ri : g.runs) {
     RunHost& r = ctx->runs[ri];
     if ((rc = dalloc(ctx, &r.htab_d, (size_t)n_m * n_l * n_r))) return rc;
@@ -494,14 +496,28 @@ static void launch_group_step(ggb_ctx* ctx, GroupHost& g, cudaStream_t s) {
   } else {
     mixed_step(g.mixed, a, s);
   }
-  if (a.theta_tab) launch_theta_potentials(a, g.theta_args, g.x_d, s);
-  launch_finalize(a, obs_source(ctx, g), 1, s);
+  if (a.theta_tab) {
+    // the exact multipoles and k_finalize read the same orbitals and share no buffer: two branches
+    cudaEventRecord(g.branch_ev[0], s);
+    cudaStreamWaitEvent(g.branch, g.branch_ev[0], 0);
+    launch_finalize(a, obs_source(ctx, g), 1, g.branch);
+    cudaEventRecord(g.branch_ev[1], g.branch);
+    launch_theta_potentials(a, g.theta_args, g.x_d, s);
+    cudaStreamWaitEvent(s, g.branch_ev[1], 0);
+  } else {
+    launch_finalize(a, obs_source(ctx, g), 1, s);
+  }
 }
 
 // n steps of every group.  With several groups, each group's steps go to its own stream, forked
 // from and joined back to s by events (inside a graph capture this becomes parallel branches).
 static int launch_steps(ggb_ctx* ctx, cudaStream_t s, int n) {
   if (n <= 0) return GGB_OK;
+  for (GroupHost& g : ctx->groups)
+    if (g.args.theta_tab && !g.branch) {
+      CK(cudaStreamCreateWithFlags(&g.branch, cudaStreamNonBlocking));
+      for (cudaEvent_t& e : g.branch_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
   if (ctx->groups.size() == 1) {
     for (int i = 0; i < n; ++i) launch_group_step(ctx, ctx->groups[0], s);
     return GGB_OK;
@@ -923,7 +939,12 @@ void ggb_destroy(ggb_ctx* ctx) {
   for (cudaStream_t gs : ctx->group_streams) cudaStreamDestroy(gs);
   for (cudaEvent_t e : ctx->group_done) cudaEventDestroy(e);
   if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
-  for (GroupHost& g : ctx->groups) mixed_release(g.mixed);
+  for (GroupHost& g : ctx->groups) {
+    if (g.branch) cudaStreamDestroy(g.branch);
+    for (cudaEvent_t e : g.branch_ev)
+      if (e) cudaEventDestroy(e);
+    mixed_release(g.mixed);
+  }
   for (void* p : ctx->allocs) cudaFree(p);
   delete ctx;
 }

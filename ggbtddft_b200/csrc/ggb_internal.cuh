@@ -120,14 +120,14 @@ struct GroupArgs {
 struct ThetaArgs {
   int n_mp;            // multipoles L = 0 .. n_mp-1 (<= 2 N_l - 1)
   int nq;              // positive fine nodes (= N_l)
-  const double* T;     // [N_m][nq][N_l]  Theta_l^m(x_q)
-  const double* wP;    // [n_mp][nq]      w_q P_L(x_q)
+  const double* T;     // [N_m][N_l][nq]  Theta_l^m(x_q)
+  const double* wP;    // [nq][n_mp]      w_q P_L(x_q)
   const double* PLj;   // [N_m][n_mp][ldS] P_L(x_j^m) at the P coupling's nodes
   const double* rq;    // [n_mp+1][N_r]   (r_(a-1) / r_a)^L for a >= 1, 0 at a = 0
-  double* fine;        // [n_runs][2][nq][N_r]  S_q = sum occ 2(|E|^2 + |O|^2), D_q = sum occ 4 Re(E conj O)
   double* rho;         // [n_runs][n_mp][N_r]
   double* vmp;         // [n_runs][n_mp][N_r]
 };
+cudaError_t configure_theta(int optin);
 void launch_theta_potentials(const GroupArgs& g, const ThetaArgs& t, const double2* x, cudaStream_t s);
 
 __device__ __forceinline__ double2 cmul_conj_phase(double2 x, double eta) {

@@ -751,53 +751,64 @@ static cudaError_t configure_radial_fp64() {
 
 constexpr int FIN_THREADS = 256;
 
-// Inclusive (forward) or suffix-exclusive (backward) compensated scan of t[0..n) in shared memory.
-// forward:  out[a] = sum_{b <= a} t[b]      backward: out[a] = sum_{b > a} t[b]
-__device__ void block_scan_dd(const double* t, double* out, int n, bool backward, dd* wsum) {
+// Compensated scans of two rows in shared memory, in place and side by side (one chain of latencies):
+// F[a] <- sum_{b <= a} F[b] (inclusive), G[a] <- sum_{b > a} G[b] (suffix, exclusive).
+__device__ void block_scans_dd(double* F, double* G, int n, dd (*wsum)[2]) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = FIN_THREADS / 32;
   const int per = (n + FIN_THREADS - 1) / FIN_THREADS;
   const int b0 = tid * per;
   // local inclusive sums in the scan direction
-  dd loc{0.0, 0.0};
-  for (int q = 0; q < per; ++q) {
-    const int k = b0 + q;
-    if (k < n) loc = dd_add(loc, dd{t[backward ? n - 1 - k : k], 0.0});
-  }
-  // warp inclusive scan of thread totals
-  dd inc = loc;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    dd o = dd_shfl_up(inc, d);
-    if (lane >= d) inc = dd_add(o, inc);
-  }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    dd w = lane < nw ? wsum[lane] : dd{0.0, 0.0};
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      dd o = dd_shfl_up(w, d);
-      if (lane >= d) w = dd_add(o, w);
-    }
-    if (lane < nw) wsum[lane] = w;
-  }
-  __syncthreads();
-  // exclusive prefix of this thread = inclusive value of the previous lane + earlier warps
-  const dd prev = dd_shfl_up(inc, 1);
-  dd run = lane == 0 ? dd{0.0, 0.0} : prev;
-  if (warp > 0) run = dd_add(wsum[warp - 1], run);
+  dd loc[2] = {{0.0, 0.0}, {0.0, 0.0}};
   for (int q = 0; q < per; ++q) {
     const int k = b0 + q;
     if (k < n) {
-      const int idx = backward ? n - 1 - k : k;
-      const double tv = t[idx];
-      if (backward) {
-        out[idx] = run.hi + run.lo;                 // exclusive (sum over b > a)
-        run = dd_add(run, dd{tv, 0.0});
-      } else {
-        run = dd_add(run, dd{tv, 0.0});
-        out[idx] = run.hi + run.lo;                 // inclusive (sum over b <= a)
+      loc[0] = dd_add(loc[0], dd{F[k], 0.0});
+      loc[1] = dd_add(loc[1], dd{G[n - 1 - k], 0.0});
+    }
+  }
+  // warp inclusive scan of thread totals
+  dd inc[2] = {loc[0], loc[1]};
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const dd o = dd_shfl_up(inc[c], d);
+      if (lane >= d) inc[c] = dd_add(o, inc[c]);
+    }
+  if (lane == 31) {
+    wsum[warp][0] = inc[0];
+    wsum[warp][1] = inc[1];
+  }
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      dd w = lane < nw ? wsum[lane][c] : dd{0.0, 0.0};
+#pragma unroll
+      for (int d = 1; d < nw; d <<= 1) {
+        const dd o = dd_shfl_up(w, d);
+        if (lane >= d) w = dd_add(o, w);
       }
+      if (lane < nw) wsum[lane][c] = w;
+    }
+  }
+  __syncthreads();
+  // exclusive prefix of this thread = inclusive value of the previous lane + earlier warps
+  dd run[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const dd prev = dd_shfl_up(inc[c], 1);
+    run[c] = lane == 0 ? dd{0.0, 0.0} : prev;
+    if (warp > 0) run[c] = dd_add(wsum[warp - 1][c], run[c]);
+  }
+  for (int q = 0; q < per; ++q) {
+    const int k = b0 + q;
+    if (k < n) {
+      run[0] = dd_add(run[0], dd{F[k], 0.0});
+      F[k] = run[0].hi + run[0].lo;                 // inclusive (sum over b <= a)
+      const double tv = G[n - 1 - k];
+      G[n - 1 - k] = run[1].hi + run[1].lo;         // exclusive (sum over b > a)
+      run[1] = dd_add(run[1], dd{tv, 0.0});
     }
   }
   __syncthreads();
@@ -841,8 +852,14 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
   for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
 }
 
-// Blocks: for each run of the group, n_den Hartree blocks (L = 0..n_den-1; block L = 0 also does
-// the exchange potential) + g.fin_ob observables blocks.  mode 0 = initial potentials (no observables,
+// exchange blocks per run: one radius per thread; without Hartree the density is the frozen one, and
+// the potential stays what mode 0 wrote
+__host__ __device__ inline int fin_xc_blocks(const GroupArgs& g, int mode) {
+  return (g.n_den > 0 || mode == 0) ? (g.n_r + FIN_THREADS - 1) / FIN_THREADS : 0;
+}
+
+// Blocks: for each run of the group, n_den Hartree blocks (L = 0..n_den-1), the exchange blocks and
+// g.fin_ob observables blocks.  mode 0 = initial potentials (no observables,
 // no step increment), mode 1 = end of step, mode 2 = end of step without the step increment and the
 // watchdog checks (the per-phase timing).
 //
@@ -859,19 +876,31 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
 // ROWS: the observables come from the orbitals x (the partial sums' kernel needs half its registers).
 template <bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
-  extern __shared__ double fsm[];  // [3][N_r]
-  __shared__ dd wsum[FIN_THREADS / 32];
-  __shared__ int s_last;
-  const int nb = g.n_den + g.fin_ob;
+  extern __shared__ double fsm[];  // [2][N_r]
+  __shared__ dd wsum[FIN_THREADS / 32][2];
+  __shared__ int s_last, s_step;
+  const int n_xc = fin_xc_blocks(g, mode);
+  const int nb = g.n_den + n_xc + g.fin_ob;
   const int ri = blockIdx.x / nb;
-  const int role = blockIdx.x - ri * nb;  // < n_den: Hartree L = role; >= n_den: observables slice
-  const int run_idx = g.runs_of_group[ri];
-  RunDev run = g.runs[run_idx];
+  const int role = blockIdx.x - ri * nb;  // Hartree L = role, then exchange, then observables blocks
+  const RunDev run = g.runs[g.runs_of_group[ri]];
   const int n_r = g.n_r, n_l = g.n_l, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int step = *g.step;
-  const bool obs_block = role >= g.n_den;
-  const int ob = role - g.n_den;
+  const bool obs_block = role >= g.n_den + n_xc;
+  const int ob = role - g.n_den - n_xc;
+  // the step counter advances once every block has read it
+  if (tid == 0) {
+    s_step = *g.step;
+    if (mode == 1) {
+      __threadfence();
+      if (atomicAdd(g.done, 1u) == gridDim.x - 1) {
+        *g.done = 0u;
+        *g.step = s_step + 1;
+      }
+    }
+  }
+  __syncthreads();
+  const int step = s_step;
 
   if (obs_block && mode != 0 && step >= run.n_t) {
     if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);
@@ -952,28 +981,26 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
     }
   }
 
-  if (!obs_block) {
+  // rho_L(r) = sum_kso occ * density_kso (hartreePotentialDensity.cuh:58-60, orbital order)
+  auto multipole = [&](int L, int q) {
+    double s = 0.0;
+    for (int k = 0; k < run.n_orb; ++k)
+      s += (double)g.col_occ[run.col0 + k] * g.dens[((size_t)(run.col0 + k) * N_DEN + L) * n_r + q];
+    return s;
+  };
+
+  if (role < g.n_den) {
     const int L = role;
-    double* rho = fsm;            // [N_r]
-    double* F = fsm + n_r;        // forward partial sums
-    double* G = fsm + 2 * n_r;    // backward partial sums
-    // rho_L(r) = sum_kso occ * density_kso (hartreePotentialDensity.cuh:58-60, orbital order)
-    for (int q = tid; q < n_r; q += FIN_THREADS) {
-      double s = 0.0;
-      for (int k = 0; k < run.n_orb; ++k)
-        s += (double)g.col_occ[run.col0 + k] * g.dens[((size_t)(run.col0 + k) * N_DEN + L) * n_r + q];
-      rho[q] = s;
-    }
-    __syncthreads();
+    double* F = fsm;              // [N_r] forward partial sums
+    double* G = fsm + n_r;        // backward partial sums
     // v_L(r_a) = r_a^-(L+1) sum_{b<=a} rho(b) r_b^L + r_a^L sum_{b>a} rho(b) r_b^-(L+1)
     for (int q = tid; q < n_r; q += FIN_THREADS) {
-      const double rb = g.r[q];
-      F[q] = rho[q] * ipow(rb, L);
-      G[q] = rho[q] / ipow(rb, L + 1);
+      const double rb = g.r[q], rho = multipole(L, q);
+      F[q] = rho * ipow(rb, L);
+      G[q] = rho / ipow(rb, L + 1);
     }
     __syncthreads();
-    block_scan_dd(F, F, n_r, false, wsum);
-    block_scan_dd(G, G, n_r, true, wsum);
+    block_scans_dd(F, G, n_r, wsum);
     for (int q = tid; q < n_r; q += FIN_THREADS) {
       const double ra = g.r[q];
       const double v = F[q] / ipow(ra, L + 1) + ipow(ra, L) * G[q];
@@ -982,14 +1009,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
     }
   }
 
-  // exchange (block L = 0, or the first observables block when Hartree is off)
-  // without Hartree the density is the frozen one: the potential stays what mode 0 wrote
-  const bool xc_block = (g.n_den > 0) ? (role == 0) : (ob == 0 && mode == 0);
-  if (xc_block) {
+  if (role >= g.n_den && !obs_block) {
     const bool pw92 = (run.flags & RUN_FLAG_PW92) != 0;
-    for (int q = tid; q < n_r; q += FIN_THREADS) {
-      double rho0 = 0.0;
-      if (g.n_den > 0) rho0 = fsm[q];
+    const int q = (role - g.n_den) * FIN_THREADS + tid;
+    if (q < n_r) {
+      const double rho0 = g.n_den > 0 ? multipole(0, q) : 0.0;
       // h_calculateExchangeCorrelationPotential.cuh:33-44
       double den = g.n_g_fac * (rho0 / 4.0 / M_PI + run.rho_frozen[q]) / g.drdx[q] * pow(g.P[q], 2.0);
       const double rq = g.r[q];
@@ -1026,26 +1050,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
       run.vexc[q] = (run.flags & RUN_FLAG_XC_FROZEN) ? run.vexc0[q] : vx;
     }
   }
-
-  // last block of a step advances the shared step counter
-  if (mode == 1) {
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      const unsigned total = gridDim.x;
-      const unsigned prev = atomicAdd(g.done, 1u);
-      if (prev == total - 1) {
-        *g.done = 0u;
-        __threadfence();
-        atomicAdd(g.step, 1);
-      }
-    }
-  }
 }
 
 void launch_finalize(const GroupArgs& g, const double2* x, int mode, cudaStream_t s) {
-  const dim3 grid(g.n_runs * (g.n_den + g.fin_ob)), block(FIN_THREADS);
-  const size_t smem = 3 * (size_t)g.n_r * sizeof(double);
+  const dim3 grid(g.n_runs * (g.n_den + fin_xc_blocks(g, mode) + g.fin_ob)), block(FIN_THREADS);
+  const size_t smem = g.n_den > 0 ? 2 * (size_t)g.n_r * sizeof(double) : 0;
   if (x) k_finalize<true><<<grid, block, smem, s>>>(g, x, mode);
   else k_finalize<false><<<grid, block, smem, s>>>(g, x, mode);
 }
@@ -1077,6 +1086,8 @@ cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max) {
     case 1: e = configure_angular_rows<1>(optin); if (e != cudaSuccess) return e;
   }
   e = configure_radial_fp64();
+  if (e != cudaSuccess) return e;
+  e = configure_theta(optin);
   if (e != cudaSuccess) return e;
   e = set_max_dynamic_smem((const void*)k_finalize<true>, optin);
   if (e != cudaSuccess) return e;

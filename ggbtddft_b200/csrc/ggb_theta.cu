@@ -4,12 +4,12 @@
 // h_calculateHartreePotential.cuh:1-56).
 //
 // Per run and step, from the orbitals x[l][col][r] at the end of the step:
-//  k_theta_fine     the density on a Gauss-Legendre grid of 2 N_l nodes +-x_q, exact for every
+//  k_theta_density  the density on a Gauss-Legendre grid of 2 N_l nodes +-x_q, exact for every
 //                   multipole up to 2 l_max: per orbital f(+-x_q) = E_q +- O_q with E (O) the sum over
 //                   l - m even (odd) of x_l Theta_l^m(x_q); summed over the run's orbitals,
 //                   S_q = sum occ 2 (|E|^2 + |O|^2) = rho(x_q) + rho(-x_q) and
-//                   D_q = sum occ 4 Re(E conj O)  = rho(x_q) - rho(-x_q).
-//  k_theta_project  rho_L(r) = sum_q w_q P_L(x_q) (S_q for even L, D_q for odd L).
+//                   D_q = sum occ 4 Re(E conj O)  = rho(x_q) - rho(-x_q);
+//                   then rho_L(r) = sum_q w_q P_L(x_q) (S_q for even L, D_q for odd L).
 //  k_theta_hartree  v_L(r_a) = sum_b rho_L(b) r_<^L / r_>^(L+1) as two linear recurrences with ratios
 //                   of radii (no power of r over- or underflows):
 //                     A_a = (r_(a-1)/r_a)^L A_(a-1) + rho_a,  B_a = (r_a/r_(a+1))^(L+1) (B_(a+1) + rho_(a+1)),
@@ -19,108 +19,133 @@
 //  k_theta_table    htab[m][j][r] = sum_{L>=1} v_L(r) P_L(x_j^m): the multipoles' potential at the
 //                   nodes of the angular phase (the monopole and exchange changes come from k_finalize
 //                   and enter the phase as in the theta form with n_har <= 4).
+// k_finalize runs beside them (they share no buffer): in the step's graph it is a parallel branch.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "ggb_internal.cuh"
 
 namespace ggb {
 
-constexpr int TH_THREADS = 256;
-constexpr int TH_WARPS = TH_THREADS / 32;
-constexpr int TH_QB = 2;          // fine nodes per warp
+// Blocks own TH_R radii: everything of those radii (the l-vectors, the densities at the nodes, the
+// potentials' multipoles) sits in shared memory, so that a single run (the helium configuration: 400
+// radii) is 100 blocks.  The tables come through shared memory too, TH_ROWS rows at a time into one of
+// two buffers by cp.async: all of a chunk's lines are in flight at once.  (Read from L2 in the loops,
+// eight loads ahead, the projection and the table waited a memory latency for every eight terms.)
+// Lanes: radius fastest, then eight nodes, multipoles or channels.  One output per thread and round.
+// Latency bound.  Helium configuration (N_r 400, N_l 65, 129 multipoles), with k_finalize beside them:
+// 27 us a step; as four kernels of a warp per (32 radii, node or multipole) that read every row
+// from L2, and k_finalize after them: 73.
+constexpr int TH_R = 4;
 constexpr int TH_ILP = 8;         // independent partial sums of the projection and table loops
+constexpr int TH_ROWS = 32;       // table rows per chunk (a multiple of TH_ILP)
 
 // pairwise sum of the partial sums
 __device__ __forceinline__ double sum_partials(const double (&a)[TH_ILP]) {
   return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
 }
 
-// Work split of the three density/potential kernels: a warp owns 32 radii and a few fine nodes
-// (k_theta_fine), one multipole (k_theta_project) or one node of the phase (k_theta_table), so that
-// a single run (the helium configuration: 13 tiles of 32 radii) still spreads over ~100 blocks; the
-// radii are the lanes, so every load of an orbital, a density or a potential row is coalesced.
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// blocks (run, 32 radii, TH_WARPS * TH_QB fine nodes): S and D of the run's orbitals at the block's
-// positive fine nodes, accumulated over the run's orbitals in order in registers
-__global__ void __launch_bounds__(TH_THREADS) k_theta_fine(GroupArgs g, ThetaArgs t, const double2* __restrict__ x) {
-  const int tiles = (g.n_r + 31) / 32;
-  const int nq = t.nq, n_l = g.n_l;
-  const int qsplit = (nq + TH_WARPS * TH_QB - 1) / (TH_WARPS * TH_QB);
-  const int ri = blockIdx.x / (tiles * qsplit);
-  const int rest = blockIdx.x - ri * tiles * qsplit;
-  const int tile = rest / qsplit, qs = rest - tile * qsplit;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = tile * 32 + lane;
-  const int q0 = (qs * TH_WARPS + warp) * TH_QB;
-  if (r >= g.n_r || q0 >= nq) return;
+// body(row0, n, rows in shared memory) for the chunks of `rows` table rows of `cols` doubles (row stride
+// ld in memory, cols in shared memory), the next chunk on its way meanwhile.  Every thread of the block
+// takes part; body must not synchronise the block.
+template <class Body>
+__device__ __forceinline__ void table_chunks(const double* table, int rows, int cols, int ld, double* buf, Body body) {
+  auto fetch = [&](int c) {
+    const int row0 = c * TH_ROWS, n = min(TH_ROWS, rows - row0);
+    double* dst = buf + (c & 1) * TH_ROWS * cols;
+    for (int i = threadIdx.x; i < n * cols; i += blockDim.x) {
+      const int row = i / cols, col = i - row * cols;
+      cp_async8(dst + i, table + (size_t)(row0 + row) * ld + col);
+    }
+    cp_async_commit();
+  };
+  const int chunks = (rows + TH_ROWS - 1) / TH_ROWS;
+  __syncthreads();                   // the buffers are free
+  if (chunks > 0) fetch(0);
+  for (int c = 0; c < chunks; ++c) {
+    if (c + 1 < chunks) fetch(c + 1);
+    else cp_async_commit();
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    body(c * TH_ROWS, min(TH_ROWS, rows - c * TH_ROWS), (const double*)(buf + (c & 1) * TH_ROWS * cols));
+    __syncthreads();
+  }
+}
+
+// S and D of the run's orbitals at the positive fine nodes, accumulated over the orbitals in order, then
+// the projections
+__global__ void __launch_bounds__(1024) k_theta_density(GroupArgs g, ThetaArgs t, const double2* __restrict__ x) {
+  extern __shared__ __align__(16) double th_sm[];
+  const int nq = t.nq, n_l = g.n_l, n_r = g.n_r, n_mp = t.n_mp;
+  double2* xs = reinterpret_cast<double2*>(th_sm);              // [N_l][TH_R]
+  double* fs = th_sm + 2 * (size_t)n_l * TH_R;                  // [2][nq][TH_R]
+  double* buf = fs + 2 * (size_t)nq * TH_R;                     // two table chunks
+  const int tiles = (n_r + TH_R - 1) / TH_R;
+  const int ri = blockIdx.x / tiles, r0 = (blockIdx.x - ri * tiles) * TH_R;
   const RunDev run = g.runs[g.runs_of_group[ri]];
-  double S[TH_QB], D[TH_QB];
-#pragma unroll
-  for (int u = 0; u < TH_QB; ++u) S[u] = D[u] = 0.0;
+  const int tid = threadIdx.x, p = tid % TH_R, item = tid / TH_R;   // this thread's node, then its multipole
+  double S = 0.0, D = 0.0;
   for (int k = 0; k < run.n_orb; ++k) {
     const int col = run.col0 + k;
     const int m = g.col_m[col];
     const double occ = (double)g.col_occ[col];
-    const double* Tm = t.T + (size_t)m * nq * n_l;
-    double2 e[TH_QB], o[TH_QB];
-#pragma unroll
-    for (int u = 0; u < TH_QB; ++u) e[u] = o[u] = make_double2(0.0, 0.0);
-    for (int l = m; l < n_l; ++l) {
-      const double2 xv = x[((size_t)l * g.n_cols + col) * g.n_r + r];
-      const bool odd = ((l - m) & 1) != 0;
-#pragma unroll
-      for (int u = 0; u < TH_QB; ++u) {
-        const int q = q0 + u;
-        const double tv = q < nq ? __ldg(Tm + (size_t)q * n_l + l) : 0.0;
-        if (odd) {
-          o[u].x = fma(tv, xv.x, o[u].x);
-          o[u].y = fma(tv, xv.y, o[u].y);
-        } else {
-          e[u].x = fma(tv, xv.x, e[u].x);
-          e[u].y = fma(tv, xv.y, e[u].y);
+    __syncthreads();                                            // the tile of the orbital before is done with
+    for (int i = tid; i < n_l * TH_R; i += blockDim.x) {
+      const int l = i / TH_R, r = r0 + i % TH_R;
+      xs[i] = r < n_r ? x[((size_t)l * g.n_cols + col) * n_r + r] : make_double2(0.0, 0.0);
+    }
+    double2 e = make_double2(0.0, 0.0), o = make_double2(0.0, 0.0);
+    // rows l = m .. N_l - 1 of Theta_l^m at every node (chunks start at even l - m)
+    table_chunks(t.T + ((size_t)m * n_l + m) * nq, n_l - m, nq, nq, buf, [&](int row0, int n, const double* T) {
+      if (item < nq) {
+        const double2* xl = xs + (m + row0) * TH_R + p;
+        int u = 0;
+        for (; u + 1 < n; u += 2) {
+          const double te = T[u * nq + item], to = T[(u + 1) * nq + item];
+          const double2 xe = xl[u * TH_R], xo = xl[(u + 1) * TH_R];
+          e.x = fma(te, xe.x, e.x);
+          e.y = fma(te, xe.y, e.y);
+          o.x = fma(to, xo.x, o.x);
+          o.y = fma(to, xo.y, o.y);
+        }
+        if (u < n) {
+          const double te = T[u * nq + item];
+          const double2 xe = xl[u * TH_R];
+          e.x = fma(te, xe.x, e.x);
+          e.y = fma(te, xe.y, e.y);
         }
       }
-    }
-#pragma unroll
-    for (int u = 0; u < TH_QB; ++u) {
-      S[u] += occ * 2.0 * (e[u].x * e[u].x + e[u].y * e[u].y + o[u].x * o[u].x + o[u].y * o[u].y);
-      D[u] += occ * 4.0 * (e[u].x * o[u].x + e[u].y * o[u].y);
-    }
+    });
+    S += occ * 2.0 * (e.x * e.x + e.y * e.y + o.x * o.x + o.y * o.y);
+    D += occ * 4.0 * (e.x * o.x + e.y * o.y);
   }
-  double* f = t.fine + (size_t)ri * 2 * nq * g.n_r;
-#pragma unroll
-  for (int u = 0; u < TH_QB; ++u) {
-    const int q = q0 + u;
-    if (q < nq) {
-      f[(size_t)q * g.n_r + r] = S[u];
-      f[((size_t)nq + q) * g.n_r + r] = D[u];
-    }
+  if (item < nq) {
+    fs[item * TH_R + p] = S;
+    fs[(nq + item) * TH_R + p] = D;
   }
-}
-
-// blocks (run, 32 radii, TH_WARPS multipoles): rho_L(r) for the warp's L, TH_ILP partial sums over
-// the fine nodes
-__global__ void __launch_bounds__(TH_THREADS) k_theta_project(GroupArgs g, ThetaArgs t) {
-  const int tiles = (g.n_r + 31) / 32;
-  const int lsplit = (t.n_mp + TH_WARPS - 1) / TH_WARPS;
-  const int ri = blockIdx.x / (tiles * lsplit);
-  const int rest = blockIdx.x - ri * tiles * lsplit;
-  const int tile = rest / lsplit, ls = rest - tile * lsplit;
-  const int r = tile * 32 + (threadIdx.x & 31);
-  const int L = ls * TH_WARPS + (threadIdx.x >> 5);
-  if (r >= g.n_r || L >= t.n_mp) return;
-  const int nq = t.nq, n_r = g.n_r;
-  const double* src = t.fine + ((size_t)ri * 2 + (L & 1)) * nq * n_r + r;
-  const double* w = t.wP + (size_t)L * nq;
-  double acc[TH_ILP];
+  for (int L0 = 0; L0 < n_mp; L0 += blockDim.x / TH_R) {
+    const int L = L0 + item;
+    double acc[TH_ILP];
 #pragma unroll
-  for (int u = 0; u < TH_ILP; ++u) acc[u] = 0.0;
-  int q = 0;
-  for (; q + TH_ILP - 1 < nq; q += TH_ILP)
+    for (int u = 0; u < TH_ILP; ++u) acc[u] = 0.0;
+    const int cols = min((int)(blockDim.x / TH_R), n_mp - L0);
+    table_chunks(t.wP + L0, nq, cols, n_mp, buf, [&](int row0, int n, const double* w) {
+      if (L >= n_mp) return;
+      const double* src = fs + ((size_t)(L & 1) * nq + row0) * TH_R + p;
+      int q = 0;
+      for (; q + TH_ILP - 1 < n; q += TH_ILP)
 #pragma unroll
-    for (int u = 0; u < TH_ILP; ++u) acc[u] = fma(__ldg(w + q + u), src[(size_t)(q + u) * n_r], acc[u]);
-  for (; q < nq; ++q) acc[0] = fma(__ldg(w + q), src[(size_t)q * n_r], acc[0]);
-  t.rho[((size_t)ri * t.n_mp + L) * n_r + r] = sum_partials(acc);
+        for (int u = 0; u < TH_ILP; ++u) acc[u] = fma(w[(q + u) * cols + item], src[(q + u) * TH_R], acc[u]);
+      for (; q < n; ++q) acc[0] = fma(w[q * cols + item], src[q * TH_R], acc[0]);
+    });
+    if (L < n_mp && r0 + p < n_r) t.rho[((size_t)ri * n_mp + L) * n_r + r0 + p] = sum_partials(acc);
+  }
 }
 
 // affine map a -> mul a + add, composed in the order of the recurrence
@@ -131,21 +156,29 @@ __device__ __forceinline__ Aff aff_then(Aff first, Aff second) {
   return Aff{second.mul * first.mul, fma(second.mul, first.add, second.add)};
 }
 
-// one warp per (run, L >= 1)
-__global__ void __launch_bounds__(TH_THREADS) k_theta_hartree(GroupArgs g, ThetaArgs t) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per_run = (t.n_mp - 1 + TH_WARPS - 1) / TH_WARPS;
-  const int ri = blockIdx.x / per_run;
-  const int L = 1 + (blockIdx.x - ri * per_run) * TH_WARPS + warp;
-  if (L >= t.n_mp) return;
+// one warp (block) per (run, L >= 1), the rows it scans in shared memory
+__global__ void __launch_bounds__(32) k_theta_hartree(GroupArgs g, ThetaArgs t) {
+  extern __shared__ __align__(16) double th_sm[];
+  const int lane = threadIdx.x;
+  const int ri = blockIdx.x / (t.n_mp - 1);
+  const int L = 1 + blockIdx.x - ri * (t.n_mp - 1);
   const int n = g.n_r;
-  const double* rho = t.rho + ((size_t)ri * t.n_mp + L) * n;
-  double* v = t.vmp + ((size_t)ri * t.n_mp + L) * n;
+  // rho_L, (r_(a-1)/r_a)^L and (r_(a-1)/r_a)^(L+1) (the grid's table)
+  double *rho = th_sm, *fL = th_sm + n, *gL = th_sm + 2 * n;
+  const double* rho_g = t.rho + ((size_t)ri * t.n_mp + L) * n;
+  const double* rq_g = t.rq + (size_t)L * n;
+  for (int a = lane; a < n; a += 32) {
+    cp_async8(rho + a, rho_g + a);
+    cp_async8(fL + a, rq_g + a);
+    cp_async8(gL + a, rq_g + n + a);
+  }
+  cp_async_commit();
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+  double* v = fL;               // a lane writes v[a] after its last use of fL[a]
   const int C = (n + 31) / 32;
   const int a0 = lane * C, a1 = min(n, a0 + C);
-  // forward: A_a = f_a A_(a-1) + rho_a, f_a = (r_(a-1)/r_a)^L (the grid's table), f_0 = 0
-  const double* fL = t.rq + (size_t)L * n;
-  const double* gL = t.rq + (size_t)(L + 1) * n;
+  // forward: A_a = f_a A_(a-1) + rho_a, f_a = (r_(a-1)/r_a)^L, f_0 = 0
   Aff mine{1.0, 0.0};
   for (int a = a0; a < a1; ++a) {
     const double f = a == 0 ? 0.0 : fL[a];
@@ -187,52 +220,64 @@ __global__ void __launch_bounds__(TH_THREADS) k_theta_hartree(GroupArgs g, Theta
     const double gg = a == n - 1 ? 0.0 : gL[a + 1];
     const double rn = a == n - 1 ? 0.0 : rho[a + 1];
     B = gg * (B + rn);
-    v[a] = (v[a] + B) / g.r[a];
+    v[a] += B;
   }
+  __syncwarp();
+  double* v_g = t.vmp + ((size_t)ri * t.n_mp + L) * n;
+  for (int a = lane; a < n; a += 32) v_g[a] = v[a] / g.r[a];
 }
 
-// blocks (run, 32 radii, TH_WARPS nodes (m, j)): htab[m][j][r] = sum_{L>=1} v_L(r) P_L(x_j^m),
-// TH_ILP partial sums over L
-__global__ void __launch_bounds__(TH_THREADS) k_theta_table(GroupArgs g, ThetaArgs t) {
-  const int tiles = (g.n_r + 31) / 32;
-  const int n_mj = g.n_m * g.n_l;
-  const int jsplit = (n_mj + TH_WARPS - 1) / TH_WARPS;
-  const int ri = blockIdx.x / (tiles * jsplit);
-  const int rest = blockIdx.x - ri * tiles * jsplit;
-  const int tile = rest / jsplit, js = rest - tile * jsplit;
-  const int r = tile * 32 + (threadIdx.x & 31);
-  const int mj = js * TH_WARPS + (threadIdx.x >> 5);
-  if (r >= g.n_r || mj >= n_mj) return;
+// htab[m][j][r] = sum_{L>=1} v_L(r) P_L(x_j^m), TH_ILP partial sums over L; blocks (run, m, radii)
+__global__ void __launch_bounds__(1024) k_theta_table(GroupArgs g, ThetaArgs t) {
+  extern __shared__ __align__(16) double th_sm[];
+  const int n_r = g.n_r, n_mp = t.n_mp, n_l = g.n_l;
+  const int tiles = (n_r + TH_R - 1) / TH_R;
+  const int rm = blockIdx.x / tiles, r0 = (blockIdx.x - rm * tiles) * TH_R;
+  const int ri = rm / g.n_m, m = rm - ri * g.n_m;
   const RunDev run = g.runs[g.runs_of_group[ri]];
-  const int n_r = g.n_r, n_mp = t.n_mp;
-  const double* v = t.vmp + (size_t)ri * n_mp * n_r + r;
-  const int m = mj / g.n_l, j = mj - m * g.n_l;
-  // TH_ILP independent partial sums: the loop is bound by the latency of its loads
+  double* vs = th_sm;                                           // [n_mp][TH_R]
+  double* buf = th_sm + (size_t)n_mp * TH_R;                    // two table chunks
+  const double* v = t.vmp + (size_t)ri * n_mp * n_r;
+  for (int i = threadIdx.x; i < n_mp * TH_R; i += blockDim.x) {
+    const int L = i / TH_R, r = r0 + i % TH_R;
+    vs[i] = L > 0 && r < n_r ? v[(size_t)L * n_r + r] : 0.0;
+  }
+  const int p = threadIdx.x % TH_R, j = threadIdx.x / TH_R;
   double acc[TH_ILP];
 #pragma unroll
   for (int u = 0; u < TH_ILP; ++u) acc[u] = 0.0;
-  if (j >= m) {
-    const double* pl = t.PLj + (size_t)m * n_mp * g.ldS + j;
-    int L = 1;
-    for (; L + TH_ILP - 1 < n_mp; L += TH_ILP)
+  table_chunks(t.PLj + ((size_t)m * n_mp + 1) * g.ldS, n_mp - 1, n_l, g.ldS, buf, [&](int row0, int n, const double* P) {
+    if (j < m || j >= n_l) return;
+    const double* vl = vs + (1 + row0) * TH_R + p;
+    int q = 0;
+    for (; q + TH_ILP - 1 < n; q += TH_ILP)
 #pragma unroll
-      for (int u = 0; u < TH_ILP; ++u)
-        acc[u] = fma(v[(size_t)(L + u) * n_r], __ldg(pl + (size_t)(L + u) * g.ldS), acc[u]);
-    for (; L < n_mp; ++L) acc[0] = fma(v[(size_t)L * n_r], __ldg(pl + (size_t)L * g.ldS), acc[0]);
+      for (int u = 0; u < TH_ILP; ++u) acc[u] = fma(vl[(q + u) * TH_R], P[(q + u) * n_l + j], acc[u]);
+    for (; q < n; ++q) acc[0] = fma(vl[q * TH_R], P[q * n_l + j], acc[0]);
+  });
+  if (j < n_l && r0 + p < n_r) run.htab[((size_t)m * n_l + j) * n_r + r0 + p] = sum_partials(acc);
+}
+
+static int theta_threads(int items) { return std::min(1024, (items * TH_R + 31) / 32 * 32); }
+static size_t theta_density_smem(int n_l, int nq, int threads) {
+  return ((size_t)(2 * n_l + 2 * nq) * TH_R + 2 * (size_t)TH_ROWS * std::max(nq, threads / TH_R)) * sizeof(double);
+}
+
+cudaError_t configure_theta(int optin) {
+  for (const void* fn : {(const void*)k_theta_density, (const void*)k_theta_hartree, (const void*)k_theta_table}) {
+    const cudaError_t e = set_max_dynamic_smem(fn, optin);
+    if (e != cudaSuccess) return e;
   }
-  run.htab[(size_t)mj * n_r + r] = sum_partials(acc);
+  return cudaSuccess;
 }
 
 void launch_theta_potentials(const GroupArgs& g, const ThetaArgs& t, const double2* x, cudaStream_t s) {
-  const int tiles = (g.n_r + 31) / 32;
-  const int qsplit = (t.nq + TH_WARPS * TH_QB - 1) / (TH_WARPS * TH_QB);
-  const int lsplit = (t.n_mp + TH_WARPS - 1) / TH_WARPS;
-  const int jsplit = (g.n_m * g.n_l + TH_WARPS - 1) / TH_WARPS;
-  k_theta_fine<<<g.n_runs * tiles * qsplit, TH_THREADS, 0, s>>>(g, t, x);
-  k_theta_project<<<g.n_runs * tiles * lsplit, TH_THREADS, 0, s>>>(g, t);
-  const int per_run = (t.n_mp - 1 + TH_WARPS - 1) / TH_WARPS;
-  if (per_run > 0) k_theta_hartree<<<g.n_runs * per_run, TH_THREADS, 0, s>>>(g, t);
-  k_theta_table<<<g.n_runs * tiles * jsplit, TH_THREADS, 0, s>>>(g, t);
+  const int tiles = (g.n_r + TH_R - 1) / TH_R;
+  const int threads = theta_threads(std::max(t.nq, t.n_mp));    // >= nq TH_R: N_l <= 220
+  k_theta_density<<<g.n_runs * tiles, threads, theta_density_smem(g.n_l, t.nq, threads), s>>>(g, t, x);
+  if (t.n_mp > 1) k_theta_hartree<<<g.n_runs * (t.n_mp - 1), 32, 3 * (size_t)g.n_r * sizeof(double), s>>>(g, t);
+  k_theta_table<<<g.n_runs * g.n_m * tiles, theta_threads(g.n_l),
+                  ((size_t)t.n_mp * TH_R + 2 * (size_t)TH_ROWS * g.n_l) * sizeof(double), s>>>(g, t);
 }
 
 }  // namespace ggb

@@ -68,3 +68,45 @@ def test_observables_noalloc_at_the_edges(n_l, n_orb, n_r):
         scale = (np.abs(x) * np.abs(z) * q).sum(-1).max() + 1e-300
         assert np.abs(got.cpu().numpy() - (p * q).sum(-1)).max() <= TOL * scale
     assert np.allclose(norm.cpu().numpy(), (np.abs(x) ** 2).sum(axis=(0, 2)), rtol=TOL, atol=0)
+
+
+@pytest.mark.parametrize("n_r,n_l,n_har", [(9, 8, 5), (13, 9, 17), (37, 33, 65), (45, 40, 33), (66, 36, 71)])
+def test_fp64_multipole_kernels_at_their_edges(n_r, n_l, n_har):
+    """The theta form's exact multipoles at radii that do not fill a block's four, nodes and multipoles
+    around the table chunk (32 rows) and the eight partial sums, against the oracle."""
+    from oracle.step_oracle import propagate
+    from tests.helpers import rel_err, to_oracle
+    run = P.reference_like(n_r, n_l, 6, "Ne3", r_mask=15.0, dt_as=10.0, perturb=0.05, seed=3)
+    run = dataclasses.replace(run, angular="theta", n_har=n_har)
+    ref = propagate(to_oracle(run))
+    tp = TimePropagation([run], precision="fp64")
+    tp.step(6)
+    x, pot, got = tp.orbitals(0), tp.potentials(0), tp.observables(0)
+    st, msg = tp.status()
+    tp.close()
+    assert st == 0, msg
+    assert rel_err(x, ref["x"]) < 1e-10          # the FP64 form's bar against the oracle
+    assert rel_err(pot["v"], ref["v"][:4]) < 1e-10
+    assert rel_err(got["norm"], ref["norm"]) < 1e-10
+
+
+@pytest.mark.parametrize("n_r,n_l,angular", [(7, 5, "reference"), (41, 8, "reference"), (33, 9, "theta"), (50, 65, "reference"),
+                                             (130, 129, "theta"), (21, 193, "theta")])
+def test_fp64_angular_tiles_at_their_edges(n_r, n_l, angular):
+    """Channel tiles of 8 and row groups of 64 (N_l 5 .. 193), radii that do not fill a tile, m = 0 and 1,
+    every coupling or the theta phase: one step against the oracle."""
+    from oracle.step_oracle import propagate
+    from tests.helpers import rel_err, to_oracle
+    run = P.reference_like(n_r, n_l, 3, "Ne3", r_mask=12.0, dt_as=10.0, perturb=0.05, seed=4)
+    run = dataclasses.replace(run, angular=angular)
+    for copies in (1, 30):                       # few tiles and many: another number of radii per tile
+        ref = propagate(to_oracle(run))
+        runs = [run.with_field(run.E) for _ in range(copies)]
+        tp = TimePropagation(runs, precision="fp64", groups=[list(range(copies))])
+        tp.step(3)
+        x, pot = tp.orbitals(copies - 1), tp.potentials(copies - 1)
+        st, msg = tp.status()
+        tp.close()
+        assert st == 0, msg
+        assert rel_err(x, ref["x"]) < 1e-10
+        assert rel_err(pot["v"], ref["v"][:4]) < 1e-10
