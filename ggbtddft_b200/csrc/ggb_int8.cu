@@ -68,6 +68,15 @@ __device__ __forceinline__ int row_exponent(double mx) {
 __device__ __forceinline__ uint32_t slice_word(double t3) {
   return ((uint32_t)__double2int_rn(t3) + 0x80808080u) ^ 0x80808080u;
 }
+// byte (3 - k) of four slice words as one word per plane k (the first word's byte lowest)
+__device__ __forceinline__ void plane_words(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, uint32_t (&p)[4]) {
+  const uint32_t a = __byte_perm(w0, w1, 0x6273), b = __byte_perm(w2, w3, 0x6273);
+  const uint32_t c = __byte_perm(w0, w1, 0x4051), d = __byte_perm(w2, w3, 0x4051);
+  p[0] = __byte_perm(a, b, 0x5410);
+  p[1] = __byte_perm(a, b, 0x7632);
+  p[2] = __byte_perm(c, d, 0x5410);
+  p[3] = __byte_perm(c, d, 0x7632);
+}
 // the four slices of t3 stored one byte at dst + k * PLANE, most significant first
 template <uint32_t PLANE>
 __device__ __forceinline__ void store_slices(uint8_t* dst, double t3) {
@@ -426,7 +435,6 @@ struct Ang8Args {
   int stages;
   const int* sexp;        // S^T row exponents [mat][m][rows]
   int rows;               // m_tiles * 128
-  int ld_stage;           // row length of the FP64 staging tiles [NP][ld_stage] (odd when it fits)
   int n_mats;             // chain matrices per variant
   int n_var;              // dithered variants of the chain matrices (a power of two)
   // theta form: the node-basis vectors of the second half after its phase, [N_l][n_cols][N_r]
@@ -468,15 +476,6 @@ __device__ __forceinline__ double2 rotd(double2 x, double e) {
   return make_double2(c * x.x + s * x.y, c * x.y - s * x.x);
 }
 
-// x_k(p) into the four slice planes: Re in row p, Im in row NP + p (the same swizzle chunk, NP being
-// a multiple of 8); sc3 = 2^e(p) 2^24
-template <int NP, uint32_t PLANE>
-__device__ __forceinline__ void slice_put(uint8_t* xb, int p, int k, double2 v, double sc3) {
-  const uint32_t o = a8_off(2 * NP, p, k);
-  store_slices<PLANE>(xb + o, v.x * sc3);
-  store_slices<PLANE>(xb + o + NP * 128, v.y * sc3);
-}
-
 // One CTA per (orbital column, NP radii): NP = 32 for N_l <= 128 (one M tile of 128 channels),
 // NP = 16 for N_l <= 256 (two M tiles), so that every CTA holds 256 TMEM columns and two CTAs share
 // an SM (one CTA's epilogue overlaps the other's products and loads).
@@ -509,7 +508,8 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ double pbase[5][NP];
-  __shared__ double pnorm2[NP];
+  __shared__ double pnorm2[A8_THREADS / NP][NP];
+  __shared__ double sdl[MAX_NL];
   __shared__ double pscale3[NP], pinv[NP];    // 2^e(p) 2^24 and 2^-e(p) of each point's B rows
   // aligned by an offset from the __shared__ array itself, so that the compiler keeps the shared
   // address space (shared loads and stores, not generic ones) for every access through it
@@ -521,20 +521,39 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   const int tilesN = (g.n_r + NP - 1) / NP;
   const int col = blockIdx.x / tilesN;
   const int r0 = (blockIdx.x - col * tilesN) * NP;
-  const int m = g.col_m[col];
-  const RunDev run = g.runs[g.col_run[col]];
   const Chain& ch = g.chain[SECOND_HALF ? 1 : 0];
   const int n_ops = ch.n_ops;
   const int acc_cols = 4 * NB;                // per M tile: weights 2^0 .. 2^-24
   const int step_raw = *g.step;
-  const int step = step_raw < run.n_t ? step_raw : run.n_t - 1;
-  const double hdt = 0.5 * g.dt;
-  const double* pco = g.coef + ((size_t)CF_P * g.n_m + m) * n_l;
   // basis reuse: the second half keeps its node-basis vectors, the first half of the step they
   // were kept for starts from them at its last product (o0 = 1, the theta chain having two)
   const bool keep_theta = THETA && SECOND_HALF && t.yth != nullptr;
   const bool from_theta = THETA && !SECOND_HALF && t.yth != nullptr && *t.yth_step == step_raw;
   const int o0 = from_theta ? 1 : 0;
+
+  // the x tile (all l, NP points): point fp = tid % NP, the l quads fg, fg + FG, ... of this thread, all
+  // requested here, so that the rest of the set-up runs under their latency
+  constexpr int FG = A8_THREADS / NP;          // l quads per round
+  constexpr int FR = NP == 32 ? 4 : 3;         // rounds: 32 quads (N_l <= 128) or 56 (N_l <= 220)
+  const int fp = threadIdx.x % NP, fg = threadIdx.x / NP;
+  double2 xv[FR][4];
+  {
+    const double2* src = (from_theta ? t.yth : xin) + (size_t)col * g.n_r + r0 + fp;
+    const size_t ls = (size_t)g.n_cols * g.n_r;
+    const bool rv = r0 + fp < g.n_r;
+#pragma unroll
+    for (int f = 0; f < FR; ++f)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int l = 4 * (fg + f * FG) + u;
+        xv[f][u] = (l < n_l && rv) ? src[(size_t)l * ls] : make_double2(0.0, 0.0);
+      }
+  }
+  const int m = g.col_m[col];
+  const RunDev run = g.runs[g.col_run[col]];
+  const int step = step_raw < run.n_t ? step_raw : run.n_t - 1;
+  const double hdt = 0.5 * g.dt;
+  const double* pco = g.coef + ((size_t)CF_P * g.n_m + m) * n_l;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < t.stages; ++s) {
@@ -565,63 +584,79 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
     pbase[2][p] = v2 * hdt;
     pbase[3][p] = v3 * hdt;
     pbase[4][p] = sb * hdt;
-    pnorm2[p] = 0.0;
   }
+  // what the fill's phase takes per l: the first product's eigenvalue (basis reuse) or the S coefficient
+  for (int l = threadIdx.x; l < n_l; l += A8_THREADS)
+    sdl[l] = SECOND_HALF ? (ch.pre_s ? pco[l] : 0.0) : g.dph[((size_t)ch.ops[0].coupling * g.n_m + m) * g.ldS + l];
   __syncthreads();
+  // the first S^T slice planes are on their way while the operand is filled
+  const int mat0 = ch.ops[o0].mat + (step_raw & (t.n_var - 1)) * t.n_mats;   // this step's variant
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int pa = 0; pa < I8_SLICES; ++pa) {
+      mbar_expect_tx(&full_bar[pa], A8_A_TILE);
+      tma_load_5d(sst + pa * A8_A_TILE, &tmS, 0, 0, pa, m, mat0, &full_bar[pa]);
+    }
+  }
 
-  // operand: the x tile (all l, NP points) [second half: l-diagonal S phase], staged in the stage
-  // buffers (free until the producer starts) as [NP][ldf], the per-point norms, then the slices
+  // operand: phases of the tile in registers (second half: the l-diagonal S phase; basis reuse: the
+  // first product's phase, the same angle as its epilogue's), the per-point norms, then the slices
   const int lk = t.k_atoms * A8_KATOM;
-  const int ldf = t.ld_stage;
-  double2* stg = reinterpret_cast<double2*>(sst);
   {
-    constexpr int U = 4;
-    double part = 0.0;          // this thread's points are fixed: p = threadIdx.x % NP (A8_THREADS % NP == 0)
-    const double2* src = from_theta ? t.yth : xin;
-    // the reuse path applies the first product's phase here, as its epilogue would (same angle)
-    const double* Dv0 = g.dph + ((size_t)ch.ops[0].coupling * g.n_m + m) * g.ldS;
-    for (int base = threadIdx.x; base < n_l * NP; base += U * A8_THREADS) {
-      double2 v[U];
+    double part = 0.0;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int idx = base + u * A8_THREADS;
-        const int l = idx / NP, p = idx - l * NP, r = r0 + p;
-        v[u] = (idx < n_l * NP && r < g.n_r) ? src[((size_t)l * g.n_cols + col) * g.n_r + r] : make_double2(0.0, 0.0);
-      }
+    for (int f = 0; f < FR; ++f)
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int idx = base + u * A8_THREADS;
-        if (idx < n_l * NP) {
-          const int l = idx / NP, p = idx - l * NP;
-          double2 w = v[u];
-          if (SECOND_HALF && ch.pre_s) w = rotd(w, pbase[4][p] + pco[l] * pbase[2][p]);
+      for (int u = 0; u < 4; ++u) {
+        const int l = 4 * (fg + f * FG) + u;
+        double2 w = xv[f][u];
+        if (l < n_l) {
+          if (SECOND_HALF && ch.pre_s) w = rotd(w, pbase[4][fp] + sdl[l] * pbase[2][fp]);
           if (!SECOND_HALF && THETA && from_theta && l >= m) {
-            const double dj = Dv0[l], p2j = legendre_p2(dj), p3j = legendre_p3(dj);
-            double ang = pbase[1][p] * dj + pbase[2][p] * p2j + pbase[3][p] * p3j + pbase[4][p];
-            if (g.theta_tab && r0 + p < g.n_r) ang += run.htab[((size_t)m * n_l + l) * g.n_r + r0 + p] * hdt;
+            const double dj = sdl[l], p2j = legendre_p2(dj), p3j = legendre_p3(dj);
+            double ang = pbase[1][fp] * dj + pbase[2][fp] * p2j + pbase[3][fp] * p3j + pbase[4][fp];
+            if (g.theta_tab && r0 + fp < g.n_r) ang += run.htab[((size_t)m * n_l + l) * g.n_r + r0 + fp] * hdt;
             w = rotd(w, ang);
           }
-          stg[p * ldf + l] = w;
-          part += w.x * w.x + w.y * w.y;
         }
+        xv[f][u] = w;
+        part += w.x * w.x + w.y * w.y;
       }
-    }
-    atomicAdd(&pnorm2[threadIdx.x % NP], part);
+    pnorm2[fg][fp] = part;
   }
   __syncthreads();
   if (threadIdx.x < NP) {
     // |Re y_j|, |Im y_j| <= |y| = |x| for every vector of the chain; the margin covers the chain's
     // rounding and the non-orthogonality of the sliced matrices (both ~2^-31)
-    const int e = row_exponent(sqrt(pnorm2[threadIdx.x]) * (1.0 + 0x1p-20));
+    double n2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < FG; ++q) n2 += pnorm2[q][threadIdx.x];
+    const int e = row_exponent(sqrt(n2) * (1.0 + 0x1p-20));
     pscale3[threadIdx.x] = pow2i(e + 24);
     pinv[threadIdx.x] = pow2i(-e);
   }
   __syncthreads();
-  // lanes along l: each warp writes consecutive bytes of one B row
-  for (int idx = threadIdx.x; idx < lk * NP; idx += A8_THREADS) {
-    const int p = idx / lk, l = idx - p * lk;
-    const double2 w = l < n_l ? stg[p * ldf + l] : make_double2(0.0, 0.0);
-    slice_put<NP, B_TILE>(xb, p, l, w, pscale3[p]);
+  // four consecutive l per thread: one word per slice plane, Re in row fp and Im in row NP + fp (the
+  // same swizzle chunk, NP being a multiple of 8); zero beyond N_l up to the K steps that are read
+  {
+    const double sc3 = pscale3[fp];
+#pragma unroll
+    for (int f = 0; f < FR; ++f) {
+      const int quad = fg + f * FG;
+      if (quad < 8 * t.k_steps) {
+        uint8_t* dst = xb + a8_off(2 * NP, fp, 4 * quad);
+        uint32_t pr[I8_SLICES], pi[I8_SLICES];
+        plane_words(slice_word(xv[f][0].x * sc3), slice_word(xv[f][1].x * sc3), slice_word(xv[f][2].x * sc3),
+                    slice_word(xv[f][3].x * sc3), pr);
+        plane_words(slice_word(xv[f][0].y * sc3), slice_word(xv[f][1].y * sc3), slice_word(xv[f][2].y * sc3),
+                    slice_word(xv[f][3].y * sc3), pi);
+#pragma unroll
+        for (int k = 0; k < I8_SLICES; ++k) {
+          *reinterpret_cast<uint32_t*>(dst + k * B_TILE) = pr[k];
+          *reinterpret_cast<uint32_t*>(dst + k * B_TILE + NP * 128) = pi[k];
+        }
+      }
+    }
   }
   fence_async_smem();
   tc_fence_before();
@@ -642,7 +677,8 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
             const int round = it / I8_SLICES;
 #pragma unroll
             for (int pa = 0; pa < I8_SLICES; ++pa, ++it) {
-              if (round > 0 && !mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) {
+              if (round == 0) continue;          // issued before the fill
+              if (!mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) {
                 ok = false;
                 break;
               }
@@ -828,7 +864,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
       constexpr int LG = 32 / NP;        // lane groups per warp: lane = (point, l-loop group)
       constexpr int NG = NW * LG;        // groups that stride the density's l loops
       double* rows = reinterpret_cast<double*>(smem + (((size_t)n_l * (NP + 1) * 16 + 255) & ~(size_t)255));
-      double* red = rows + COEF_N * n_l;                    // [NG][N_DEN][NP]
+      double* red = rows + ((COEF_N * n_l + 1) & ~1);       // [NG][N_DEN][NP], 16-byte aligned
       double* prr = red + NG * N_DEN * NP;                  // [2][NP]: r and r^-2 of each point (0 past N_r)
       for (int i = threadIdx.x; i < COEF_N * n_l; i += A8_THREADS) {
         const int c = i / n_l, l = i - c * n_l;
@@ -838,40 +874,43 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
         const int r = r0 + threadIdx.x;
         const double rr = r < g.n_r ? g.r[r] : 0.0;
         prr[threadIdx.x] = rr;
-        prr[NP + threadIdx.x] = r < g.n_r ? pow(rr, -2.0) : 0.0;
+        prr[NP + threadIdx.x] = r < g.n_r ? 1.0 / (rr * rr) : 0.0;
       }
       __syncthreads();
-      // dipole and acceleration: one thread per l, summing this CTA's NP radii in order (the same
-      // terms as observables_tile; one partial per (l, NP radii))
-      for (int l = threadIdx.x; l < n_l; l += A8_THREADS) {
-        double sx = 0.0, sy = 0.0, sz = 0.0, sw = 0.0;
-        if (l >= m) {
-          const double c_u = rows[CF_CU * n_l + l], c_d = rows[CF_CD * n_l + l];
-          const bool has_u = l + 1 < n_l, has_d = l >= 1;
-          for (int p = 0; p < NP; ++p) {
-            const double rr = prr[p], fr2 = prr[NP + p];
-            const double2 xl = xs[l * (NP + 1) + p];
-            const double2 xu = has_u ? xs[(l + 1) * (NP + 1) + p] : make_double2(0.0, 0.0);
-            const double2 xd = has_d ? xs[(l - 1) * (NP + 1) + p] : make_double2(0.0, 0.0);
-            double2 z1, z2;
-            if (l == m) {
-              z1 = make_double2(rr * c_u * xu.x, rr * c_u * xu.y);
-              z2 = make_double2(fr2 * c_u * xu.x, fr2 * c_u * xu.y);
-            } else if (l == n_l - 1) {
-              z1 = make_double2(rr * c_d * xd.x, rr * c_d * xd.y);
-              z2 = make_double2(fr2 * c_d * xd.x, fr2 * c_d * xd.y);
-            } else {
-              z1 = make_double2(rr * c_u * xu.x + rr * c_d * xd.x, rr * c_u * xu.y + rr * c_d * xd.y);
-              z2 = make_double2(fr2 * (c_u * xu.x + c_d * xd.x), fr2 * (c_u * xu.y + c_d * xd.y));
-            }
-            sx += xl.x * z1.x + xl.y * z1.y;
-            sy += xl.x * z1.y - xl.y * z1.x;
-            sz += xl.x * z2.x + xl.y * z2.y;
-            sw += xl.x * z2.y - xl.y * z2.x;
-          }
+      // dipole and acceleration: `parts` threads per l, each over its share of the CTA's NP radii, then
+      // the shares added in order (one partial per (l, NP radii))
+      double4* ored = reinterpret_cast<double4*>(red);      // [parts][lw], parts lw <= A8_THREADS
+      const int lw = (n_l + 31) & ~31, parts = A8_THREADS >= lw ? A8_THREADS / lw : 1;
+      const int part = threadIdx.x / lw, lo = threadIdx.x - part * lw;
+      double4 osum = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (part < parts && lo < n_l && lo >= m) {
+        // the first row has no lower, the last no upper neighbour
+        const bool has_u = lo + 1 < n_l, has_d = lo > m;
+        const double c_u = has_u ? rows[CF_CU * n_l + lo] : 0.0, c_d = has_d ? rows[CF_CD * n_l + lo] : 0.0;
+        const double2* xl_p = xs + lo * (NP + 1);
+        for (int p = part * NP / parts; p < (part + 1) * NP / parts; ++p) {
+          const double2 xl = xl_p[p];
+          const double2 xu = has_u ? xl_p[p + NP + 1] : make_double2(0.0, 0.0);
+          const double2 xd = has_d ? xl_p[p - NP - 1] : make_double2(0.0, 0.0);
+          const double zx = c_u * xu.x + c_d * xd.x, zy = c_u * xu.y + c_d * xd.y;
+          const double px = xl.x * zx + xl.y * zy, py = xl.x * zy - xl.y * zx;     // conj(x_l) . z
+          osum.x = fma(prr[p], px, osum.x);
+          osum.y = fma(prr[p], py, osum.y);
+          osum.z = fma(prr[NP + p], px, osum.z);
+          osum.w = fma(prr[NP + p], py, osum.w);
         }
-        g.obs[((size_t)col * n_l + l) * g.n_tiles + r0 / NP] = make_double4(sx, sy, sz, sw);
       }
+      if (parts > 1) {
+        if (part < parts) ored[part * lw + lo] = osum;
+        __syncthreads();
+        if (part == 0)
+          for (int q = 1; q < parts; ++q) {
+            const double4 v = ored[q * lw + lo];
+            osum.x += v.x; osum.y += v.y; osum.z += v.z; osum.w += v.w;
+          }
+      }
+      if (part == 0 && lo < n_l) g.obs[((size_t)col * n_l + lo) * g.n_tiles + r0 / NP] = osum;
+      if (parts > 1) __syncthreads();         // the shares' memory is the density's next
       // density multipoles: every lane works (point lane % NP), the literal l loops strided over the
       // NG lane groups, then the groups summed in order
       const int n_den = g.n_den > 0 ? g.n_den : 1;   // L = 0 is always needed for the norm
@@ -931,21 +970,19 @@ k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int 
   int8_t* b = X + (size_t)l * 12 * plane + (size_t)col * k_pad;
   // four radii per thread and plane: one 32-bit store each
   for (int r4 = 4 * threadIdx.x; r4 < n_r; r4 += 4 * SX_THREADS) {
-    uint32_t pr[I8_SLICES] = {0, 0, 0, 0}, pi[I8_SLICES] = {0, 0, 0, 0}, pn[I8_SLICES] = {0, 0, 0, 0};
+    uint32_t pr[I8_SLICES], pi[I8_SLICES], pn[I8_SLICES], wr[4], wi[4], wn[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int r = r4 + u;
       const double2 v = r < n_r ? xr[r] : make_double2(0.0, 0.0);
       // -Xi is sliced from -x itself: negating a digit -128 would not fit an int8
-      const uint32_t wr = slice_word(v.x * sc * 16777216.0), wi = slice_word(v.y * sc * 16777216.0),
-                     wn = slice_word(-v.y * sc * 16777216.0);
-#pragma unroll
-      for (int qq = 0; qq < I8_SLICES; ++qq) {
-        pr[qq] |= ((wr >> (24 - 8 * qq)) & 0xffu) << (8 * u);
-        pi[qq] |= ((wi >> (24 - 8 * qq)) & 0xffu) << (8 * u);
-        pn[qq] |= ((wn >> (24 - 8 * qq)) & 0xffu) << (8 * u);
-      }
+      wr[u] = slice_word(v.x * sc * 16777216.0);
+      wi[u] = slice_word(v.y * sc * 16777216.0);
+      wn[u] = slice_word(-v.y * sc * 16777216.0);
     }
+    plane_words(wr[0], wr[1], wr[2], wr[3], pr);
+    plane_words(wi[0], wi[1], wi[2], wi[3], pi);
+    plane_words(wn[0], wn[1], wn[2], wn[3], pn);
 #pragma unroll
     for (int qq = 0; qq < I8_SLICES; ++qq) {
       reinterpret_cast<uint32_t*>(b + qq * plane + r4)[0] = pr[qq];
@@ -1050,14 +1087,11 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   q.np = q.a_m_tiles == 1 ? 32 : 16;     // the kernel takes k_atoms = m_tiles = (NP == 32 ? 1 : 2)
   q.a_stages = I8_SLICES;   // the MMA issue loop relies on stage = slice plane
   q.a_smem = q.np == 32 ? a8_smem<32>(q.a_k_atoms, q.a_stages) : a8_smem<16>(q.a_k_atoms, q.a_stages);
-  // FP64 staging: the input tile [NP][ld] in the stage buffers (an odd ld when it fits), the last
-  // product [N_l][NP + 1] over the operand planes and stage buffers
-  q.a_ld = ((size_t)q.np * (n_l | 1) * 16 <= (size_t)q.a_stages * A8_A_TILE) ? (n_l | 1) : n_l;
+  // FP64 staging of the last product, [N_l][NP + 1], over the operand planes and stage buffers
   // the second half's tail: output tile, coefficient rows and the multipoles' warp partials
-  const size_t tail = (((size_t)n_l * (q.np + 1) * 16 + 255) & ~(size_t)255) + (size_t)COEF_N * n_l * 8 +
+  const size_t tail = (((size_t)n_l * (q.np + 1) * 16 + 255) & ~(size_t)255) + ((size_t)COEF_N * n_l + 1) * 8 +
                       (size_t)(A8_THREADS / 32) * N_DEN * 32 * 8 + 2 * (size_t)q.np * 8;
-  if ((size_t)q.np * q.a_ld * 16 > (size_t)q.a_stages * A8_A_TILE || tail > q.a_smem - 1024 ||
-      q.a_smem > 110 * 1024) {
+  if (tail > q.a_smem - 1024 || q.a_smem > 110 * 1024) {
     err = "int8 angular chain: shared memory";
     return GGB_ERR_ARG;
   }
@@ -1142,7 +1176,6 @@ void int8_angular(MixedGroup& mg, const GroupArgs& a, int half, const double2* x
   t.stages = q.a_stages;
   t.sexp = q.sexp;
   t.rows = q.a_rows;
-  t.ld_stage = q.a_ld;
   t.n_mats = q.n_mats;
   t.n_var = I8_S_VARIANTS;
   t.yth = q.yth;
