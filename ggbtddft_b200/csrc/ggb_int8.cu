@@ -26,9 +26,9 @@
 //   two row scales exactly and rounds once to FP64.  The orbitals stay complex128 between products.
 //   int32 range: |a b| <= 2^14, at most 8 products per k and accumulator, K <= 8192: <= 2^30.
 //
-//  k_slice_w_i8      W[l][k][i] -> A(i,k) planes [variant][l][8][rows][k] (Wr a1..a4, Wi a1..a4) + exponents
+//  k_slice_w_i8      W[l][k][i] -> A(i,k) stages [variant][l][row tile][k block][8][128][32] (Wr a1..a4, Wi a1..a4) + exponents
 //  k_build_st_i8     chain matrices -> S^T planes [variant n_mats + mat][m][4][rows][lk] + exponents
-//  k_slice_x         orbitals (complex128) -> radial B operand planes (Xr, Xi, -Xi) + exponents
+//  k_slice_x         orbitals (complex128) -> radial B operand stages (Xr, Xi, -Xi) + exponents
 //  k_radial_i8       persistent radial product, kind::i8, 32-byte swizzle, 16 MMAs per 32-wide k block
 //                    (each covers all x slices m of one W slice j):
 //                      Re_s += Wr_j Xr_m + Wi_j (-Xi)_m,  Im_s += Wr_j Xi_m + Wi_j Xr_m   (j + m = s)
@@ -125,7 +125,18 @@ __global__ void k_w_rowmax(const double2* __restrict__ W, int* __restrict__ wexp
   wexp[(size_t)l * rows_pad + i] = row_exponent(mx);
 }
 
-// A(i,k) planes, transposed through shared memory (read along i, write along k)
+// Operand tiles of the radial product in memory are the shared-memory image of a pipeline stage: per
+// (tile of rows, 32-wide k block) the slice planes one after the other, each [rows][32 bytes] with the
+// 32-byte swizzle already applied (the two 16-byte halves of a row change places in rows 4 .. 7 of every
+// eight), so that a stage is one contiguous copy.  As a [rows][k] matrix a stage was a TMA box of 32-byte
+// rows, 1024 and more of them, which paced
+// the copies: 69 -> 53 us for one argon run (N_r 600, N_l 97: 302 MB of W, 5.7 TB/s), 176 -> 155 us for
+// ten, 990 -> 859 us for 21 at N_r 1000, N_l 161.
+__host__ __device__ __forceinline__ uint32_t r8_row_off(int row, int k) {
+  return (uint32_t)(row * 32 + ((((k >> 4) & 1) ^ ((row >> 2) & 1)) << 4) + (k & 15));
+}
+
+// A(i,k) tiles, transposed through shared memory (read along i, write along k)
 __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restrict__ wexp, int8_t* __restrict__ Wi8,
                              int n_r, int rows_pad, int k_pad, int variant, int n_var) {
   __shared__ double2 t[32][33];
@@ -137,10 +148,12 @@ __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restric
     t[q][tx] = (k < n_r && i < n_r) ? W[((size_t)l * n_r + k) * n_r + i] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  const size_t plane = (size_t)rows_pad * k_pad;
-  int8_t* base = Wi8 + (size_t)l * 8 * plane;
+  constexpr int PLANE = 128 * 32;                     // one slice plane of a stage
+  const int n_kb = k_pad / 32;
   for (int q = ty; q < 32; q += 8) {
     const int i = i0 + q, k = k0 + tx;
+    int8_t* base = Wi8 + (((size_t)l * (rows_pad / 128) + i / 128) * n_kb + k0 / 32) * (2 * I8_SLICES * PLANE) +
+                   r8_row_off(i % 128, tx);
     if (i < rows_pad && k < k_pad) {
       const double sc = ldexp(1.0, wexp[(size_t)l * rows_pad + i]);
       const double2 w = t[tx][q];
@@ -148,11 +161,10 @@ __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restric
       int8_t sr[I8_SLICES], si[I8_SLICES];
       slice4_dithered(w.x * sc, dither_offset(variant, n_var, h), sr);
       slice4_dithered(w.y * sc, dither_offset(variant, n_var, h * 0x165667B1u), si);
-      const size_t o = (size_t)i * k_pad + k;
 #pragma unroll
       for (int p = 0; p < I8_SLICES; ++p) {
-        base[p * plane + o] = sr[p];
-        base[(I8_SLICES + p) * plane + o] = si[p];
+        base[p * PLANE] = sr[p];
+        base[(I8_SLICES + p) * PLANE] = si[p];
       }
     }
   }
@@ -243,7 +255,7 @@ struct R8Tile {
 
 template <int BN>
 __global__ void __launch_bounds__(R8_THREADS, 1)
-k_radial_i8(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __restrict__ X,
             const int* __restrict__ wexp, const int* __restrict__ xexp, int n_r, int rows_pad, int n_cols,
             int cols_pad, int n_l, int n_k_blocks, int stages, const int* __restrict__ step, int n_var,
             double2* __restrict__ Y, unsigned* status) {
@@ -288,6 +300,10 @@ k_radial_i8(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
   if (warp == 0) {
     if (lane == 0) {
       const int var = *step & (n_var - 1);     // this step's variant of W
+      const int8_t* Wv = W + (size_t)var * w_variant;
+      // W streams through L2 once a step (its variants alternate): read by one CTA only, it must not push
+      // the orbitals, the chain matrices and the kept vectors out; read by several, it stays for them
+      const uint64_t w_policy = l2_evict_first();
       int it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
@@ -301,8 +317,11 @@ k_radial_i8(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUt
           }
           uint8_t* st = smem + (size_t)s * T::STAGE;
           mbar_expect_tx(&full_bar[s], T::STAGE);
-          tma_load_5d(st, &tmW, kb * R8_BK, mt * R8_BM, 0, l, var, &full_bar[s]);
-          tma_load_4d(st + T::A_STAGE, &tmX, kb * R8_BK, nt * BN, 0, l, &full_bar[s]);
+          const int8_t* wsrc = Wv + ((size_t)(l * m_tiles + mt) * n_k_blocks + kb) * T::A_STAGE;
+          if (n_tiles == 1) bulk_g2s_hint(st, wsrc, T::A_STAGE, &full_bar[s], w_policy);
+          else bulk_g2s(st, wsrc, T::A_STAGE, &full_bar[s]);
+          bulk_g2s(st + T::A_STAGE, X + ((size_t)(l * n_tiles + nt) * n_k_blocks + kb) * (T::STAGE - T::A_STAGE),
+                   T::STAGE - T::A_STAGE, &full_bar[s]);
         }
       }
       if (!ok)
@@ -942,10 +961,10 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
 }
 
 // Radial B operand of one (l, orbital column) row: exponent f with max(|Re|, |Im|) 2^f in
-// [63.75, 127.5) over the row, then Xr, Xi, -Xi as four slices each ([l][12][cols_pad][k_pad]).
+// [63.75, 127.5) over the row, then Xr, Xi, -Xi as four slices each ([l][column tile][k block][12][bn][32]).
 constexpr int SX_THREADS = 128;
 __global__ void __launch_bounds__(SX_THREADS)
-k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int k_pad, int8_t* __restrict__ X,
+k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int bn, int k_pad, int8_t* __restrict__ X,
           int* __restrict__ xexp) {
   const int row = blockIdx.x;                  // l * n_cols + col
   const int l = row / n_cols, col = row - l * n_cols;
@@ -966,8 +985,9 @@ k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int 
   const int f = row_exponent(mx);
   if (threadIdx.x == 0) xexp[(size_t)l * cols_pad + col] = f;
   const double sc = pow2i(f);
-  const size_t plane = (size_t)cols_pad * k_pad;
-  int8_t* b = X + (size_t)l * 12 * plane + (size_t)col * k_pad;
+  // stage (l, column tile, k block): 12 planes of [bn][32 bytes]
+  const int nt = col / bn, row_in = col - nt * bn, plane = bn * 32;
+  int8_t* xt = X + (size_t)(l * (cols_pad / bn) + nt) * (k_pad / 32) * (R8_X_PLANES * plane);
   // four radii per thread and plane: one 32-bit store each
   for (int r4 = 4 * threadIdx.x; r4 < n_r; r4 += 4 * SX_THREADS) {
     uint32_t pr[I8_SLICES], pi[I8_SLICES], pn[I8_SLICES], wr[4], wi[4], wn[4];
@@ -983,11 +1003,12 @@ k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int 
     plane_words(wr[0], wr[1], wr[2], wr[3], pr);
     plane_words(wi[0], wi[1], wi[2], wi[3], pi);
     plane_words(wn[0], wn[1], wn[2], wn[3], pn);
+    int8_t* b = xt + (size_t)(r4 >> 5) * (R8_X_PLANES * plane) + r8_row_off(row_in, r4 & 31);
 #pragma unroll
     for (int qq = 0; qq < I8_SLICES; ++qq) {
-      reinterpret_cast<uint32_t*>(b + qq * plane + r4)[0] = pr[qq];
-      reinterpret_cast<uint32_t*>(b + (I8_SLICES + qq) * plane + r4)[0] = pi[qq];
-      reinterpret_cast<uint32_t*>(b + (2 * I8_SLICES + qq) * plane + r4)[0] = pn[qq];
+      reinterpret_cast<uint32_t*>(b + qq * plane)[0] = pr[qq];
+      reinterpret_cast<uint32_t*>(b + (I8_SLICES + qq) * plane)[0] = pi[qq];
+      reinterpret_cast<uint32_t*>(b + (2 * I8_SLICES + qq) * plane)[0] = pn[qq];
     }
   }
 }
@@ -1030,6 +1051,7 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   if (q.tune_stages > 0) q.stages = std::min(q.tune_stages, q.stages);
   // W planes and row exponents
   const size_t nw = (size_t)n_l * R8_W_PLANES * mg.rows_pad * mg.k_pad;    // one variant
+  q.w_variant = nw;
   I8_CK(cudaMalloc(&q.W, nw * I8_W_VARIANTS));
   I8_CK(cudaMalloc(&q.wexp, (size_t)n_l * mg.rows_pad * sizeof(int)));
   k_w_rowmax<<<dim3((mg.rows_pad + 127) / 128, n_l), 128>>>(W_fp64, q.wexp, n_r, mg.rows_pad);
@@ -1047,33 +1069,6 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   if (!enc) {
     err = "cuTensorMapEncodeTiled unavailable";
     return GGB_ERR_CUDA;
-  }
-  {
-    cuuint64_t dims[5] = {(cuuint64_t)mg.k_pad, (cuuint64_t)mg.rows_pad, R8_W_PLANES, (cuuint64_t)n_l,
-                          (cuuint64_t)I8_W_VARIANTS};
-    cuuint64_t strides[4] = {(cuuint64_t)mg.k_pad, (cuuint64_t)mg.rows_pad * mg.k_pad,
-                             (cuuint64_t)R8_W_PLANES * mg.rows_pad * mg.k_pad, (cuuint64_t)nw};
-    cuuint32_t box[5] = {R8_BK, R8_BM, R8_W_PLANES, 1, 1};
-    cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    if (enc(&q.tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, q.W, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-        CUDA_SUCCESS) {
-      err = "tensor map (int8 W) failed";
-      return GGB_ERR_CUDA;
-    }
-  }
-  {
-    cuuint64_t dims[4] = {(cuuint64_t)mg.k_pad, (cuuint64_t)q.cols_pad, R8_X_PLANES, (cuuint64_t)n_l};
-    cuuint64_t strides[3] = {(cuuint64_t)mg.k_pad, (cuuint64_t)q.cols_pad * mg.k_pad,
-                             (cuuint64_t)R8_X_PLANES * q.cols_pad * mg.k_pad};
-    cuuint32_t box[4] = {R8_BK, (cuuint32_t)q.bn, R8_X_PLANES, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    if (enc(&q.tmX, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, q.X, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-        CUDA_SUCCESS) {
-      err = "tensor map (int8 x) failed";
-      return GGB_ERR_CUDA;
-    }
   }
   // angular chain: S^T slices
   q.a_m_tiles = (n_l + 127) / 128;
@@ -1161,9 +1156,9 @@ void int8_radial(MixedGroup& mg, const GroupArgs& a, cudaStream_t s) {
   const dim3 g(tiles < q.ctas ? tiles : q.ctas);
   const int nkb = mg.k_pad / R8_BK;
   switch (q.bn) {
-    case 16: k_radial_i8<16><<<g, R8_THREADS, q.smem, s>>>(q.tmW, q.tmX, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
-    case 32: k_radial_i8<32><<<g, R8_THREADS, q.smem, s>>>(q.tmW, q.tmX, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
-    default: k_radial_i8<64><<<g, R8_THREADS, q.smem, s>>>(q.tmW, q.tmX, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
+    case 16: k_radial_i8<16><<<g, R8_THREADS, q.smem, s>>>(q.W, q.w_variant, q.X, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
+    case 32: k_radial_i8<32><<<g, R8_THREADS, q.smem, s>>>(q.W, q.w_variant, q.X, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
+    default: k_radial_i8<64><<<g, R8_THREADS, q.smem, s>>>(q.W, q.w_variant, q.X, q.wexp, q.xexp, a.n_r, mg.rows_pad, a.n_cols, q.cols_pad, a.n_l, nkb, q.stages, a.step, I8_W_VARIANTS, mg.Yd, a.status); break;
   }
 }
 
@@ -1194,7 +1189,7 @@ void int8_angular(MixedGroup& mg, const GroupArgs& a, int half, const double2* x
 
 void int8_slice_x(MixedGroup& mg, const GroupArgs& a, const double2* x, cudaStream_t s) {
   const I8Group& q = mg.i8;
-  k_slice_x<<<a.n_l * a.n_cols, SX_THREADS, 0, s>>>(x, a.n_r, a.n_cols, q.cols_pad, mg.k_pad, q.X, q.xexp);
+  k_slice_x<<<a.n_l * a.n_cols, SX_THREADS, 0, s>>>(x, a.n_r, a.n_cols, q.cols_pad, q.bn, mg.k_pad, q.X, q.xexp);
 }
 
 void int8_release(I8Group& q) {

@@ -385,12 +385,6 @@ constexpr int RAD_KC = 16;                // k per stage (3 stages of ~35 KB: tw
 constexpr int RAD_STAGES = 3;
 constexpr int RAD_THREADS = 32 * (RAD_CW + 1);
 
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
 // Tiles (l, radius tile, column tile), the column tile fastest so that CTAs running side by side
 // read the same W rows (one HBM read, the others from L2).
 template <int TC>
