@@ -460,7 +460,8 @@ static int prepare(ggb_ctx* ctx) {
     a.fin_cnt = g.fin_cnt_d; a.fin_scr = g.fin_scr_d;
     int max_orb = 0;
     for (int ri : g.runs) max_orb = std::max(max_orb, ctx->runs[ri].d.n_orb);
-    a.fin_ob = std::min(FIN_OB, ((n_l + 1) * max_orb + 7) / 8);
+    // one row per warp while all runs' blocks fit on the GPU about three times over
+    a.fin_ob = std::min({FIN_OB, ((n_l + 1) * max_orb + 7) / 8, std::max(8, 3 * FIN_OB / (int)g.runs.size())});
     a.obs_parts = ctx->dims.precision == GGB_SPLIT_INT8 ? 1 : 2;
     // the int8 form's initial density is summed over the lane groups of its own tiles (4 of 32 radii,
     // 8 of 16), so that its potentials do not depend on the FP64 kernel's tile
@@ -621,7 +622,7 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
     if ((rc = dalloc(ctx, &g.r_d, nr)) || (rc = dalloc(ctx, &g.drdx_d, nr)) || (rc = dalloc(ctx, &g.P_d, nr)) ||
         (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (dims->precision != GGB_FP64 && (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles))) ||
         (rc = dalloc(ctx, &g.step_d, 1)) || (rc = dalloc(ctx, &g.done_d, 1)) ||
-        (rc = dalloc(ctx, &g.fin_cnt_d, g.runs.size())) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
+        (rc = dalloc(ctx, &g.fin_cnt_d, nc)) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
         (rc = dalloc(ctx, &g.col_run_d, nc)) || (rc = dalloc(ctx, &g.col_m_d, nc)) ||
         (rc = dalloc(ctx, &g.col_occ_d, nc)) || (rc = dalloc(ctx, &g.runs_d, g.runs.size())))
       return bad(rc, "alloc");
@@ -729,7 +730,7 @@ int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const
   CK(cudaMemset(r.vexc0_d, 0, nr * sizeof(double)));
   CK(cudaMemset(g.step_d, 0, sizeof(int)));
   CK(cudaMemset(g.done_d, 0, sizeof(unsigned)));
-  CK(cudaMemset(g.fin_cnt_d, 0, g.runs.size() * sizeof(unsigned)));
+  CK(cudaMemset(g.fin_cnt_d, 0, g.n_cols * sizeof(unsigned)));
   r.orb_set = true;
   g.needs_init = true;
   if (ctx->dims.precision != GGB_FP64 && ctx->prepared) {

@@ -128,7 +128,9 @@ __global__ void k_w_rowmax(const double2* __restrict__ W, int* __restrict__ wexp
 // Operand tiles of the radial product in memory are the shared-memory image of a pipeline stage: per
 // (tile of rows, 32-wide k block) the slice planes one after the other, each [rows][32 bytes] with the
 // 32-byte swizzle already applied (the two 16-byte halves of a row change places in rows 4 .. 7 of every
-// eight), so that a stage is one contiguous copy.  As a [rows][k] matrix a stage was a TMA box of 32-byte
+// eight), so that a stage is one contiguous copy.  The last tiles are only as high as the matrix needs:
+// N_r rounded up to 8 rows of W (the product's further rows are what follows in the buffer, never
+// read from the accumulators), the orbital columns rounded up to 16 (the MMAs' N follows).  As a [rows][k] matrix a stage was a TMA box of 32-byte
 // rows, 1024 and more of them, which paced
 // the copies: 69 -> 53 us for one argon run (N_r 600, N_l 97: 302 MB of W, 5.7 TB/s), 176 -> 155 us for
 // ten, 990 -> 859 us for 21 at N_r 1000, N_l 161.
@@ -138,7 +140,7 @@ __host__ __device__ __forceinline__ uint32_t r8_row_off(int row, int k) {
 
 // A(i,k) tiles, transposed through shared memory (read along i, write along k)
 __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restrict__ wexp, int8_t* __restrict__ Wi8,
-                             int n_r, int rows_pad, int k_pad, int variant, int n_var) {
+                             int n_r, int rows8, int rows_pad, int k_pad, int variant, int n_var) {
   __shared__ double2 t[32][33];
   const int l = blockIdx.z;
   const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
@@ -148,13 +150,14 @@ __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restric
     t[q][tx] = (k < n_r && i < n_r) ? W[((size_t)l * n_r + k) * n_r + i] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  constexpr int PLANE = 128 * 32;                     // one slice plane of a stage
   const int n_kb = k_pad / 32;
   for (int q = ty; q < 32; q += 8) {
     const int i = i0 + q, k = k0 + tx;
-    int8_t* base = Wi8 + (((size_t)l * (rows_pad / 128) + i / 128) * n_kb + k0 / 32) * (2 * I8_SLICES * PLANE) +
+    // the last row tile is rows8 - 128 mt rows high
+    const int mt = i / 128, plane = min(128, rows8 - 128 * mt) * 32;
+    int8_t* base = Wi8 + ((size_t)l * rows8 + 128 * mt) * n_kb * (2 * I8_SLICES * 32) + (size_t)(k0 / 32) * (2 * I8_SLICES) * plane +
                    r8_row_off(i % 128, tx);
-    if (i < rows_pad && k < k_pad) {
+    if (i < rows8 && k < k_pad) {
       const double sc = ldexp(1.0, wexp[(size_t)l * rows_pad + i]);
       const double2 w = t[tx][q];
       const uint32_t h = dither_hash((uint32_t)l, (uint32_t)i, (uint32_t)k);
@@ -163,8 +166,8 @@ __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restric
       slice4_dithered(w.y * sc, dither_offset(variant, n_var, h * 0x165667B1u), si);
 #pragma unroll
       for (int p = 0; p < I8_SLICES; ++p) {
-        base[p * PLANE] = sr[p];
-        base[(I8_SLICES + p) * PLANE] = si[p];
+        base[p * plane] = sr[p];
+        base[(I8_SLICES + p) * plane] = si[p];
       }
     }
   }
@@ -289,9 +292,15 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   volatile int* abort_p = &abort_flag;
+  // rows of a W stage and columns of an x stage: full tiles but for the last ones
+  const int rows8 = (n_r + 7) & ~7, cols16 = (n_cols + 15) & ~15;
+  auto tile_rows = [&](int mt) { return min(R8_BM, rows8 - mt * R8_BM); };
+  auto tile_cols = [&](int nt) { return min(BN, cols16 - nt * BN); };
   // tile order: N tile fastest, so CTAs that share a W tile run side by side (one HBM read)
   auto decode = [&](int tile, int& mt, int& nt, int& l) {
-    nt = tile % n_tiles;
+    // (rotated from round to round where every round would give a CTA the same N tile: the last one
+    // is narrower)
+    nt = (tile + (gridDim.x % n_tiles == 0 ? tile / (int)gridDim.x : 0)) % n_tiles;
     const int rest = tile / n_tiles;
     mt = rest % m_tiles;
     l = rest / m_tiles;
@@ -309,19 +318,20 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
         int mt, nt, l;
         decode(tile, mt, nt, l);
-        for (int kb = 0; kb < n_k_blocks; ++kb, ++it) {
+        const uint32_t wb = R8_W_PLANES * R8_BK * tile_rows(mt), xb = R8_X_PLANES * R8_BK * tile_cols(nt);
+        const int8_t* wsrc = Wv + ((size_t)l * rows8 + mt * R8_BM) * n_k_blocks * (R8_W_PLANES * R8_BK);
+        const int8_t* xsrc = X + ((size_t)l * cols16 + nt * BN) * n_k_blocks * (R8_X_PLANES * R8_BK);
+        for (int kb = 0; kb < n_k_blocks; ++kb, ++it, wsrc += wb, xsrc += xb) {
           const int s = it % stages;
           if (it >= stages && !mbar_wait(&empty_bar[s], ((it / stages) & 1) ^ 1, abort_p)) {
             ok = false;
             break;
           }
           uint8_t* st = smem + (size_t)s * T::STAGE;
-          mbar_expect_tx(&full_bar[s], T::STAGE);
-          const int8_t* wsrc = Wv + ((size_t)(l * m_tiles + mt) * n_k_blocks + kb) * T::A_STAGE;
-          if (n_tiles == 1) bulk_g2s_hint(st, wsrc, T::A_STAGE, &full_bar[s], w_policy);
-          else bulk_g2s(st, wsrc, T::A_STAGE, &full_bar[s]);
-          bulk_g2s(st + T::A_STAGE, X + ((size_t)(l * n_tiles + nt) * n_k_blocks + kb) * (T::STAGE - T::A_STAGE),
-                   T::STAGE - T::A_STAGE, &full_bar[s]);
+          mbar_expect_tx(&full_bar[s], wb + xb);
+          if (n_tiles == 1) bulk_g2s_hint(st, wsrc, wb, &full_bar[s], w_policy);
+          else bulk_g2s(st, wsrc, wb, &full_bar[s]);
+          bulk_g2s(st + T::A_STAGE, xsrc, xb, &full_bar[s]);
         }
       }
       if (!ok)
@@ -329,8 +339,6 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc[I8_SLICES] = {idesc_i8(R8_BM, 4 * BN), idesc_i8(R8_BM, 3 * BN), idesc_i8(R8_BM, 2 * BN),
-                                          idesc_i8(R8_BM, BN)};
       // descriptors: those of stage 0 plus the byte offset / 16 in the start-address field (this
       // thread's issue rate paces the products)
       const uint64_t desc0 = sdesc_kmajor(smem_u32(smem), 32, 6);
@@ -341,6 +349,11 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
         if (use >= 1 && !mbar_wait(&acce_bar[buf], (use - 1) & 1, abort_p)) break;
         tc_fence_after();
         const uint32_t d0 = tmem + buf * T::ACC_COLS;
+        int mt, nt, l;
+        decode(tile, mt, nt, l);
+        const uint32_t bn = tile_cols(nt), wp = tile_rows(mt) * R8_BK, xp = bn * R8_BK;   // columns, plane sizes
+        const uint32_t idesc[I8_SLICES] = {idesc_i8(R8_BM, 4 * bn), idesc_i8(R8_BM, 3 * bn), idesc_i8(R8_BM, 2 * bn),
+                                           idesc_i8(R8_BM, bn)};
         bool ok = true;
         for (int kb = 0; kb < n_k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[s], ph, abort_p)) {
@@ -350,16 +363,16 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
           tc_fence_after();
           const uint64_t da = desc0 + (uint64_t)(((uint32_t)s * T::STAGE) >> 4);
           // one 32-wide k block: for each W slice j, one MMA per real product covers the x slices
-          // m = 0 .. 3 - j at once (the x planes of each kind are contiguous rows), N = (4 - j) BN,
+          // m = 0 .. 3 - j at once (the x planes of each kind are contiguous rows), N = (4 - j) bn,
           // written from accumulator group j on, so that column group m lands on weight 2^-8(j+m)
           const uint64_t xr = da + (T::A_STAGE >> 4);
-          const uint64_t xi = xr + ((I8_SLICES * T::B_PLANE) >> 4);
-          const uint64_t xn = xr + ((2 * I8_SLICES * T::B_PLANE) >> 4);
+          const uint64_t xi = xr + ((I8_SLICES * xp) >> 4);
+          const uint64_t xn = xr + ((2 * I8_SLICES * xp) >> 4);
 #pragma unroll
           for (int j = 0; j < I8_SLICES; ++j) {
-            const uint64_t wr = da + ((j * T::A_PLANE) >> 4);
-            const uint64_t wi = da + (((I8_SLICES + j) * T::A_PLANE) >> 4);
-            const uint32_t dre = d0 + j * BN, dim = d0 + (4 + j) * BN;
+            const uint64_t wr = da + ((j * wp) >> 4);
+            const uint64_t wi = da + (((I8_SLICES + j) * wp) >> 4);
+            const uint32_t dre = d0 + j * bn, dim = d0 + (4 + j) * bn;
             const uint32_t first = (kb == 0 && j == 0) ? 0u : 1u;
             tc_mma_i8(dre, wr, xr, idesc[j], first);
             tc_mma_i8(dre, wi, xn, idesc[j], 1u);
@@ -391,13 +404,14 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
       const int i = mt * R8_BM + 32 * q + lane, c0 = nt * BN;
       const int ew = (i < n_r) ? wexp[(size_t)l * rows_pad + i] : 0;
       const uint32_t d0 = tmem + buf * T::ACC_COLS + lane_base;
+      const int bn = tile_cols(nt), used = min(bn, n_cols - c0);
 #pragma unroll 1
-      for (int cc = 0; cc < BN; cc += 8) {
+      for (int cc = 0; cc < used; cc += 8) {
         uint32_t re[4][8], im[4][8];
 #pragma unroll
         for (int sidx = 0; sidx < 4; ++sidx) {
-          tmem_ld8(d0 + sidx * BN + cc, re[sidx]);
-          tmem_ld8(d0 + (4 + sidx) * BN + cc, im[sidx]);
+          tmem_ld8(d0 + sidx * bn + cc, re[sidx]);
+          tmem_ld8(d0 + (4 + sidx) * bn + cc, im[sidx]);
         }
         tmem_ld_wait();
 #pragma unroll
@@ -985,9 +999,10 @@ k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int 
   const int f = row_exponent(mx);
   if (threadIdx.x == 0) xexp[(size_t)l * cols_pad + col] = f;
   const double sc = pow2i(f);
-  // stage (l, column tile, k block): 12 planes of [bn][32 bytes]
-  const int nt = col / bn, row_in = col - nt * bn, plane = bn * 32;
-  int8_t* xt = X + (size_t)(l * (cols_pad / bn) + nt) * (k_pad / 32) * (R8_X_PLANES * plane);
+  // stage (l, column tile, k block): 12 planes of [columns of the tile][32 bytes]
+  const int cols16 = (n_cols + 15) & ~15;
+  const int nt = col / bn, row_in = col - nt * bn, plane = min(bn, cols16 - nt * bn) * 32;
+  int8_t* xt = X + ((size_t)l * cols16 + nt * bn) * (k_pad / 32) * (R8_X_PLANES * 32);
   // four radii per thread and plane: one 32-bit store each
   for (int r4 = 4 * threadIdx.x; r4 < n_r; r4 += 4 * SX_THREADS) {
     uint32_t pr[I8_SLICES], pi[I8_SLICES], pn[I8_SLICES], wr[4], wi[4], wn[4];
@@ -1050,14 +1065,15 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   q.stages = r8_stages(q.bn);
   if (q.tune_stages > 0) q.stages = std::min(q.tune_stages, q.stages);
   // W planes and row exponents
-  const size_t nw = (size_t)n_l * R8_W_PLANES * mg.rows_pad * mg.k_pad;    // one variant
+  const int rows8 = (n_r + 7) & ~7;
+  const size_t nw = (size_t)n_l * R8_W_PLANES * rows8 * mg.k_pad;    // one variant
   q.w_variant = nw;
   I8_CK(cudaMalloc(&q.W, nw * I8_W_VARIANTS));
   I8_CK(cudaMalloc(&q.wexp, (size_t)n_l * mg.rows_pad * sizeof(int)));
   k_w_rowmax<<<dim3((mg.rows_pad + 127) / 128, n_l), 128>>>(W_fp64, q.wexp, n_r, mg.rows_pad);
   const dim3 tb(32, 8), tg((mg.rows_pad + 31) / 32, (mg.k_pad + 31) / 32, n_l);
   for (int v = 0; v < I8_W_VARIANTS; ++v)
-    k_slice_w_i8<<<tg, tb>>>(W_fp64, q.wexp, q.W + nw * v, n_r, mg.rows_pad, mg.k_pad, v, I8_W_VARIANTS);
+    k_slice_w_i8<<<tg, tb>>>(W_fp64, q.wexp, q.W + nw * v, n_r, rows8, mg.rows_pad, mg.k_pad, v, I8_W_VARIANTS);
   I8_CK(cudaGetLastError());
   // radial B operand planes
   const size_t nx = (size_t)n_l * R8_X_PLANES * q.cols_pad * mg.k_pad;

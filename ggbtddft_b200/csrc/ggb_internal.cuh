@@ -109,7 +109,7 @@ struct GroupArgs {
   unsigned* done;           // block counter for the last-block step increment
   int fin_ob;               // observables blocks per run
   int den_groups;           // lane groups of the FP64 angular kernel's density sums (0: as many as fit)
-  unsigned* fin_cnt;        // [n_runs] finished observables blocks of the step (last-block totals)
+  unsigned* fin_cnt;        // [n_cols] finished observables rows of the step
   double* fin_scr;          // [n_cols][N_l + 1][5] row sums of the observables (hi, lo); row N_l: the norm
   Chain chain[3];   // first half, second half, empty (initial partials)
 };

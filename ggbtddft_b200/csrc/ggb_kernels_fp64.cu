@@ -863,8 +863,8 @@ __host__ __device__ inline int fin_xc_blocks(const GroupArgs& g, int mode) {
 // one column on 200 radii and 25 us for nine on 600).  Otherwise from the partial sums per tile of
 // radii that the int8 and BF16 angular kernels leave (an eighth of the orbitals' bytes: the orbitals
 // of an ensemble are not in L2), with one more row per orbital for the norm, from the density.  The
-// rows' sums go to a scratch array, and the last of the run's blocks to finish (a per-run counter) adds
-// them over l, writes the totals and runs the NaN / norm-growth watchdog.  (Blocks that took a slice of
+// rows' sums go to a scratch array, and the last of an orbital's rows to finish (a counter per orbital)
+// adds them over l, writes the totals and runs the NaN / norm-growth watchdog.  (Blocks that took a slice of
 // l with one warp per orbital walked its rows one after another: 27 us for nine orbitals, N_l 97, and
 // 88 us for 21 such runs at N_l 161, now 14 and 47 us.)
 // ROWS: the observables come from the orbitals x (the partial sums' kernel needs half its registers).
@@ -872,7 +872,7 @@ template <bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
   extern __shared__ double fsm[];  // [2][N_r]
   __shared__ dd wsum[FIN_THREADS / 32][2];
-  __shared__ int s_last, s_step;
+  __shared__ int s_step;
   const int n_xc = fin_xc_blocks(g, mode);
   const int nb = g.n_den + n_xc + g.fin_ob;
   const int ri = blockIdx.x / nb;
@@ -902,7 +902,43 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
     const int n_orb = run.n_orb;
     double2* scr = reinterpret_cast<double2*>(g.fin_scr);     // [col][N_l + 1][5]; row N_l: the norm
     const int rows = n_l * n_orb + (ROWS ? 0 : n_orb);
-    for (int i = ob * (FIN_THREADS / 32) + warp; i < rows; i += g.fin_ob * (FIN_THREADS / 32)) {
+    auto sum_rows = [&](int k) {
+      const int col = run.col0 + k;
+      double2* o = scr + (size_t)col * (n_l + 1) * 5;
+      dd s[5];
+      int last = 0;
+      if (lane == 0) last = atomicAdd(g.fin_cnt + col, 1u) == (unsigned)(n_l - (ROWS ? 1 : 0));
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        __threadfence();
+#pragma unroll
+        for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
+        for (int lp = lane; lp < n_l + (ROWS ? 0 : 1); lp += 32)
+#pragma unroll
+          for (int q = 0; q < 5; ++q) {
+            const double2 v = __ldcg(o + (size_t)lp * 5 + q);
+            sum2_add(s[q], dd{v.x, v.y});
+          }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
+        const double nrm = s[4].hi + s[4].lo;
+        if (lane == 0) {
+          if (mode == 0) {
+            run.norm0[k] = nrm;                 // for the growth watchdog
+          } else {
+            run.dip_tot[(size_t)k * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
+            run.acc_tot[(size_t)k * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
+            run.norm[(size_t)k * run.n_t + step] = nrm;
+            if (mode == 1) {
+              if (!(nrm == nrm) || isinf(nrm) || !(s[0].hi == s[0].hi) || !(s[2].hi == s[2].hi)) atomicOr(g.status, ST_NAN);
+              if (nrm > run.norm0[k] * (1.0 + g.norm_tol) + 1e-300) atomicOr(g.status, ST_NORM_GROWTH);
+            }
+          }
+          g.fin_cnt[col] = 0u;                  // for the next launch (stream-ordered after this one)
+        }
+      }
+    };
+    const int i0 = ob * (FIN_THREADS / 32) + warp, stride = g.fin_ob * (FIN_THREADS / 32);
+    for (int i = i0; i < rows; i += stride) {
       const int l = i / n_orb, k = i - l * n_orb;
       dd s[5];
       if constexpr (ROWS) {
@@ -927,51 +963,23 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
           for (int q = 0; q < 4; ++q) sum2_warp(s[q]);
         }
       }
+      const int col = run.col0 + k;
+      double2* o = scr + (size_t)col * (n_l + 1) * 5;
       if (lane == 0) {
         if (mode != 0 && g.per_l && l < n_l) {
           run.dip[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
           run.acc[((size_t)l * n_orb + k) * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
         }
-        double2* o = scr + ((size_t)(run.col0 + k) * (n_l + 1) + l) * 5;
 #pragma unroll
-        for (int q = 0; q < 5; ++q) o[q] = make_double2(s[q].hi, s[q].lo);
+        for (int q = 0; q < 5; ++q) o[l * 5 + q] = make_double2(s[q].hi, s[q].lo);
       }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      s_last = atomicAdd(g.fin_cnt + ri, 1u) == (unsigned)(g.fin_ob - 1);
-    }
-    __syncthreads();
-    if (s_last) {
-      __threadfence();
-      // totals over l, the norm; one warp per orbital
-      for (int k = warp; k < n_orb; k += FIN_THREADS / 32) {
-        dd s[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
-        const double2* o = scr + (size_t)(run.col0 + k) * (n_l + 1) * 5;
-        for (int l = lane; l < n_l + (ROWS ? 0 : 1); l += 32)
-#pragma unroll
-          for (int q = 0; q < 5; ++q) {
-            const double2 v = __ldcg(o + (size_t)l * 5 + q);
-            sum2_add(s[q], dd{v.x, v.y});
-          }
-#pragma unroll
-        for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
-        const double nrm = s[4].hi + s[4].lo;
-        if (lane == 0 && mode == 0) run.norm0[k] = nrm;   // for the growth watchdog
-        if (lane == 0 && mode != 0) {
-          run.dip_tot[(size_t)k * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
-          run.acc_tot[(size_t)k * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
-          run.norm[(size_t)k * run.n_t + step] = nrm;
-          if (mode == 1) {
-            if (!(nrm == nrm) || isinf(nrm) || !(s[0].hi == s[0].hi) || !(s[2].hi == s[2].hi)) atomicOr(g.status, ST_NAN);
-            if (nrm > run.norm0[k] * (1.0 + g.norm_tol) + 1e-300) atomicOr(g.status, ST_NORM_GROWTH);
-          }
-        }
+      if (i + stride < rows) continue;
+      // one fence for this warp's rows, then each counts; the last of an orbital's rows adds the totals
+      if (lane == 0) __threadfence();
+      for (int ii = i0; ii <= i; ii += stride) {
+        const int kk = ii == i ? k : ii % n_orb;
+        sum_rows(kk);
       }
-      if (tid == 0) g.fin_cnt[ri] = 0u;   // for the next launch (stream-ordered after this one)
     }
   }
 

@@ -20,10 +20,10 @@ constexpr unsigned ST_TC_TIMEOUT = 8u;   // a bounded wait in a tensor-core kern
 // Integer-split form (ggb_int8.cu): int8 slice planes of W, of the chain matrices and of the radial
 // B operand, with per-row power-of-two exponents of the constant operators.
 struct I8Group {
-  int8_t* W = nullptr;       // [variant][N_l][row tile][k block][8][128][32]: Wr slices 1-4, Wi slices 1-4; A(i,k) = W[l][k][i] 2^e(l,i)
+  int8_t* W = nullptr;       // [variant][N_l][row tile][k block][8][rows of the tile][32]: Wr slices 1-4, Wi slices 1-4; A(i,k) = W[l][k][i] 2^e(l,i)
   size_t w_variant = 0;      // bytes of one variant
   int* wexp = nullptr;       // [N_l][rows_pad]
-  int8_t* X = nullptr;       // [N_l][column tile][k block][12][bn][32]: Xr, Xi, -Xi slices 1-4 of x 2^xexp(l, col)
+  int8_t* X = nullptr;       // [N_l][column tile][k block][12][columns of the tile][32]: Xr, Xi, -Xi slices 1-4 of x 2^xexp(l, col)
   int* xexp = nullptr;       // [N_l][cols_pad]
   int8_t* St = nullptr;      // [variant][mat][m][4][rows][lk]: S^T slices, rows scaled by 2^sexp
   int n_mats = 0;            // chain matrices per variant
