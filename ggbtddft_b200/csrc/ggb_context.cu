@@ -22,6 +22,8 @@ using namespace ggb;
 
 namespace {
 
+constexpr int COUNTERS = 4;       // ints before the row counters of a group's counter block
+
 struct GroupHost {
   ggb_group_desc d{};
   int n_cols = 0, n_tiles = 0, obs_seg = TR, ldS = 0;
@@ -40,9 +42,9 @@ struct GroupHost {
   int *col_run_d = nullptr, *col_m_d = nullptr, *col_occ_d = nullptr, *runs_d = nullptr;
   double* dens_d = nullptr;
   double4* obs_d = nullptr;
+  // step counter, k_finalize's block counter, the basis reuse's step, then k_finalize's row counters: one
+  // block that set_orbitals clears
   int* step_d = nullptr;
-  unsigned* done_d = nullptr;
-  unsigned* fin_cnt_d = nullptr;
   double* fin_scr_d = nullptr;
   bool needs_init = true;
   GroupArgs args{};
@@ -63,7 +65,8 @@ struct RunHost {
   double *rho_frozen_d = nullptr, *norm_d = nullptr, *norm0_d = nullptr;
   double2 *dip_d = nullptr, *acc_d = nullptr, *dip_tot_d = nullptr, *acc_tot_d = nullptr;
   double* htab_d = nullptr;      // theta form with n_har > 4
-  std::vector<int> l, m, occ;
+  std::vector<int> l, m, occ;            // as last set
+  std::vector<double> rho_frozen;
 };
 
 }  // namespace
@@ -456,8 +459,10 @@ static int prepare(ggb_ctx* ctx) {
     a.mats = g.mats_d; a.frag = g.frag_d; a.dph = g.dph_d; a.coef = g.coef_d;
     a.col_run = g.col_run_d; a.col_m = g.col_m_d; a.col_occ = g.col_occ_d; a.runs_of_group = g.runs_d;
     a.runs = ctx->runs_dev;
-    a.dens = g.dens_d; a.obs = g.obs_d; a.step = g.step_d; a.status = ctx->status_d; a.done = g.done_d;
-    a.fin_cnt = g.fin_cnt_d; a.fin_scr = g.fin_scr_d;
+    a.dens = g.dens_d; a.obs = g.obs_d; a.step = g.step_d; a.status = ctx->status_d;
+    a.done = (unsigned*)g.step_d + 1;
+    a.yth_step = g.step_d + 2;
+    a.fin_cnt = (unsigned*)g.step_d + COUNTERS; a.fin_scr = g.fin_scr_d;
     int max_orb = 0;
     for (int ri : g.runs) max_orb = std::max(max_orb, ctx->runs[ri].d.n_orb);
     // one row per warp while all runs' blocks fit on the GPU about three times over
@@ -621,8 +626,7 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
     const size_t nr = g.d.n_r, nl = g.d.n_l, nc = g.n_cols;
     if ((rc = dalloc(ctx, &g.r_d, nr)) || (rc = dalloc(ctx, &g.drdx_d, nr)) || (rc = dalloc(ctx, &g.P_d, nr)) ||
         (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (dims->precision != GGB_FP64 && (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles))) ||
-        (rc = dalloc(ctx, &g.step_d, 1)) || (rc = dalloc(ctx, &g.done_d, 1)) ||
-        (rc = dalloc(ctx, &g.fin_cnt_d, nc)) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
+        (rc = dalloc(ctx, &g.step_d, COUNTERS + nc)) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
         (rc = dalloc(ctx, &g.col_run_d, nc)) || (rc = dalloc(ctx, &g.col_m_d, nc)) ||
         (rc = dalloc(ctx, &g.col_occ_d, nc)) || (rc = dalloc(ctx, &g.runs_d, g.runs.size())))
       return bad(rc, "alloc");
@@ -640,12 +644,14 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
   for (RunHost& r : ctx->runs) {
     const GroupHost& g = ctx->groups[r.d.group];
     const size_t nr = g.d.n_r, nl = g.d.n_l, no = r.d.n_orb, nt = dims->n_t;
-    if ((rc = dalloc(ctx, &r.E_d, nt)) || (rc = dalloc(ctx, &r.v_d, 4 * nr)) || (rc = dalloc(ctx, &r.v0_d, nr)) ||
-        (rc = dalloc(ctx, &r.vexc_d, nr)) || (rc = dalloc(ctx, &r.vexc0_d, nr)) ||
-        (rc = dalloc(ctx, &r.rho_frozen_d, nr)) || (rc = dalloc(ctx, &r.norm_d, no * nt)) ||
+    // v[4], v0, vexc, vexc0 in one block: set_orbitals clears them together
+    if ((rc = dalloc(ctx, &r.E_d, nt)) || (rc = dalloc(ctx, &r.v_d, 7 * nr)) || (rc = dalloc(ctx, &r.rho_frozen_d, nr)) || (rc = dalloc(ctx, &r.norm_d, no * nt)) ||
         (rc = dalloc(ctx, &r.norm0_d, no)) || (rc = dalloc(ctx, &r.dip_tot_d, no * nt)) ||
         (rc = dalloc(ctx, &r.acc_tot_d, no * nt)))
       return bad(rc, "alloc");
+    r.v0_d = r.v_d + 4 * nr;
+    r.vexc_d = r.v_d + 5 * nr;
+    r.vexc0_d = r.v_d + 6 * nr;
     if (dims->per_l)
       if ((rc = dalloc(ctx, &r.dip_d, nl * no * nt)) || (rc = dalloc(ctx, &r.acc_d, nl * no * nt)))
         return bad(rc, "alloc");
@@ -701,6 +707,15 @@ int ggb_set_angular(ggb_ctx* ctx, int group, int coupling, int m, const double* 
   return GGB_OK;
 }
 
+// Copies `bytes` from a host or device pointer to host memory (plain host memory without a driver call).
+static int to_host(ggb_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  cudaPointerAttributes at;
+  CK(cudaPointerGetAttributes(&at, src));
+  if (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost) std::memcpy(dst, src, bytes);
+  else CK(cudaMemcpy(dst, src, bytes, cudaMemcpyDefault));
+  return GGB_OK;
+}
+
 int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const int* m, const int* occ,
                      const double* rho_frozen) {
   if (!ctx) return GGB_ERR_ARG;
@@ -709,34 +724,44 @@ int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const
   RunHost& r = ctx->runs[run];
   GroupHost& g = ctx->groups[r.d.group];
   const int no = r.d.n_orb, nr = g.d.n_r, nl = g.d.n_l;
-  r.l.assign(no, 0); r.m.assign(no, 0); r.occ.assign(no, 0);
-  CK(cudaMemcpy(r.l.data(), l, no * sizeof(int), cudaMemcpyDefault));
-  CK(cudaMemcpy(r.m.data(), m, no * sizeof(int), cudaMemcpyDefault));
-  CK(cudaMemcpy(r.occ.data(), occ, no * sizeof(int), cudaMemcpyDefault));
+  // a scan restarts hundreds of runs: what the device already holds (same l, m, occupations and frozen
+  // density, compared by value) is not sent again, and each run costs one copy, two clears and one wait
+  std::vector<int> nl_(no), nm(no), nocc(no);
+  std::vector<double> rho(nr);
+  int rc;
+  if ((rc = to_host(ctx, nl_.data(), l, no * sizeof(int))) || (rc = to_host(ctx, nm.data(), m, no * sizeof(int))) ||
+      (rc = to_host(ctx, nocc.data(), occ, no * sizeof(int))) ||
+      (rc = to_host(ctx, rho.data(), rho_frozen, nr * sizeof(double))))
+    return rc;
   for (int k = 0; k < no; ++k)
-    if (r.m[k] < 0 || r.m[k] >= g.d.n_m || r.l[k] < r.m[k] || r.l[k] >= nl)
-      return fail(ctx, GGB_ERR_ARG, "orbital %d: l=%d m=%d outside 0<=m<N_m, m<=l<N_l", k, r.l[k], r.m[k]);
-  CK(cudaMemcpy(g.col_m_d + r.col0, r.m.data(), no * sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(g.col_occ_d + r.col0, r.occ.data(), no * sizeof(int), cudaMemcpyHostToDevice));
-  std::vector<int> cr(no, run);
-  CK(cudaMemcpy(g.col_run_d + r.col0, cr.data(), no * sizeof(int), cudaMemcpyHostToDevice));
+    if (nm[k] < 0 || nm[k] >= g.d.n_m || nl_[k] < nm[k] || nl_[k] >= nl)
+      return fail(ctx, GGB_ERR_ARG, "orbital %d: l=%d m=%d outside 0<=m<N_m, m<=l<N_l", k, nl_[k], nm[k]);
+  if (!r.orb_set || nm != r.m || nocc != r.occ) {
+    std::vector<int> cr(no, run);
+    CK(cudaMemcpy(g.col_m_d + r.col0, nm.data(), no * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(g.col_occ_d + r.col0, nocc.data(), no * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(g.col_run_d + r.col0, cr.data(), no * sizeof(int), cudaMemcpyHostToDevice));
+  }
+  // (bytes: a NaN or a signed zero is sent again only where it changes)
+  if (!r.orb_set || std::memcmp(rho.data(), r.rho_frozen.data(), nr * sizeof(double)) != 0)
+    CK(cudaMemcpy(r.rho_frozen_d, rho.data(), nr * sizeof(double), cudaMemcpyHostToDevice));
+  r.l.swap(nl_);
+  r.m.swap(nm);
+  r.occ.swap(nocc);
+  r.rho_frozen.swap(rho);
   // x[l][kso][r] -> group x[l][col0 + kso][r]
   CK(cudaMemcpy2D(g.x_d + (size_t)r.col0 * nr, (size_t)g.n_cols * nr * sizeof(double2), x,
                   (size_t)no * nr * sizeof(double2), (size_t)no * nr * sizeof(double2), nl, cudaMemcpyDefault));
-  CK(cudaMemcpy(r.rho_frozen_d, rho_frozen, nr * sizeof(double), cudaMemcpyDefault));
-  CK(cudaMemset(r.v_d, 0, 4 * (size_t)nr * sizeof(double)));
-  CK(cudaMemset(r.v0_d, 0, nr * sizeof(double)));
-  CK(cudaMemset(r.vexc_d, 0, nr * sizeof(double)));
-  CK(cudaMemset(r.vexc0_d, 0, nr * sizeof(double)));
-  CK(cudaMemset(g.step_d, 0, sizeof(int)));
-  CK(cudaMemset(g.done_d, 0, sizeof(unsigned)));
-  CK(cudaMemset(g.fin_cnt_d, 0, g.n_cols * sizeof(unsigned)));
+  CK(cudaMemsetAsync(r.v_d, 0, 7 * (size_t)nr * sizeof(double), 0));
+  CK(cudaMemsetAsync(g.step_d, 0, (COUNTERS + (size_t)g.n_cols) * sizeof(int), 0));
   r.orb_set = true;
   g.needs_init = true;
-  if (ctx->dims.precision != GGB_FP64 && ctx->prepared) {
-    int rc = mixed_load_orbitals(g.mixed, g.args, g.x_d);
+  if (ctx->dims.precision == GGB_SPLIT_BF16 && ctx->prepared) {
+    rc = mixed_load_orbitals(g.mixed, g.args, g.x_d);
     if (rc) return fail(ctx, rc, "orbital conversion failed");
   }
+  // set-up calls are synchronous: the caller may reuse x, and may step on any stream
+  CK(cudaStreamSynchronize(0));
   return GGB_OK;
 }
 
@@ -757,7 +782,7 @@ int ggb_step(ggb_ctx* ctx, int n_steps, void* stream) {
   const bool was_prepared = ctx->prepared;
   int rc = prepare(ctx);
   if (rc) return rc;
-  if (!was_prepared && ctx->dims.precision != GGB_FP64)
+  if (!was_prepared && ctx->dims.precision == GGB_SPLIT_BF16)
     for (GroupHost& g : ctx->groups)
       if ((rc = mixed_load_orbitals(g.mixed, g.args, g.x_d))) return fail(ctx, rc, "orbital conversion failed");
   for (GroupHost& g : ctx->groups)

@@ -471,9 +471,8 @@ struct Ang8Args {
   int n_mats;             // chain matrices per variant
   int n_var;              // dithered variants of the chain matrices (a power of two)
   // theta form: the node-basis vectors of the second half after its phase, [N_l][n_cols][N_r]
-  // (nullptr: not kept), and the step whose first half may start from them (-1: none)
+  // (nullptr: not kept); g.yth_step says which step's first half may start from them
   double2* yth;
-  int* yth_step;
 };
 
 // Byte offset of (row n, k) of slice plane 0 in the B operand: per 128-wide k atom, the four slice
@@ -527,8 +526,8 @@ __device__ __forceinline__ double2 rotd(double2 x, double e) {
 // the second half's node-basis vector after its phase, which the second half keeps (t.yth, one
 // FP64 copy); the next first half loads it, applies its own phase in the prologue and runs only
 // its last product, one product instead of two.  The skipped pair V^T V is the identity up to the
-// int8 operands' rounding (~2^-31 of each row), which is then not applied.  t.yth_step names the
-// step that may start from the kept vectors; setting orbitals invalidates it.
+// int8 operands' rounding (~2^-31 of each row), which is then not applied.  g.yth_step names the
+// step that may start from the kept vectors; setting orbitals clears it.
 template <int NP, bool SECOND_HALF, bool THETA>
 __global__ void __launch_bounds__(A8_THREADS, 2)
 k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
@@ -561,7 +560,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   // basis reuse: the second half keeps its node-basis vectors, the first half of the step they
   // were kept for starts from them at its last product (o0 = 1, the theta chain having two)
   const bool keep_theta = THETA && SECOND_HALF && t.yth != nullptr;
-  const bool from_theta = THETA && !SECOND_HALF && t.yth != nullptr && *t.yth_step == step_raw;
+  const bool from_theta = THETA && !SECOND_HALF && t.yth != nullptr && *g.yth_step == step_raw + 1;
   const int o0 = from_theta ? 1 : 0;
 
   // the x tile (all l, NP points): point fp = tid % NP, the l quads fg, fg + FG, ... of this thread, all
@@ -884,7 +883,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   } else {
     // the kept vectors serve the first half of the next step (the step counter advances once
     // per step, after this kernel)
-    if (keep_theta && blockIdx.x == 0 && threadIdx.x == 0) *t.yth_step = step_raw + 1;
+    if (keep_theta && blockIdx.x == 0 && threadIdx.x == 0) *g.yth_step = step_raw + 2;
     const double2* xs = reinterpret_cast<const double2*>(smem);
     for (int idx = threadIdx.x; idx < n_l * NP; idx += A8_THREADS) {
       const int l = idx / NP, p = idx - l * NP, r = r0 + p;
@@ -1126,8 +1125,6 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   // products on the FP64 kernel keep the full chain
   if (q.theta_reuse && a.theta && !mg.angular_fp64 && a.chain[0].n_ops == 2 && a.chain[1].n_ops == 2) {
     I8_CK(cudaMalloc(&q.yth, (size_t)n_l * a.n_cols * n_r * sizeof(double2)));
-    I8_CK(cudaMalloc(&q.yth_step, sizeof(int)));
-    I8_CK(cudaMemset(q.yth_step, 0xFF, sizeof(int)));   // -1: nothing kept yet
   }
   {
     // the variants follow one another along the matrix index: matrix mat of variant v is mat + v n_mats
@@ -1190,7 +1187,6 @@ void int8_angular(MixedGroup& mg, const GroupArgs& a, int half, const double2* x
   t.n_mats = q.n_mats;
   t.n_var = I8_S_VARIANTS;
   t.yth = q.yth;
-  t.yth_step = q.yth_step;
   const dim3 grid(a.n_cols * ((a.n_r + q.np - 1) / q.np));
 #define GGB_A8(NP, SH, TH) k_angular_i8<NP, SH, TH><<<grid, A8_THREADS, q.a_smem, s>>>(q.tmS, a, t, xin, xout)
   if (q.np == 32) {
@@ -1216,7 +1212,6 @@ void int8_release(I8Group& q) {
   cudaFree(q.St);
   cudaFree(q.sexp);
   cudaFree(q.yth);
-  cudaFree(q.yth_step);
   q = I8Group();
 }
 

@@ -104,7 +104,9 @@ struct GroupArgs {
   RunDev* runs;             // ctx-wide device array
   double* dens;
   double4* obs;
-  int* step;                // ctx-wide step counter
+  int* step;                // the group's step counter
+  int* yth_step;            // int8 theta form, basis reuse: 1 + the step whose first half may start from the
+                            //   kept node-basis vectors (0: none)
   unsigned* status;
   unsigned* done;           // block counter for the last-block step increment
   int fin_ob;               // observables blocks per run
