@@ -27,7 +27,7 @@
 //   int32 range: |a b| <= 2^14, at most 8 products per k and accumulator, K <= 8192: <= 2^30.
 //
 //  k_slice_w_i8      W[l][k][i] -> A(i,k) stages [variant][l][row tile][k block][8][128][32] (Wr a1..a4, Wi a1..a4) + exponents
-//  k_build_st_i8     chain matrices -> S^T planes [variant n_mats + mat][m][4][rows][lk] + exponents
+//  k_build_st_i8     chain matrices -> S^T stage images [variant n_mats + mat][m] + exponents
 //  k_slice_x         orbitals (complex128) -> radial B operand stages (Xr, Xi, -Xi) + exponents
 //  k_radial_i8       persistent radial product, kind::i8, 32-byte swizzle, 16 MMAs per 32-wide k block
 //                    (each covers all x slices m of one W slice j):
@@ -173,9 +173,45 @@ __global__ void k_slice_w_i8(const double2* __restrict__ W, const int* __restric
   }
 }
 
-// S^T planes of the chain matrices: St[mat][m][slice][j][l] with the row (j) exponents
+// S^T planes of the chain matrices as the shared-memory images of the angular kernel's stages: per
+// (variant, mat, m), per M tile of 128 rows (channels j) and k atom of 128 (l), the four slice planes
+// [rows][pitch bytes], K-major, the swizzle of that pitch applied.  Only what the products need: the rows
+// rounded up to 8, the k atom's 32-wide steps (pitch 32, 64 or 128; three steps take 128).  N_l = 161:
+// 126 KB a matrix where full 128 x 128 tiles are 256, and these copies (one matrix per 16 radii, product
+// and orbital) were at what L2 delivers to the SMs.
+struct StGeom {
+  int rows8, k_steps, psum;           // rows, 32-wide k steps, sum of the atoms' pitches
+  __host__ __device__ int rows(int mt) const { return rows8 - 128 * mt < 128 ? rows8 - 128 * mt : 128; }
+  __host__ __device__ int pitch(int ka) const {
+    const int nk = k_steps - 4 * ka;
+    return nk <= 0 ? 0 : nk == 1 ? 32 : nk == 2 ? 64 : 128;
+  }
+  __host__ __device__ size_t tile(int mt, int ka) const {   // offset of a tile's first plane
+    return (size_t)4 * (128 * mt * psum + (ka ? rows(mt) * pitch(0) : 0));
+  }
+  __host__ __device__ size_t bytes() const { return (size_t)4 * rows8 * psum; }
+  static StGeom of(int n_l) {
+    StGeom g{(n_l + 7) & ~7, (n_l + 31) / 32, 0};
+    g.psum = g.pitch(0) + g.pitch(1);
+    return g;
+  }
+};
+// A product's tiles (i = M tile, k atom) pass through the four stages (one per slice plane, 16 KB) in
+// rounds: the first tile, then the three others at once where their planes fit a stage together (N_l = 161:
+// 15.5 KB), else one by one.  A stage is refilled when its products are done, and the copy's latency is
+// waited for between rounds.
+static bool st_one_round(const StGeom& g) {
+  return g.rows(0) * g.pitch(1) + g.rows(1) * (g.pitch(0) + g.pitch(1)) <= 128 * 128;
+}
+// byte of (row, k) in a plane of this pitch
+__device__ __forceinline__ int st_off(int pitch, int row, int k) {
+  const int x = pitch == 128 ? row & 7 : pitch == 64 ? (row >> 1) & 3 : (row >> 2) & 1;
+  return row * pitch + (((k >> 4) ^ x) << 4) + (k & 15);
+}
+
+// S^T images with the row (j) exponents
 __global__ void k_build_st_i8(const double* __restrict__ mats, int8_t* __restrict__ St, int* __restrict__ sexp,
-                              int n_mm, int n_m, int n_l, int ldS, int rows, int lk, int variant, int n_var) {
+                              int n_mm, int n_m, int n_l, int ldS, int rows, StGeom geo, int variant, int n_var) {
   const int row = blockIdx.x;                 // (mat * n_m + m) * rows + j
   const int mm = row / rows, j = row - mm * rows;
   if (mm >= n_mm) return;
@@ -192,14 +228,17 @@ __global__ void k_build_st_i8(const double* __restrict__ mats, int8_t* __restric
   const int e = row_exponent(red[0]);
   if (threadIdx.x == 0 && variant == 0) sexp[row] = e;
   const double sc = ldexp(1.0, e);
-  const size_t plane = (size_t)rows * lk;
-  for (int l = threadIdx.x; l < lk; l += blockDim.x) {
+  if (j >= geo.rows8) return;
+  const int mt = j / 128;
+  for (int l = threadIdx.x; l < 32 * geo.k_steps; l += blockDim.x) {
     const double v = (j < n_l && l < n_l) ? mats[((size_t)mm * n_l + l) * ldS + j] * sc : 0.0;
     int8_t s[I8_SLICES];
     // the hash leaves out m, so that a matrix gets the same variants in any group of runs
     slice4_dithered(v, dither_offset(variant, n_var, dither_hash((uint32_t)(mm / n_m), (uint32_t)j, (uint32_t)l)), s);
+    const int ka = l / 128, pitch = geo.pitch(ka);
+    int8_t* t = St + (size_t)mm * geo.bytes() + geo.tile(mt, ka) + st_off(pitch, j - 128 * mt, l - 128 * ka);
 #pragma unroll
-    for (int p = 0; p < I8_SLICES; ++p) St[(size_t)mm * I8_SLICES * plane + p * plane + (size_t)j * lk + l] = s[p];
+    for (int p = 0; p < I8_SLICES; ++p) t[(size_t)p * geo.rows(mt) * pitch] = s[p];
   }
 }
 
@@ -222,6 +261,15 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
 }
+__device__ __forceinline__ void tc_mma_i8_if(uint32_t elected, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(elected));
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -238,10 +286,8 @@ __device__ __forceinline__ long long combine_int(const uint32_t (&d)[4][W], int 
   return (long long)(int)d[0][u] * 16777216LL + (long long)(int)d[1][u] * 65536LL + (long long)(int)d[2][u] * 256LL +
          (long long)(int)d[3][u];
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-               : "r"(taddr));
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t (&v)[2]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr));
 }
 
 template <int BN>
@@ -454,11 +500,13 @@ k_radial_i8(const int8_t* __restrict__ W, size_t w_variant, const int8_t* __rest
 // angular chain, kind::i8
 // ---------------------------------------------------------------------------------------------
 
-constexpr int A8_THREADS = 320;
+constexpr int A8_THREADS = 576;          // TMA warp, MMA warp, 16 epilogue warps
 constexpr int A8_EPI_WARP0 = 2;
+constexpr int A8_BLOCKS_PER_SM = 2;
 constexpr int A8_KATOM = 128;            // int8 per 128-byte swizzled row
 constexpr int A8_A_TILE = 128 * 128;     // one S^T slice plane: 128 rows (j) x 128 k (l), one stage
-constexpr int A8_PTS = 16;               // points per epilogue thread and product
+constexpr int A8_PTS = 8;                // points per epilogue thread and product
+constexpr int A8_DEN_WARPS = 10;         // warps of the density's partial sums (fixes their order)
 constexpr int A8_TMEM_COLS = 256;        // 4 accumulators x 2 NP columns x m_tiles: two CTAs per SM
 
 struct Ang8Args {
@@ -466,14 +514,23 @@ struct Ang8Args {
   int m_tiles;            // ceil(N_l / 128)
   int k_steps;            // ceil(N_l / 32): 32-wide K steps that carry data
   int stages;
+  const int8_t* St;       // S^T images [variant n_mats + mat][m], geo.bytes() each
+  StGeom geo;
+  int one_round;          // tiles 1 .. 3 pass through the stages together
   const int* sexp;        // S^T row exponents [mat][m][rows]
   int rows;               // m_tiles * 128
+  int sms;
   int n_mats;             // chain matrices per variant
   int n_var;              // dithered variants of the chain matrices (a power of two)
   // theta form: the node-basis vectors of the second half after its phase, [N_l][n_cols][N_r]
   // (nullptr: not kept); g.yth_step says which step's first half may start from them
   double2* yth;
 };
+
+// descriptor of a K-major operand of this row pitch with its swizzle
+__device__ __forceinline__ uint64_t a8_sdesc(uint32_t saddr, int pitch) {
+  return sdesc_kmajor(saddr, (uint32_t)pitch, pitch == 128 ? 2u : pitch == 64 ? 4u : 6u);
+}
 
 // Byte offset of (row n, k) of slice plane 0 in the B operand: per 128-wide k atom, the four slice
 // planes of nrows K-major 128-byte-swizzled rows each, one after the other (plane q at + q nrows 128),
@@ -508,6 +565,29 @@ __device__ __forceinline__ double2 rotd(double2 x, double e) {
   return make_double2(c * x.x + s * x.y, c * x.y - s * x.x);
 }
 
+template <int V>
+struct I8c {
+  static constexpr int value = V;
+};
+// end of the round that starts at tile i
+template <int K_ATOMS>
+__device__ __forceinline__ int a8_round_end(int one_round, int i) {
+  return K_ATOMS == 2 && i > 0 && one_round ? 4 : i + 1;
+}
+// slice plane pa of tiles [i0, i1) into a stage, one after the other
+template <int K_ATOMS>
+__device__ __forceinline__ void a8_load_round(StGeom geo, const int8_t* mat, int i0, int i1, int pa, uint8_t* stage, uint64_t* bar) {
+  uint32_t bytes = 0;
+  for (int i = i0; i < i1; ++i) bytes += geo.rows(i / K_ATOMS) * geo.pitch(i % K_ATOMS);
+  mbar_expect_tx(bar, bytes);
+  for (int i = i0; i < i1; ++i) {
+    const int mt = i / K_ATOMS, ka = i % K_ATOMS;
+    const uint32_t plane = geo.rows(mt) * geo.pitch(ka);
+    bulk_g2s(stage, mat + geo.tile(mt, ka) + pa * plane, plane, bar);
+    stage += plane;
+  }
+}
+
 // One CTA per (orbital column, NP radii): NP = 32 for N_l <= 128 (one M tile of 128 channels),
 // NP = 16 for N_l <= 256 (two M tiles), so that every CTA holds 256 TMEM columns and two CTAs share
 // an SM (one CTA's epilogue overlaps the other's products and loads).
@@ -529,8 +609,8 @@ __device__ __forceinline__ double2 rotd(double2 x, double e) {
 // int8 operands' rounding (~2^-31 of each row), which is then not applied.  g.yth_step names the
 // step that may start from the kept vectors; setting orbitals clears it.
 template <int NP, bool SECOND_HALF, bool THETA>
-__global__ void __launch_bounds__(A8_THREADS, 2)
-k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
+__global__ void __launch_bounds__(A8_THREADS, A8_BLOCKS_PER_SM)
+k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
   constexpr int NB = 2 * NP;                 // B rows: Re of NP points, then Im
   constexpr int B_TILE = NB * 128;           // one slice plane, one k atom
   constexpr int K_ATOMS = NP == 32 ? 1 : 2;  // = M tiles = ceil(N_l / 128)
@@ -542,13 +622,16 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   __shared__ double pbase[5][NP];
   __shared__ double pnorm2[A8_THREADS / NP][NP];
   __shared__ double sdl[MAX_NL];
+  __shared__ double prr[2][NP];               // second half: r and r^-2 of each point (0 past N_r)
   __shared__ double pscale3[NP], pinv[NP];    // 2^e(p) 2^24 and 2^-e(p) of each point's B rows
   // aligned by an offset from the __shared__ array itself, so that the compiler keeps the shared
   // address space (shared loads and stores, not generic ones) for every access through it
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* xb = smem;                                              // 4 planes x k_atoms x B_TILE
-  uint8_t* sst = smem + (size_t)I8_SLICES * XPLANE;                 // stages x 16 KB
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // stages of 16 KB, then the operand: the MMAs read 128 rows of a stage's tile whatever its height, up to
+  // 16 KB past the last stage, which is the operand's memory (what they read there is never used)
+  uint8_t* sst = smem;
+  uint8_t* xb = smem + I8_SLICES * A8_A_TILE;                       // 4 planes x k_atoms x B_TILE, 32 KB
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_l = g.n_l;
   const int tilesN = (g.n_r + NP - 1) / NP;
   const int col = blockIdx.x / tilesN;
@@ -557,6 +640,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   const int n_ops = ch.n_ops;
   const int acc_cols = 4 * NB;                // per M tile: weights 2^0 .. 2^-24
   const int step_raw = *g.step;
+  const int m = g.col_m[col], col_run = g.col_run[col];
   // basis reuse: the second half keeps its node-basis vectors, the first half of the step they
   // were kept for starts from them at its last product (o0 = 1, the theta chain having two)
   const bool keep_theta = THETA && SECOND_HALF && t.yth != nullptr;
@@ -566,7 +650,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   // the x tile (all l, NP points): point fp = tid % NP, the l quads fg, fg + FG, ... of this thread, all
   // requested here, so that the rest of the set-up runs under their latency
   constexpr int FG = A8_THREADS / NP;          // l quads per round
-  constexpr int FR = NP == 32 ? 4 : 3;         // rounds: 32 quads (N_l <= 128) or 56 (N_l <= 220)
+  constexpr int FR = 2;                        // rounds: 32 quads (N_l <= 128, FG = 18) or 56 (N_l <= 220, FG = 36)
   const int fp = threadIdx.x % NP, fg = threadIdx.x / NP;
   double2 xv[FR][4];
   {
@@ -581,8 +665,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
         xv[f][u] = (l < n_l && rv) ? src[(size_t)l * ls] : make_double2(0.0, 0.0);
       }
   }
-  const int m = g.col_m[col];
-  const RunDev run = g.runs[g.col_run[col]];
+  const RunDev run = g.runs[col_run];
   const int step = step_raw < run.n_t ? step_raw : run.n_t - 1;
   const double hdt = 0.5 * g.dt;
   const double* pco = g.coef + ((size_t)CF_P * g.n_m + m) * n_l;
@@ -616,6 +699,10 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
     pbase[2][p] = v2 * hdt;
     pbase[3][p] = v3 * hdt;
     pbase[4][p] = sb * hdt;
+    if (SECOND_HALF) {
+      prr[0][p] = rv ? rr : 0.0;
+      prr[1][p] = rv ? 1.0 / (rr * rr) : 0.0;
+    }
   }
   // what the fill's phase takes per l: the first product's eigenvalue (basis reuse) or the S coefficient
   for (int l = threadIdx.x; l < n_l; l += A8_THREADS)
@@ -625,10 +712,9 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   const int mat0 = ch.ops[o0].mat + (step_raw & (t.n_var - 1)) * t.n_mats;   // this step's variant
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int pa = 0; pa < I8_SLICES; ++pa) {
-      mbar_expect_tx(&full_bar[pa], A8_A_TILE);
-      tma_load_5d(sst + pa * A8_A_TILE, &tmS, 0, 0, pa, m, mat0, &full_bar[pa]);
-    }
+    for (int pa = 0; pa < I8_SLICES; ++pa)
+      a8_load_round<K_ATOMS>(t.geo, t.St + ((size_t)mat0 * g.n_m + m) * t.geo.bytes(), 0, a8_round_end<K_ATOMS>(t.one_round, 0), pa,
+                             sst + pa * A8_A_TILE, &full_bar[pa]);
   }
 
   // operand: phases of the tile in registers (second half: the l-diagonal S phase; basis reuse: the
@@ -694,6 +780,12 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // bring the x tile of the block that follows on this SM to L2, one row (NP radii of one l) per thread
+  if (const unsigned nb = blockIdx.x + A8_BLOCKS_PER_SM * t.sms; nb < gridDim.x && (int)threadIdx.x < n_l) {
+    const int ncol = nb / tilesN, nr0 = (nb - ncol * tilesN) * NP;
+    const double2* row = (from_theta ? t.yth : xin) + ((size_t)threadIdx.x * g.n_cols + ncol) * g.n_r + nr0;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row), "r"(min(NP, g.n_r - nr0) * 16) : "memory");
+  }
   const uint32_t tmem = tmem_slot;
   volatile int* abort_p = &abort_flag;
 
@@ -703,77 +795,91 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
       bool ok = true;
       for (int o = o0; o < n_ops && ok; ++o) {
         const int mat = ch.ops[o].mat + (step_raw & (t.n_var - 1)) * t.n_mats;   // this step's variant
-        // stage pa takes slice plane pa; the ring turns once per (tile, atom)
-        for (int mt = 0; mt < t.m_tiles && ok; ++mt)
-          for (int ka = 0; ka < t.k_atoms && ok; ++ka) {
-            const int round = it / I8_SLICES;
+        const int8_t* src = t.St + ((size_t)mat * g.n_m + m) * t.geo.bytes();
+        // stage pa takes slice plane pa; the ring turns once per round
+        for (int i0 = 0, i1; i0 < K_ATOMS * K_ATOMS && ok; i0 = i1) {
+          i1 = a8_round_end<K_ATOMS>(t.one_round, i0);
+          const int round = it / I8_SLICES;
 #pragma unroll
-            for (int pa = 0; pa < I8_SLICES; ++pa, ++it) {
-              if (round == 0) continue;          // issued before the fill
-              if (!mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) {
-                ok = false;
-                break;
-              }
-              mbar_expect_tx(&full_bar[pa], A8_A_TILE);
-              tma_load_5d(sst + pa * A8_A_TILE, &tmS, ka * A8_KATOM, mt * 128, pa, m, mat, &full_bar[pa]);
+          for (int pa = 0; pa < I8_SLICES; ++pa, ++it) {
+            if (round == 0) continue;          // issued before the fill
+            if (!mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) {
+              ok = false;
+              break;
             }
+            a8_load_round<K_ATOMS>(t.geo, src, i0, i1, pa, sst + pa * A8_A_TILE, &full_bar[pa]);
           }
+        }
       }
       if (!ok)
         for (int q = (it > t.stages ? it - t.stages : 0); q < it; ++q) mbar_drain(&full_bar[q % t.stages], (q / t.stages) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // one MMA per (S^T slice pa, 32-wide k step): N = (4 - pa) NB rows of the stacked x slice planes
-      // 0 .. 3 - pa, written at TMEM column pa NB, so that its column group pb lands on the
-      // accumulator of weight 2^-8(pa + pb)
-      const uint32_t idesc[I8_SLICES] = {idesc_i8(128, 4 * NB), idesc_i8(128, 3 * NB), idesc_i8(128, 2 * NB),
-                                          idesc_i8(128, NB)};
-      // The loads come four per (M tile, k atom), one per slice plane pa, into a ring of four
-      // stages, so stage pa always holds plane pa and the ring turns once per (tile, atom).  The
-      // descriptors of stage pa and k step kk are those of stage 0 (or of the B operand's atom) plus
-      // the byte offset / 16 in the start-address field, which keeps this thread's loop short: it
-      // shares its SM sub-partition with busy epilogue warps, and its issue rate paces the products.
-      const uint64_t adesc = sdesc_kmajor(smem_u32(sst), 128, 2);
-      const uint64_t bdesc = sdesc_kmajor(smem_u32(xb), 128, 2);
-      int round = 0;
-      for (int o = o0; o < n_ops; ++o) {
-        if (o > o0 && !mbar_wait(&xb_bar, (o - o0 - 1) & 1, abort_p)) break;
-        tc_fence_after();
-        bool ok = true;
-        for (int mt = 0; mt < t.m_tiles && ok; ++mt) {
-          const uint32_t d0 = tmem + acc_cols * mt;
-          for (int ka = 0; ka < t.k_atoms && ok; ++ka, ++round) {
+    // one MMA per (S^T slice pa, 32-wide k step): N = (4 - pa) NB rows of the stacked x slice planes
+    // 0 .. 3 - pa, written at TMEM column pa NB, so that its column group pb lands on the
+    // accumulator of weight 2^-8(pa + pb)
+    constexpr uint32_t idesc[I8_SLICES] = {idesc_i8(128, 4 * NB), idesc_i8(128, 3 * NB), idesc_i8(128, 2 * NB),
+                                           idesc_i8(128, NB)};
+    // The loads come four per round, one per slice plane pa, into a ring of four stages, so stage pa always
+    // holds plane pa and the ring turns once per round.  Descriptors are those of stage 0 (or of the B
+    // operand's atom) plus the byte offset / 16 in the start-address field.  This warp shares its SM
+    // sub-partition with busy epilogue warps, and its issue rate paces the products.  (Rows past the M
+    // tile's images, and the accumulator lanes they reach, hold what the buffer held: they only ever meet
+    // the zero columns past N_l of the next product.)
+    const uint32_t elected = elect_one();
+    const uint64_t adesc0 = a8_sdesc(smem_u32(sst), t.geo.pitch(0)), adesc1 = a8_sdesc(smem_u32(sst), t.geo.pitch(1));
+    const uint64_t bdesc = sdesc_kmajor(smem_u32(xb), 128, 2);
+    uint32_t plane[K_ATOMS * K_ATOMS];
+#pragma unroll
+    for (int i = 0; i < K_ATOMS * K_ATOMS; ++i) plane[i] = (uint32_t)(t.geo.rows(i / K_ATOMS) * t.geo.pitch(i % K_ATOMS)) >> 4;
+    int round = 0;
+    for (int o = o0; o < n_ops; ++o) {
+      if (o > o0 && !__all_sync(0xffffffffu, mbar_wait(&xb_bar, (o - o0 - 1) & 1, abort_p))) break;
+      tc_fence_after();
+      // tiles I0 .. I1 - 1 as one round, unrolled
+      auto issue_round = [&](auto I0, auto I1) -> bool {
+#pragma unroll
+        for (int pa = 0; pa < I8_SLICES; ++pa) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[pa], round & 1, abort_p))) return false;
+          tc_fence_after();
+          uint32_t off = (pa * A8_A_TILE) >> 4;
+#pragma unroll
+          for (int i = decltype(I0)::value; i < decltype(I1)::value; ++i) {
+            const int mt = i / K_ATOMS, ka = i % K_ATOMS;
+            const uint32_t d0 = tmem + acc_cols * mt + pa * NB;
+            const uint64_t ak = (ka ? adesc1 : adesc0) + off;
             const uint64_t bk = bdesc + (uint64_t)((ka * I8_SLICES * B_TILE) >> 4);
-            const int nk = min(A8_KATOM / 32, t.k_steps - ka * (A8_KATOM / 32));
+            const int nk = K_ATOMS == 2 && ka == 0 ? A8_KATOM / 32 : t.k_steps - ka * (A8_KATOM / 32);
 #pragma unroll
-            for (int pa = 0; pa < I8_SLICES; ++pa) {
-              if (!mbar_wait(&full_bar[pa], round & 1, abort_p)) {
-                ok = false;
-                break;
-              }
-              tc_fence_after();
-              const uint64_t ak = adesc + (uint64_t)((pa * A8_A_TILE) >> 4);
-#pragma unroll
-              for (int kk = 0; kk < A8_KATOM / 32; ++kk)
-                if (kk < nk) tc_mma_i8(d0 + pa * NB, ak + 2 * kk, bk + 2 * kk, idesc[pa], (ka | kk | pa) ? 1u : 0u);
-              tc_commit(&empty_bar[pa]);
-            }
+            for (int kk = 0; kk < A8_KATOM / 32; ++kk)
+              if (kk < nk) tc_mma_i8_if(elected, d0, ak + 2 * kk, bk + 2 * kk, idesc[pa], (ka | kk | pa) ? 1u : 0u);
+            off += plane[i];
           }
+          tc_commit_if(elected, &empty_bar[pa]);
         }
-        // one commit for all M tiles: every tile's products read the whole operand, which the
-        // epilogue overwrites with the next product's
-        tc_commit(&acc_bar);
-        if (!ok) break;
+        ++round;
+        return true;
+      };
+      bool ok = issue_round(I8c<0>(), I8c<1>());
+      if constexpr (K_ATOMS == 2) {
+        if (t.one_round) {
+          ok = ok && issue_round(I8c<1>(), I8c<4>());
+        } else {
+          ok = ok && issue_round(I8c<1>(), I8c<2>()) && issue_round(I8c<2>(), I8c<3>()) && issue_round(I8c<3>(), I8c<4>());
+        }
       }
+      // one commit for all M tiles: every tile's products read the whole operand, which the
+      // epilogue overwrites with the next product's
+      tc_commit_if(elected, &acc_bar);
+      if (!ok) break;
     }
   } else {
     const int ew = warp - A8_EPI_WARP0;
     const int q = warp & 3;                     // TMEM lane quarter of this warp
-    const int grp = ew >> 2;
-    const int mt = (t.m_tiles == 2) ? grp : 0;
+    const int grp = ew >> 2;                    // four warps per lane quarter share its (M tile, points)
+    const int mt = (t.m_tiles == 2) ? grp >> 1 : 0;
     const int j = 128 * mt + 32 * q + lane;     // eigen-channel (M row) of this thread
-    const int p_begin = (t.m_tiles == 2) ? 0 : A8_PTS * grp;
+    const int p_begin = A8_PTS * ((t.m_tiles == 2) ? grp & 1 : grp);
     // staging of the last product, [N_l][NP + 1] (the odd row length keeps both this write, lanes
     // along l, and the reads below, lanes along the points, free of bank conflicts)
     double2* stage_out = reinterpret_cast<double2*>(smem);
@@ -800,20 +906,22 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
       const double* Dv = g.dph + ((size_t)op.coupling * g.n_m + m) * g.ldS;
       const double dj = (op.phase != PH_NONE && j >= m && j < n_l) ? Dv[j] : 0.0;
       const int pb = op.phase == PH_P ? 1 : op.phase == PH_D ? 2 : 3;
-      // the theta form: angle = pbase1 x_j + pbase2 P_2(x_j) + pbase3 P_3(x_j) + pbase4 (all x dt/2)
-      const bool th = THETA && op.phase == PH_THETA && j >= m && j < n_l;
-      const double p2j = th ? legendre_p2(dj) : 0.0, p3j = th ? legendre_p3(dj) : 0.0;
+      // the theta form: angle = pbase1 x_j + pbase2 P_2(x_j) + pbase3 P_3(x_j) + pbase4 (all x dt/2), zero for
+      // channels below m and past N_l
+      const bool ph_theta = THETA && op.phase == PH_THETA, act = j >= m && j < n_l;
+      const double p2j = legendre_p2(dj), p3j = legendre_p3(dj);
       const bool post_s = last && !SECOND_HALF && ch.post_s && j < n_l;
       const double pj = post_s ? pco[j] : 0.0;
       const double sj = pow2i(-t.sexp[((size_t)op.mat * g.n_m + m) * t.rows + j]);   // S^T row scale
-      // software pipeline over chunks of 4 points: the next chunk's accumulators are requested
+      // software pipeline over chunks of 2 points: the next chunk's accumulators are requested
       // from tensor memory before this chunk is rotated and sliced
-      uint32_t re[4][4], im[4][4];
+      constexpr int CH = 2;
+      uint32_t re[4][CH], im[4][CH];
       auto tload = [&](int p0) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-          tmem_ld4(d0 + s * NB + p0, re[s]);
-          tmem_ld4(d0 + s * NB + NP + p0, im[s]);
+          tmem_ld2(d0 + s * NB + p0, re[s]);
+          tmem_ld2(d0 + s * NB + NP + p0, im[s]);
         }
       };
       auto tready = [&]() {
@@ -827,24 +935,24 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
       tload(p_begin);
       tready();
 #pragma unroll 1
-      for (int c4 = 0; c4 < A8_PTS / 4; ++c4) {
-        const int p0 = p_begin + 4 * c4;
+      for (int c = 0; c < A8_PTS / CH; ++c) {
+        const int p0 = p_begin + CH * c;
         // the accumulators hold y 2^(e_j + e_p) 2^24; rotations commute with the scale, and the
         // next product's slices want y 2^e_p 2^24: one exact power of two in between
-        double2 v[4];
+        double2 v[CH];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < CH; ++u)
           v[u] = make_double2((double)combine_int(re, u) * sj, (double)combine_int(im, u) * sj);
-        if (c4 + 1 < A8_PTS / 4) tload(p0 + 4);
+        if (c + 1 < A8_PTS / CH) tload(p0 + CH);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < CH; ++u) {
           const int p = p0 + u;
           if constexpr (THETA) {
-            if (th) {
+            if (ph_theta) {
               double ang = pbase[1][p] * dj + pbase[2][p] * p2j + pbase[3][p] * p3j + pbase[4][p];
               // n_har > 4: the multipoles L >= 1 at this node come from the exact-quadrature table
-              if (g.theta_tab && r0 + p < g.n_r) ang += run.htab[((size_t)m * n_l + j) * g.n_r + r0 + p] * hdt;
-              v[u] = rotd(v[u], ang);
+              if (g.theta_tab && act && r0 + p < g.n_r) ang += run.htab[((size_t)m * n_l + j) * g.n_r + r0 + p] * hdt;
+              v[u] = rotd(v[u], act ? ang : 0.0);
             }
           } else {
             if (dj != 0.0) v[u] = rotd(v[u], pbase[pb][p] * dj);
@@ -865,7 +973,7 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
             stage_out[j * (NP + 1) + p] = make_double2(v[u].x * sc, v[u].y * sc);
           }
         }
-        if (c4 + 1 < A8_PTS / 4) tready();
+        if (c + 1 < A8_PTS / CH) tready();
       }
       tc_fence_before();
       if (!last) {
@@ -885,6 +993,14 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
     // per step, after this kernel)
     if (keep_theta && blockIdx.x == 0 && threadIdx.x == 0) *g.yth_step = step_raw + 2;
     const double2* xs = reinterpret_cast<const double2*>(smem);
+    // the observables' thread layout and its coefficients, requested before the store
+    const int lw = (n_l + 31) & ~31, parts = A8_THREADS / lw;     // N_l <= 220
+    const int part = threadIdx.x / lw, lo = threadIdx.x - part * lw;
+    double c_u = 0.0, c_d = 0.0;
+    if (SECOND_HALF && part < parts && lo < n_l) {
+      if (lo + 1 < n_l) c_u = g.coef[((size_t)CF_CU * g.n_m + m) * n_l + lo];
+      if (lo > m) c_d = g.coef[((size_t)CF_CD * g.n_m + m) * n_l + lo];
+    }
     for (int idx = threadIdx.x; idx < n_l * NP; idx += A8_THREADS) {
       const int l = idx / NP, p = idx - l * NP, r = r0 + p;
       if (r < g.n_r) xout[((size_t)l * g.n_cols + col) * g.n_r + r] = xs[l * (NP + 1) + p];
@@ -892,33 +1008,23 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
     if (SECOND_HALF) {
       // FP64 dipole and acceleration partial sums and density multipoles of the new orbitals, from
       // the staged tile, with the coefficient rows of this m staged after it.
-      constexpr int NW = A8_THREADS / 32;
       constexpr int LG = 32 / NP;        // lane groups per warp: lane = (point, l-loop group)
-      constexpr int NG = NW * LG;        // groups that stride the density's l loops
+      constexpr int NG = A8_DEN_WARPS * LG;   // groups that stride the density's l loops
       double* rows = reinterpret_cast<double*>(smem + (((size_t)n_l * (NP + 1) * 16 + 255) & ~(size_t)255));
-      double* red = rows + ((COEF_N * n_l + 1) & ~1);       // [NG][N_DEN][NP], 16-byte aligned
-      double* prr = red + NG * N_DEN * NP;                  // [2][NP]: r and r^-2 of each point (0 past N_r)
-      for (int i = threadIdx.x; i < COEF_N * n_l; i += A8_THREADS) {
-        const int c = i / n_l, l = i - c * n_l;
-        rows[i] = g.coef[((size_t)c * g.n_m + m) * n_l + l];
-      }
-      if (threadIdx.x < NP) {
-        const int r = r0 + threadIdx.x;
-        const double rr = r < g.n_r ? g.r[r] : 0.0;
-        prr[threadIdx.x] = rr;
-        prr[NP + threadIdx.x] = r < g.n_r ? 1.0 / (rr * rr) : 0.0;
-      }
-      __syncthreads();
+      double* red = rows + ((COEF_N * n_l + 1) & ~1);       // [NG][N_DEN][NP] (and the observables' shares), 16-byte aligned
+      const int n_den = g.n_den > 0 ? g.n_den : 1;   // L = 0 is always needed for the norm
+      if (n_den > 1)
+        for (int i = threadIdx.x; i < COEF_N * n_l; i += A8_THREADS) {
+          const int c = i / n_l, l = i - c * n_l;
+          rows[i] = g.coef[((size_t)c * g.n_m + m) * n_l + l];
+        }
       // dipole and acceleration: `parts` threads per l, each over its share of the CTA's NP radii, then
       // the shares added in order (one partial per (l, NP radii))
       double4* ored = reinterpret_cast<double4*>(red);      // [parts][lw], parts lw <= A8_THREADS
-      const int lw = (n_l + 31) & ~31, parts = A8_THREADS >= lw ? A8_THREADS / lw : 1;
-      const int part = threadIdx.x / lw, lo = threadIdx.x - part * lw;
       double4 osum = make_double4(0.0, 0.0, 0.0, 0.0);
       if (part < parts && lo < n_l && lo >= m) {
         // the first row has no lower, the last no upper neighbour
         const bool has_u = lo + 1 < n_l, has_d = lo > m;
-        const double c_u = has_u ? rows[CF_CU * n_l + lo] : 0.0, c_d = has_d ? rows[CF_CD * n_l + lo] : 0.0;
         const double2* xl_p = xs + lo * (NP + 1);
         for (int p = part * NP / parts; p < (part + 1) * NP / parts; ++p) {
           const double2 xl = xl_p[p];
@@ -926,10 +1032,10 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
           const double2 xd = has_d ? xl_p[p - NP - 1] : make_double2(0.0, 0.0);
           const double zx = c_u * xu.x + c_d * xd.x, zy = c_u * xu.y + c_d * xd.y;
           const double px = xl.x * zx + xl.y * zy, py = xl.x * zy - xl.y * zx;     // conj(x_l) . z
-          osum.x = fma(prr[p], px, osum.x);
-          osum.y = fma(prr[p], py, osum.y);
-          osum.z = fma(prr[NP + p], px, osum.z);
-          osum.w = fma(prr[NP + p], py, osum.w);
+          osum.x = fma(prr[0][p], px, osum.x);
+          osum.y = fma(prr[0][p], py, osum.y);
+          osum.z = fma(prr[1][p], px, osum.z);
+          osum.w = fma(prr[1][p], py, osum.w);
         }
       }
       if (parts > 1) {
@@ -945,12 +1051,13 @@ k_angular_i8(const __grid_constant__ CUtensorMap tmS, GroupArgs g, Ang8Args t, c
       if (parts > 1) __syncthreads();         // the shares' memory is the density's next
       // density multipoles: every lane works (point lane % NP), the literal l loops strided over the
       // NG lane groups, then the groups summed in order
-      const int n_den = g.n_den > 0 ? g.n_den : 1;   // L = 0 is always needed for the norm
       const int pt = lane % NP, gi = warp * LG + lane / NP;
       double d[N_DEN] = {0.0, 0.0, 0.0, 0.0};
-      density_partials<double2, NP + 1>(n_den, m, n_l, xs, pt, rows, gi, NG, d);
+      if (warp < A8_DEN_WARPS) {
+        density_partials<double2, NP + 1>(n_den, m, n_l, xs, pt, rows, gi, NG, d);
 #pragma unroll
-      for (int L = 0; L < N_DEN; ++L) red[(gi * N_DEN + L) * NP + pt] = d[L];
+        for (int L = 0; L < N_DEN; ++L) red[(gi * N_DEN + L) * NP + pt] = d[L];
+      }
       __syncthreads();
       if (threadIdx.x < n_den * NP) {
         const int L = threadIdx.x / NP, pp = threadIdx.x - L * NP, rl = r0 + pp;
@@ -1080,11 +1187,6 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   I8_CK(cudaMemset(q.X, 0, nx));
   I8_CK(cudaMalloc(&q.xexp, (size_t)n_l * q.cols_pad * sizeof(int)));
   I8_CK(cudaMemset(q.xexp, 0, (size_t)n_l * q.cols_pad * sizeof(int)));
-  EncodeTiledFn enc = tensor_map_encoder();
-  if (!enc) {
-    err = "cuTensorMapEncodeTiled unavailable";
-    return GGB_ERR_CUDA;
-  }
   // angular chain: S^T slices
   q.a_m_tiles = (n_l + 127) / 128;
   q.a_k_atoms = (n_l + A8_KATOM - 1) / A8_KATOM;
@@ -1100,7 +1202,7 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   // FP64 staging of the last product, [N_l][NP + 1], over the operand planes and stage buffers
   // the second half's tail: output tile, coefficient rows and the multipoles' warp partials
   const size_t tail = (((size_t)n_l * (q.np + 1) * 16 + 255) & ~(size_t)255) + ((size_t)COEF_N * n_l + 1) * 8 +
-                      (size_t)(A8_THREADS / 32) * N_DEN * 32 * 8 + 2 * (size_t)q.np * 8;
+                      (size_t)A8_THREADS * 4 * 8 + 2 * (size_t)q.np * 8;
   if (tail > q.a_smem - 1024 || q.a_smem > 110 * 1024) {
     err = "int8 angular chain: shared memory";
     return GGB_ERR_ARG;
@@ -1110,36 +1212,22 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
     err = "int8 angular chain: observables partials do not match its tile";
     return GGB_ERR_STATE;
   }
-  const int rows = 128 * q.a_m_tiles, lk = A8_KATOM * q.a_k_atoms;
+  const int rows = 128 * q.a_m_tiles;
   q.a_rows = rows;
   const int n_mm = n_mats * a.n_m;
-  const size_t nst = (size_t)n_mm * I8_SLICES * rows * lk;    // one variant
+  const StGeom geo = StGeom::of(n_l);
+  const size_t nst = (size_t)n_mm * geo.bytes();    // one variant
   q.n_mats = n_mats;
   I8_CK(cudaMalloc(&q.St, nst * I8_S_VARIANTS));
   I8_CK(cudaMalloc(&q.sexp, (size_t)n_mm * rows * sizeof(int)));
   for (int v = 0; v < I8_S_VARIANTS; ++v)
-    k_build_st_i8<<<n_mm * rows, 256>>>(a.mats, q.St + nst * v, q.sexp, n_mm, a.n_m, n_l, a.ldS, rows, lk, v,
+    k_build_st_i8<<<n_mm * rows, 256>>>(a.mats, q.St + nst * v, q.sexp, n_mm, a.n_m, n_l, a.ldS, rows, geo, v,
                                         I8_S_VARIANTS);
   I8_CK(cudaGetLastError());
   // basis reuse of the theta form (one phase op and one closing product per half); the angular
   // products on the FP64 kernel keep the full chain
   if (q.theta_reuse && a.theta && !mg.angular_fp64 && a.chain[0].n_ops == 2 && a.chain[1].n_ops == 2) {
     I8_CK(cudaMalloc(&q.yth, (size_t)n_l * a.n_cols * n_r * sizeof(double2)));
-  }
-  {
-    // the variants follow one another along the matrix index: matrix mat of variant v is mat + v n_mats
-    cuuint64_t dims[5] = {(cuuint64_t)lk, (cuuint64_t)rows, I8_SLICES, (cuuint64_t)a.n_m,
-                          (cuuint64_t)n_mats * I8_S_VARIANTS};
-    cuuint64_t strides[4] = {(cuuint64_t)lk, (cuuint64_t)rows * lk, (cuuint64_t)I8_SLICES * rows * lk,
-                             (cuuint64_t)a.n_m * I8_SLICES * rows * lk};
-    cuuint32_t box[5] = {A8_KATOM, 128, 1, 1, 1};
-    cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    if (enc(&q.tmS, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, q.St, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
-        CUDA_SUCCESS) {
-      err = "tensor map (int8 S^T) failed";
-      return GGB_ERR_CUDA;
-    }
   }
   int dev = 0, optin = 0, sms = 0;
   I8_CK(cudaGetDevice(&dev));
@@ -1182,13 +1270,17 @@ void int8_angular(MixedGroup& mg, const GroupArgs& a, int half, const double2* x
   t.m_tiles = q.a_m_tiles;
   t.k_steps = (a.n_l + 31) / 32;
   t.stages = q.a_stages;
+  t.St = q.St;
+  t.geo = StGeom::of(a.n_l);
+  t.one_round = q.a_m_tiles == 2 && st_one_round(t.geo);
   t.sexp = q.sexp;
   t.rows = q.a_rows;
+  t.sms = q.ctas;
   t.n_mats = q.n_mats;
   t.n_var = I8_S_VARIANTS;
   t.yth = q.yth;
   const dim3 grid(a.n_cols * ((a.n_r + q.np - 1) / q.np));
-#define GGB_A8(NP, SH, TH) k_angular_i8<NP, SH, TH><<<grid, A8_THREADS, q.a_smem, s>>>(q.tmS, a, t, xin, xout)
+#define GGB_A8(NP, SH, TH) k_angular_i8<NP, SH, TH><<<grid, A8_THREADS, q.a_smem, s>>>(a, t, xin, xout)
   if (q.np == 32) {
     if (half == 0) { if (a.theta) GGB_A8(32, false, true); else GGB_A8(32, false, false); }
     else { if (a.theta) GGB_A8(32, true, true); else GGB_A8(32, true, false); }

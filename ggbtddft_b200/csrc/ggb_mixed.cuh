@@ -25,10 +25,9 @@ struct I8Group {
   int* wexp = nullptr;       // [N_l][rows_pad]
   int8_t* X = nullptr;       // [N_l][column tile][k block][12][columns of the tile][32]: Xr, Xi, -Xi slices 1-4 of x 2^xexp(l, col)
   int* xexp = nullptr;       // [N_l][cols_pad]
-  int8_t* St = nullptr;      // [variant][mat][m][4][rows][lk]: S^T slices, rows scaled by 2^sexp
+  int8_t* St = nullptr;      // [variant][mat][m]: S^T slice planes as stage images, rows scaled by 2^sexp
   int n_mats = 0;            // chain matrices per variant
   int* sexp = nullptr;       // [mat][m][rows]
-  CUtensorMap tmS;
   int bn = 16, cols_pad = 0, stages = 2, ctas = 0;
   int tune_bn = 0, tune_stages = 0;   // ggb_set_tuning (0: built-in choice)
   size_t smem = 0;

@@ -100,6 +100,22 @@ __device__ __forceinline__ void tc_commit(uint64_t* b) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
                : "memory");
 }
+// One lane of a converged warp (the same one every time).  A warp that issues MMAs runs as a whole, with
+// its index from a shuffle and its waits voted on, so that descriptors and loop counters stay in uniform
+// registers; only the instructions themselves are predicated on the elected lane.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+  return e;
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t elected, uint64_t* b) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(b)),
+      "r"(elected)
+      : "memory");
+}
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
