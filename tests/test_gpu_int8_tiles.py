@@ -69,3 +69,17 @@ def test_observables_partials_match_the_orbitals(n_l, n_orb_runs):
             assert np.abs(tot[key][:, 1] - want.sum(0)).max() <= 1e-13 * scale * n_l
         assert np.allclose(got["norm"][:, 1], (np.abs(x) ** 2).sum(axis=(0, 2)), rtol=1e-13, atol=0)
     tp.close()
+
+
+@pytest.mark.parametrize("n_r", [511, 512, 513, 1023, 1024, 1025])
+def test_slices_of_rows_at_the_register_limits(n_r):
+    """Rows of one and two quads per thread and longer ones (read twice): the radial product of a short
+    l range against the FP64 product."""
+    base = P.reference_like(n_r, 2, 2, "H", r_mask=10.0).with_field(np.zeros(2))
+    run = _random(base, n_r)
+    tp = TimePropagation([run], precision="split_int8")
+    tp.step(1)
+    got = tp.orbitals(0)
+    tp.close()
+    want = np.einsum("lba,lkb->lka", run.W, run.x0)
+    assert np.linalg.norm(got - want) < 1e-6 * np.linalg.norm(want)
