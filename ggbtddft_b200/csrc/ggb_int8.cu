@@ -958,7 +958,7 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
             if (dj != 0.0) v[u] = rotd(v[u], pbase[pb][p] * dj);
           }
           if (post_s) v[u] = rotd(v[u], pbase[4][p] + pj * pbase[2][p]);
-          if (ykeep && r0 + p < g.n_r) {
+          if (NP != 32 && ykeep && r0 + p < g.n_r) {
             const double sc = pinv[p] * 0x1p-24;
             ykeep[p] = make_double2(v[u].x * sc, v[u].y * sc);
           }
@@ -971,6 +971,20 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
           } else if (j < n_l) {
             const double sc = pinv[p] * 0x1p-24;
             stage_out[j * (NP + 1) + p] = make_double2(v[u].x * sc, v[u].y * sc);
+          }
+        }
+        if (NP == 32 && ykeep) {
+          // two points are 32 bytes: one store where the row starts on them (ten runs, N_l 97: second half
+          // 172 -> 164 us; with two M tiles the same form costs 4 %, in registers, and the points are
+          // stored one by one above)
+          const double s0 = pinv[p0] * 0x1p-24, s1 = pinv[p0 + 1] * 0x1p-24;
+          if (!(g.n_r & 1) && r0 + p0 + 1 < g.n_r) {
+            asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(ykeep + p0), "d"(v[0].x * s0), "d"(v[0].y * s0),
+                         "d"(v[1].x * s1), "d"(v[1].y * s1)
+                         : "memory");
+          } else {
+            if (r0 + p0 < g.n_r) ykeep[p0] = make_double2(v[0].x * s0, v[0].y * s0);
+            if (r0 + p0 + 1 < g.n_r) ykeep[p0 + 1] = make_double2(v[1].x * s1, v[1].y * s1);
           }
         }
         if (c + 1 < A8_PTS / CH) tready();
