@@ -26,6 +26,7 @@ constexpr int COUNTERS = 4;       // ints before the row counters of a group's c
 
 struct GroupHost {
   ggb_group_desc d{};
+  int run0 = 0;                  // first entry of the device run table, which lists the groups' runs in order
   int n_cols = 0, n_tiles = 0, obs_seg = TR, ldS = 0;
   std::vector<int> runs;         // ctx run indices
   bool grid_set = false, w_set = false;
@@ -39,7 +40,7 @@ struct GroupHost {
   double *frag_d = nullptr;
   double *mats_d = nullptr, *dph_d = nullptr, *coef_d = nullptr;
   double2 *x_d = nullptr, *y_d = nullptr;     // FP64 orbitals
-  int *col_run_d = nullptr, *col_m_d = nullptr, *col_occ_d = nullptr, *runs_d = nullptr;
+  int *col_run_d = nullptr, *col_m_d = nullptr, *col_occ_d = nullptr;
   double* dens_d = nullptr;
   double4* obs_d = nullptr;
   // step counter, k_finalize's block counter, the basis reuse's step, then k_finalize's row counters: one
@@ -59,7 +60,7 @@ struct GroupHost {
 
 struct RunHost {
   ggb_run_desc d{};
-  int col0 = 0;
+  int col0 = 0, in_group = 0;    // first column and position in the group
   bool orb_set = false, field_set = false;
   double *E_d = nullptr, *v_d = nullptr, *v0_d = nullptr, *vexc_d = nullptr, *vexc0_d = nullptr;
   double *rho_frozen_d = nullptr, *norm_d = nullptr, *norm0_d = nullptr;
@@ -457,8 +458,8 @@ static int prepare(ggb_ctx* ctx) {
     a.n_g_fac = (double)(n_g * (n_g + 1)) / 2.0;
     a.r = g.r_d; a.drdx = g.drdx_d; a.P = g.P_d;
     a.mats = g.mats_d; a.frag = g.frag_d; a.dph = g.dph_d; a.coef = g.coef_d;
-    a.col_run = g.col_run_d; a.col_m = g.col_m_d; a.col_occ = g.col_occ_d; a.runs_of_group = g.runs_d;
-    a.runs = ctx->runs_dev;
+    a.col_run = g.col_run_d; a.col_m = g.col_m_d; a.col_occ = g.col_occ_d;
+    a.runs = ctx->runs_dev + g.run0;
     a.dens = g.dens_d; a.obs = g.obs_d; a.step = g.step_d; a.status = ctx->status_d;
     a.done = (unsigned*)g.step_d + 1;
     a.yth_step = g.step_d + 2;
@@ -483,7 +484,8 @@ static int prepare(ggb_ctx* ctx) {
     RunHost& r = ctx->runs[i];
     if (!r.orb_set) return fail(ctx, GGB_ERR_STATE, "run %zu: orbitals not set", i);
     if (!r.field_set) return fail(ctx, GGB_ERR_STATE, "run %zu: field not set", i);
-    rd[i] = RunDev{r.E_d, r.v_d, r.v0_d, r.vexc_d, r.vexc0_d, r.rho_frozen_d, r.dip_d, r.acc_d,
+    const GroupHost& g = ctx->groups[r.d.group];
+    rd[g.run0 + r.in_group] = RunDev{r.E_d, r.v_d, r.v0_d, r.vexc_d, r.vexc0_d, r.rho_frozen_d, r.dip_d, r.acc_d,
                    r.dip_tot_d, r.acc_tot_d, r.norm_d, r.norm0_d, r.htab_d, r.col0, r.d.n_orb, ctx->dims.n_t,
                    r.d.flags};
   }
@@ -617,10 +619,11 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
       g.theta = theta;
     }
     r.col0 = g.n_cols;
+    r.in_group = (int)g.runs.size();
     g.n_cols += r.d.n_orb;
     g.runs.push_back(i);
   }
-  int rc;
+  int rc, run0 = 0;
   for (GroupHost& g : ctx->groups) {
     if (g.runs.empty()) return bad(GGB_ERR_ARG, "empty group");
     const size_t nr = g.d.n_r, nl = g.d.n_l, nc = g.n_cols;
@@ -628,7 +631,7 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
         (rc = dalloc(ctx, &g.dens_d, nc * N_DEN * nr)) || (dims->precision != GGB_FP64 && (rc = dalloc(ctx, &g.obs_d, 2 * nc * nl * g.n_tiles))) ||
         (rc = dalloc(ctx, &g.step_d, COUNTERS + nc)) || (rc = dalloc(ctx, &g.fin_scr_d, nc * (nl + 1) * 10)) ||
         (rc = dalloc(ctx, &g.col_run_d, nc)) || (rc = dalloc(ctx, &g.col_m_d, nc)) ||
-        (rc = dalloc(ctx, &g.col_occ_d, nc)) || (rc = dalloc(ctx, &g.runs_d, g.runs.size())))
+        (rc = dalloc(ctx, &g.col_occ_d, nc)))
       return bad(rc, "alloc");
     if (dims->precision == GGB_FP64 || dims->precision == GGB_SPLIT_INT8) {
       if ((rc = dalloc(ctx, &g.W_d, nl * nr * nr)) || (rc = dalloc(ctx, &g.x_d, nl * nc * nr)) ||
@@ -639,7 +642,8 @@ int ggb_create(const ggb_dims* dims, const ggb_group_desc* groups, const ggb_run
       if ((rc = dalloc(ctx, &g.W_d, nl * nr * nr)) || (rc = dalloc(ctx, &g.x_d, nl * nc * nr)))
         return bad(rc, "alloc");
     }
-    cudaMemcpy(g.runs_d, g.runs.data(), g.runs.size() * sizeof(int), cudaMemcpyHostToDevice);
+    g.run0 = run0;
+    run0 += (int)g.runs.size();
   }
   for (RunHost& r : ctx->runs) {
     const GroupHost& g = ctx->groups[r.d.group];
@@ -737,7 +741,7 @@ int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const
     if (nm[k] < 0 || nm[k] >= g.d.n_m || nl_[k] < nm[k] || nl_[k] >= nl)
       return fail(ctx, GGB_ERR_ARG, "orbital %d: l=%d m=%d outside 0<=m<N_m, m<=l<N_l", k, nl_[k], nm[k]);
   if (!r.orb_set || nm != r.m || nocc != r.occ) {
-    std::vector<int> cr(no, run);
+    std::vector<int> cr(no, r.in_group);
     CK(cudaMemcpy(g.col_m_d + r.col0, nm.data(), no * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.col_occ_d + r.col0, nocc.data(), no * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.col_run_d + r.col0, cr.data(), no * sizeof(int), cudaMemcpyHostToDevice));

@@ -97,11 +97,10 @@ struct GroupArgs {
   const double* frag;       // the chain matrices in fragment order of the FP64 angular kernel
   const double* dph;
   const double* coef;
-  const int* col_run;   // [n_cols] run index within ctx
+  const int* col_run;   // [n_cols] run index within the group
   const int* col_m;
   const int* col_occ;
-  const int* runs_of_group;  // [n_runs] ctx run indices
-  RunDev* runs;             // ctx-wide device array
+  RunDev* runs;             // [n_runs] the group's part of the context's device array
   double* dens;
   double4* obs;
   int* step;                // the group's step counter

@@ -872,29 +872,26 @@ template <bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
   extern __shared__ double fsm[];  // [2][N_r]
   __shared__ dd wsum[FIN_THREADS / 32][2];
-  __shared__ int s_step;
   const int n_xc = fin_xc_blocks(g, mode);
   const int nb = g.n_den + n_xc + g.fin_ob;
   const int ri = blockIdx.x / nb;
   const int role = blockIdx.x - ri * nb;  // Hartree L = role, then exchange, then observables blocks
-  const RunDev run = g.runs[g.runs_of_group[ri]];
   const int n_r = g.n_r, n_l = g.n_l, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const bool obs_block = role >= g.n_den + n_xc;
   const int ob = role - g.n_den - n_xc;
-  // the step counter advances once every block has read it
-  if (tid == 0) {
-    s_step = *g.step;
-    if (mode == 1) {
-      __threadfence();
-      if (atomicAdd(g.done, 1u) == gridDim.x - 1) {
-        *g.done = 0u;
-        *g.step = s_step + 1;
-      }
+  const int step = *g.step;
+  const RunDev run = g.runs[ri];
+  // the step counter advances once every thread of every block has read it
+  asm volatile("" ::"r"(step) : "memory");
+  __syncthreads();
+  if (mode == 1 && tid == 0) {
+    __threadfence();
+    if (atomicAdd(g.done, 1u) == gridDim.x - 1) {
+      *g.done = 0u;
+      *g.step = step + 1;
     }
   }
-  __syncthreads();
-  const int step = s_step;
 
   if (obs_block && mode != 0 && step >= run.n_t) {
     if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);

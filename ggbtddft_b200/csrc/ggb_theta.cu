@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(1024) k_theta_density(GroupArgs g, ThetaArgs t
   double* buf = fs + 2 * (size_t)nq * TH_R;                     // two table chunks
   const int tiles = (n_r + TH_R - 1) / TH_R;
   const int ri = blockIdx.x / tiles, r0 = (blockIdx.x - ri * tiles) * TH_R;
-  const RunDev run = g.runs[g.runs_of_group[ri]];
+  const RunDev run = g.runs[ri];
   const int tid = threadIdx.x, p = tid % TH_R, item = tid / TH_R;   // this thread's node, then its multipole
   double S = 0.0, D = 0.0;
   for (int k = 0; k < run.n_orb; ++k) {
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(1024) k_theta_table(GroupArgs g, ThetaArgs t) 
   const int tiles = (n_r + TH_R - 1) / TH_R;
   const int rm = blockIdx.x / tiles, r0 = (blockIdx.x - rm * tiles) * TH_R;
   const int ri = rm / g.n_m, m = rm - ri * g.n_m;
-  const RunDev run = g.runs[g.runs_of_group[ri]];
+  const RunDev run = g.runs[ri];
   double* vs = th_sm;                                           // [n_mp][TH_R]
   double* buf = th_sm + (size_t)n_mp * TH_R;                    // two table chunks
   const double* v = t.vmp + (size_t)ri * n_mp * n_r;
