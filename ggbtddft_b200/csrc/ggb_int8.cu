@@ -614,7 +614,6 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
   constexpr int NB = 2 * NP;                 // B rows: Re of NP points, then Im
   constexpr int B_TILE = NB * 128;           // one slice plane, one k atom
   constexpr int K_ATOMS = NP == 32 ? 1 : 2;  // = M tiles = ceil(N_l / 128)
-  constexpr uint32_t XPLANE = K_ATOMS * B_TILE;  // one slice plane over all k atoms
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ uint64_t full_bar[4], empty_bar[4], acc_bar, xb_bar, drain_bar;
   __shared__ uint32_t tmem_slot;
@@ -1186,7 +1185,11 @@ k_slice_x(const double2* __restrict__ x, int n_r, int n_cols, int cols_pad, int 
 template <int BN>
 static size_t r8_smem(int stages) { return (size_t)stages * R8Tile<BN>::STAGE + 1024; }
 
-static int r8_bn(int n_cols) { return n_cols <= 16 ? 16 : n_cols <= 32 ? 32 : 64; }
+// Columns per tile: the narrowest that takes them all, else 64 (fewest reads of W), but 32 where 64 would
+// leave a second tile of 32 or fewer: the 32-column tile has two accumulator buffers, so its epilogue runs
+// under the next tile's products (90 columns on 600 radii: 126 against 137 us; 72 on 700: 193 against 199;
+// 108 on 900: 556 against 443, 117 on 800: 384 against 348, 189 on 1000: 1011 against 871).
+static int r8_bn(int n_cols) { return n_cols <= 16 ? 16 : n_cols <= 32 || (n_cols > 64 && n_cols <= 96) ? 32 : 64; }
 
 static int r8_stages(int bn) {
   const int stage = R8_W_PLANES * R8_BM * R8_BK + R8_X_PLANES * bn * R8_BK;
