@@ -250,21 +250,21 @@ class ClockSampler:
 
 
 # DRAM traffic per algorithmic byte, dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture
-# (--set full, cold caches) over the launch's algorithmic bytes, for the split_int8 kernels of the
-# committed profiling workloads: ar16-n600 (N_l = 97, the one-M-tile kernel, and the radial product)
-# and ar16-n400-l160 (N_l = 161, the two-M-tile kernel).  The ensemble is too large to capture whole;
-# its traffic is estimated group by group from these ratios (orbital traffic grows in proportion to
-# N_r N_l columns; W in proportion to N_r^2 N_l).  The two-M-tile angular ratios come from the capture
-# with basis reuse (first half: kept vectors in, orbitals out; second half: orbitals in and out, kept
-# vectors out); the one-M-tile ones from a capture of the two-product form of both halves.
+# (--set full, cold caches) over the launch's algorithmic bytes, for the split_int8 kernels on 16 argon
+# runs (144 orbital columns) with basis reuse: N_r 600, N_l 97 (the one-M-tile kernel, and the radial
+# product) and N_r 400, N_l 161 (the two-M-tile kernel).  The ensemble is too large to capture whole; its
+# traffic is estimated group by group from these ratios (orbital traffic grows in proportion to
+# N_r N_l columns; W in proportion to N_r^2 N_l).  First half: kept vectors in, orbitals out; second half:
+# orbitals in and out, kept vectors out.
 MEASURED_TRAFFIC_RATIO = {
-    ("split_int8", "radial", 1): 554.63 / 514.02, ("split_int8", "radial", 2): 554.63 / 514.02,
-    ("split_int8", "angular_first", 1): 212.18 / 268.19, ("split_int8", "angular_second", 1): 241.05 / 268.19,
-    ("split_int8", "angular_first", 2): (149.01 + 104.49) / 296.76,
-    ("split_int8", "angular_second", 2): (150.63 + 279.10) / 445.15,
+    ("split_int8", "radial", 1): (385.98 + 111.78) / 514.02, ("split_int8", "radial", 2): (330.47 + 119.91) / 465.74,
+    ("split_int8", "angular_first", 1): (134.41 + 90.97) / 268.19,
+    ("split_int8", "angular_second", 1): (137.18 + 236.60) / 402.28,
+    ("split_int8", "angular_first", 2): (148.80 + 105.64) / 296.76,
+    ("split_int8", "angular_second", 2): (154.89 + 269.47) / 445.13,
 }
 TRAFFIC_SOURCE = ("per group: algorithmic bytes x (DRAM bytes / algorithmic bytes) of an ncu capture of the same "
-                  "kernel on ar16-n600 (one M tile, radial) or ar16-n400-l160 (two M tiles)")
+                  "kernel on 16 runs at N_r 600, l_max 96 (one M tile) or N_r 400, l_max 160 (two M tiles)")
 
 
 def measured_traffic(runs, groups, precision, phase, theta_reuse: bool = False):

@@ -596,8 +596,8 @@ __device__ __forceinline__ void a8_load_round(StGeom geo, const int8_t* mat, int
 // as four int8 slice planes.  Every point carries one power-of-two scale for its Re and Im rows,
 // chosen from the 2-norm of its l-vector: each product of the chain is an orthogonal matrix and
 // each phase unitary, so that norm bounds every entry of every intermediate vector and one
-// exponent serves the whole chain.  The chain matrices S^T stream through a TMA pipeline, one
-// slice plane per stage.  Orbitals in and out are complex128 (xout may alias xin: each CTA reads
+// exponent serves the whole chain.  The chain matrices S^T stream through a pipeline of bulk
+// copies, one slice plane (or the row tiles of one that fit, a round) per stage.  Orbitals in and out are complex128 (xout may alias xin: each CTA reads
 // its whole tile before it writes).
 //
 // Basis reuse (theta form, t.yth set): a half-step is x <- V diag(phase) V^T x with V orthogonal,

@@ -866,7 +866,7 @@ __host__ __device__ inline int fin_xc_blocks(const GroupArgs& g, int mode) {
 // rows' sums go to a scratch array, and the last of an orbital's rows to finish (a counter per orbital)
 // adds them over l, writes the totals and runs the NaN / norm-growth watchdog.  (Blocks that took a slice of
 // l with one warp per orbital walked its rows one after another: 27 us for nine orbitals, N_l 97, and
-// 88 us for 21 such runs at N_l 161, now 14 and 47 us.)
+// 88 us for 21 such runs at N_l 161, now 10 and 48 us.)
 // ROWS: the observables come from the orbitals x (the partial sums' kernel needs half its registers).
 template <bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const double2* x, int mode) {
