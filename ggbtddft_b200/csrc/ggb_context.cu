@@ -23,6 +23,13 @@ using namespace ggb;
 namespace {
 
 constexpr int COUNTERS = 4;       // ints before the row counters of a group's counter block
+// Steps of the long graph, and of the long graph of a context whose steps fork (k_finalize beside the
+// exact multipoles).  A forked step costs the graph's first instantiation and launch 60 us more than a
+// straight one: at 32 steps a new helium context's first call took 5.7 ms against 3.6 at eight (3.6
+// without the fork, whose step is 9 us longer), three int8 groups 13.3 against 7.9.  Later calls take the
+// same at eight and at 32 (69 us a helium step): a launch every eight steps hides behind them.
+constexpr int GRAPH_STEPS = 32;
+constexpr int GRAPH_STEPS_FORKED = 8;
 
 struct GroupHost {
   ggb_group_desc d{};
@@ -81,9 +88,9 @@ struct ggb_ctx {
   bool prepared = false;
   std::string err;
   int device = 0;
-  // graphs of `graph_steps` steps and of one step: a call of n steps replays the first n / 32 times
-  // and the second n % 32 times, so every step runs from a graph
-  int graph_steps = 32;
+  // graphs of `graph_steps` steps and of one step: a call of n steps replays the first n / graph_steps times
+  // and the second n % graph_steps times, so every step runs from a graph
+  int graph_steps = GRAPH_STEPS;
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph1_exec = nullptr;
   cudaStream_t cap_stream = nullptr;
@@ -792,14 +799,15 @@ int ggb_step(ggb_ctx* ctx, int n_steps, void* stream) {
   for (GroupHost& g : ctx->groups)
     if (g.needs_init)
       if ((rc = launch_init(ctx, g, s))) return rc;
-  const int G = ctx->graph_steps;
   if (!ctx->graph_exec) {
     // capture once, on the first call, so that later calls only replay
+    for (const GroupHost& g : ctx->groups)
+      if (g.args.theta_tab) ctx->graph_steps = GRAPH_STEPS_FORKED;
     if (!ctx->cap_stream) CK(cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
     for (int k = 0; k < 2; ++k) {
       cudaGraph_t graph;
       CK(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
-      const int rc_cap = launch_steps(ctx, ctx->cap_stream, k == 0 ? G : 1);
+      const int rc_cap = launch_steps(ctx, ctx->cap_stream, k == 0 ? ctx->graph_steps : 1);
       CK(cudaStreamEndCapture(ctx->cap_stream, &graph));
       if (rc_cap) {
         cudaGraphDestroy(graph);
@@ -810,6 +818,7 @@ int ggb_step(ggb_ctx* ctx, int n_steps, void* stream) {
     }
   }
   if (n_steps == 0) return GGB_OK;
+  const int G = ctx->graph_steps;
   for (int i = 0; i + G <= n_steps; i += G) CK(cudaGraphLaunch(ctx->graph_exec, s));
   for (int i = 0; i < n_steps % G; ++i) CK(cudaGraphLaunch(ctx->graph1_exec, s));
   CK(cudaGetLastError());

@@ -127,7 +127,8 @@ int ggb_set_field(ggb_ctx* ctx, int run, const double* E, int n_t);
 /* Advance every run by n_steps steps, asynchronously on `stream` (a cudaStream_t).
    The first call after ggb_set_orbitals computes the initial potentials
    (h_timePropagation.cuh:47-57).  Every step runs from a captured CUDA graph: a 32-step graph
-   replayed n_steps / 32 times, then a 1-step graph n_steps % 32 times. */
+   replayed n_steps / 32 times, then a 1-step graph n_steps % 32 times (8 in place of 32 where a
+   group has more than four Hartree multipoles). */
 int ggb_step(ggb_ctx* ctx, int n_steps, void* stream);
 
 /* Profiling hook: launch one phase of the step for every group on `stream`

@@ -90,6 +90,26 @@ def test_fp64_multipole_kernels_at_their_edges(n_r, n_l, n_har):
     assert rel_err(got["norm"], ref["norm"]) < 1e-10
 
 
+@pytest.mark.parametrize("n_har", [4, 17])
+def test_steps_in_one_call_equal_single_steps(n_har):
+    """Calls on both sides of the long graph's length, with and without the forked potentials: the same
+    kernels on the same data, so the same bits as one step at a time."""
+    run = P.reference_like(37, 9, 64, "Ne3", r_mask=15.0, dt_as=10.0, perturb=0.05, seed=3)
+    run = dataclasses.replace(run, angular="theta", n_har=n_har)
+    one, many = (TimePropagation([run], precision="fp64", per_l=True) for _ in range(2))
+    done = 0
+    for n in (0, 1, 7, 8, 9, 33):
+        many.step(n)
+        for _ in range(n):
+            one.step(1)
+        done += n
+        assert np.array_equal(many.orbitals(0), one.orbitals(0)), done
+    for a, b in zip(many.observables(0), one.observables(0)):
+        assert np.array_equal(np.asarray(a), np.asarray(b))
+    one.close()
+    many.close()
+
+
 @pytest.mark.parametrize("n_r,n_l,angular", [(7, 5, "reference"), (41, 8, "reference"), (33, 9, "theta"), (50, 65, "reference"),
                                              (130, 129, "theta"), (21, 193, "theta")])
 def test_fp64_angular_tiles_at_their_edges(n_r, n_l, angular):
