@@ -718,7 +718,8 @@ int ggb_set_angular(ggb_ctx* ctx, int group, int coupling, int m, const double* 
   return GGB_OK;
 }
 
-// Copies `bytes` from a host or device pointer to host memory (plain host memory without a driver call).
+// Copies `bytes` from a host or device pointer to host memory: host memory without a driver call, so the
+// caller waits first for whatever is still to fill it.
 static int to_host(ggb_ctx* ctx, void* dst, const void* src, size_t bytes) {
   cudaPointerAttributes at;
   CK(cudaPointerGetAttributes(&at, src));
@@ -740,6 +741,9 @@ int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const
   std::vector<int> nl_(no), nm(no), nocc(no);
   std::vector<double> rho(nr);
   int rc;
+  // host arrays are read when what was queued before this call on the legacy or a blocking stream is done
+  // (an asynchronous copy into a pinned array), as copies on the legacy stream would be
+  CK(cudaStreamSynchronize(0));
   if ((rc = to_host(ctx, nl_.data(), l, no * sizeof(int))) || (rc = to_host(ctx, nm.data(), m, no * sizeof(int))) ||
       (rc = to_host(ctx, nocc.data(), occ, no * sizeof(int))) ||
       (rc = to_host(ctx, rho.data(), rho_frozen, nr * sizeof(double))))
