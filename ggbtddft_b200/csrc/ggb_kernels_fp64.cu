@@ -917,16 +917,17 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
           }
 #pragma unroll
         for (int q = 0; q < 5; ++q) sum2_warp(s[q]);
-        const double nrm = s[4].hi + s[4].lo;
+        // a sum that overflowed is a NaN in hi + lo only (hi stays infinite)
+        const double nrm = s[4].hi + s[4].lo, dip = s[0].hi + s[0].lo, acc = s[2].hi + s[2].lo;
         if (lane == 0) {
           if (mode == 0) {
             run.norm0[k] = nrm;                 // for the growth watchdog
           } else {
-            run.dip_tot[(size_t)k * run.n_t + step] = make_double2(s[0].hi + s[0].lo, s[1].hi + s[1].lo);
-            run.acc_tot[(size_t)k * run.n_t + step] = make_double2(s[2].hi + s[2].lo, s[3].hi + s[3].lo);
+            run.dip_tot[(size_t)k * run.n_t + step] = make_double2(dip, s[1].hi + s[1].lo);
+            run.acc_tot[(size_t)k * run.n_t + step] = make_double2(acc, s[3].hi + s[3].lo);
             run.norm[(size_t)k * run.n_t + step] = nrm;
             if (mode == 1) {
-              if (!(nrm == nrm) || isinf(nrm) || !(s[0].hi == s[0].hi) || !(s[2].hi == s[2].hi)) atomicOr(g.status, ST_NAN);
+              if (!(nrm == nrm) || isinf(nrm) || !(dip == dip) || !(acc == acc)) atomicOr(g.status, ST_NAN);
               if (nrm > run.norm0[k] * (1.0 + g.norm_tol) + 1e-300) atomicOr(g.status, ST_NORM_GROWTH);
             }
           }
