@@ -698,7 +698,11 @@ int ggb_set_radial_propagators(ggb_ctx* ctx, int group, const double* W) {
   const size_t n = (size_t)g.d.n_l * g.d.n_r * g.d.n_r;
   CK(cudaMemcpy(g.W_d, W, n * sizeof(double2), cudaMemcpyDefault));
   g.w_set = true;
-  ctx->prepared = ctx->prepared && ctx->dims.precision == GGB_FP64;
+  if (ctx->prepared && ctx->dims.precision != GGB_FP64) {
+    // the split forms' operands in place: the captured graphs keep the buffers they name
+    const int rc = mixed_set_w(g.mixed, g.args, g.W_d);
+    if (rc) return fail(ctx, rc, "propagator conversion failed");
+  }
   return GGB_OK;
 }
 

@@ -1211,6 +1211,16 @@ static size_t a8_smem(int k_atoms, int stages) {
     }                                                                    \
   } while (0)
 
+// the W planes and row exponents of these propagators, into the buffers of int8_prepare (legacy stream)
+void int8_slice_w(MixedGroup& mg, const GroupArgs& a, const double2* W_fp64) {
+  const I8Group& q = mg.i8;
+  const int n_r = a.n_r, n_l = a.n_l, rows8 = (n_r + 7) & ~7;
+  k_w_rowmax<<<dim3((mg.rows_pad + 127) / 128, n_l), 128>>>(W_fp64, q.wexp, n_r, mg.rows_pad);
+  const dim3 tb(32, 8), tg((mg.rows_pad + 31) / 32, (mg.k_pad + 31) / 32, n_l);
+  for (int v = 0; v < I8_W_VARIANTS; ++v)
+    k_slice_w_i8<<<tg, tb>>>(W_fp64, q.wexp, q.W + q.w_variant * v, n_r, rows8, mg.rows_pad, mg.k_pad, v, I8_W_VARIANTS);
+}
+
 int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats, std::string& err) {
   const int n_r = a.n_r, n_l = a.n_l;
   I8Group& q = mg.i8;
@@ -1224,10 +1234,7 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
   q.w_variant = nw;
   I8_CK(cudaMalloc(&q.W, nw * I8_W_VARIANTS));
   I8_CK(cudaMalloc(&q.wexp, (size_t)n_l * mg.rows_pad * sizeof(int)));
-  k_w_rowmax<<<dim3((mg.rows_pad + 127) / 128, n_l), 128>>>(W_fp64, q.wexp, n_r, mg.rows_pad);
-  const dim3 tb(32, 8), tg((mg.rows_pad + 31) / 32, (mg.k_pad + 31) / 32, n_l);
-  for (int v = 0; v < I8_W_VARIANTS; ++v)
-    k_slice_w_i8<<<tg, tb>>>(W_fp64, q.wexp, q.W + nw * v, n_r, rows8, mg.rows_pad, mg.k_pad, v, I8_W_VARIANTS);
+  int8_slice_w(mg, a, W_fp64);
   I8_CK(cudaGetLastError());
   // radial B operand planes
   const size_t nx = (size_t)n_l * R8_X_PLANES * q.cols_pad * mg.k_pad;

@@ -643,6 +643,11 @@ static int stages_for(int bn) {
   return s;
 }
 
+static void split_w(MixedGroup& m, const GroupArgs& a, const double2* W_fp64) {
+  const dim3 tb(32, 8), tg((m.rows_pad + 31) / 32, (m.k_pad + 31) / 32, a.n_l);
+  k_split_w<<<tg, tb>>>(W_fp64, m.Wsp, a.n_r, m.rows_pad, m.k_pad);
+}
+
 int mixed_prepare(MixedGroup& m, GroupArgs& a, const double2* W_fp64, double2* x_fp64, double2* y_fp64,
                   int precision, std::string& err) {
   if (precision != GGB_SPLIT_BF16 && precision != GGB_SPLIT_INT8) {
@@ -686,8 +691,7 @@ int mixed_prepare(MixedGroup& m, GroupArgs& a, const double2* W_fp64, double2* x
   MX_CK(cudaMemset(m.Xsp, 0, nxs * sizeof(__nv_bfloat16)));
   const size_t nws = (size_t)n_l * W_PLANES * m.rows_pad * m.k_pad;
   MX_CK(cudaMalloc(&m.Wsp, nws * sizeof(__nv_bfloat16)));
-  const dim3 tb(32, 8), tg((m.rows_pad + 31) / 32, (m.k_pad + 31) / 32, n_l);
-  k_split_w<<<tg, tb>>>(W_fp64, m.Wsp, n_r, m.rows_pad, m.k_pad);
+  split_w(m, a, W_fp64);
   MX_CK(cudaGetLastError());
   const size_t n_mat_el = (size_t)n_mats * a.n_m * n_l * a.ldS;
   MX_CK(cudaMalloc(&m.mats_f, n_mat_el * sizeof(float)));
@@ -730,6 +734,13 @@ int mixed_prepare(MixedGroup& m, GroupArgs& a, const double2* W_fp64, double2* x
   MX_CK(cudaDeviceSynchronize());
   m.ready = true;
   return GGB_OK;
+}
+
+int mixed_set_w(MixedGroup& m, const GroupArgs& a, const double2* W_fp64) {
+  if (!m.ready) return GGB_ERR_STATE;
+  if (m.precision == GGB_SPLIT_INT8) int8_slice_w(m, a, W_fp64);
+  else split_w(m, a, W_fp64);
+  return cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess ? GGB_OK : GGB_ERR_CUDA;
 }
 
 int mixed_load_orbitals(MixedGroup& m, const GroupArgs& a, const double2* x_fp64) {

@@ -76,6 +76,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn tensor_map_encoder();
 
 int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats, std::string& err);
+void int8_slice_w(MixedGroup& mg, const GroupArgs& a, const double2* W_fp64);
 void int8_radial(MixedGroup& mg, const GroupArgs& a, cudaStream_t s);
 void int8_angular(MixedGroup& mg, const GroupArgs& a, int half, const double2* xin, double2* xout, cudaStream_t s);
 void int8_slice_x(MixedGroup& mg, const GroupArgs& a, const double2* x, cudaStream_t s);
@@ -88,6 +89,7 @@ void launch_angular_tc(const MixedGroup& mg, const GroupArgs& a, int half, const
 
 int mixed_prepare(MixedGroup& m, GroupArgs& a, const double2* W_fp64, double2* x_fp64, double2* y_fp64,
                   int precision, std::string& err);
+int mixed_set_w(MixedGroup& m, const GroupArgs& a, const double2* W_fp64);   // other propagators, in place
 int mixed_load_orbitals(MixedGroup& m, const GroupArgs& a, const double2* x_fp64);
 int mixed_store_orbitals(MixedGroup& m, const GroupArgs& a, double2* x_fp64);
 void mixed_init(MixedGroup& m, const GroupArgs& a, const double2* x_fp64, cudaStream_t s);

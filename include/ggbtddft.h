@@ -109,7 +109,8 @@ int ggb_set_grid(ggb_ctx* ctx, int group, const double* r, const double* drdx, c
 /* Radial propagators W[l][a][b], complex128, the propagatorL%03d.bin layout
    (h_initialisePropagators.cuh:12-22).  Applied as x_l <- A x_l with A(a,b) = W[l][b][a],
    i.e. the column-major reading of cublasZgemmBatched in h_propagationH0
-   (h_timePropagation.cuh:1-30). */
+   (h_timePropagation.cuh:1-30).  Called again after a step, the next steps take the new ones (the
+   orbitals stay; synchronous, with no step in flight). */
 int ggb_set_radial_propagators(ggb_ctx* ctx, int group, const double* W);
 
 /* Eigen-system of one angular coupling for one m: V[l][j] (N_l x N_l) and D[j] (N_l), the
