@@ -907,6 +907,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
       if (lane == 0) last = atomicAdd(g.fin_cnt + col, 1u) == (unsigned)(n_l - (ROWS ? 1 : 0));
       if (__shfl_sync(0xffffffffu, last, 0)) {
         __threadfence();
+        __syncwarp();                           // lane 0 counted; the shuffle alone orders no memory
 #pragma unroll
         for (int q = 0; q < 5; ++q) s[q] = dd{0.0, 0.0};
         for (int lp = lane; lp < n_l + (ROWS ? 0 : 1); lp += 32)
