@@ -1083,9 +1083,10 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
-    if (abort_flag && lane == 0) {
-      tc_commit(&drain_bar);
-      mbar_drain(&drain_bar, 0);
+    if (abort_flag) {
+      // the lane that issued the products commits them (elect.sync gives the same one every time)
+      tc_commit_if(elect_one(), &drain_bar);
+      if (lane == 0) mbar_drain(&drain_bar, 0);
     }
     __syncwarp();
     tc_fence_after();
