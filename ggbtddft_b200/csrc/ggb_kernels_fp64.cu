@@ -696,34 +696,59 @@ k_radial_fp64_rows(int n_r, int l_keep, const double2* __restrict__ W, const dou
 
 static int g_radial_sms = 0;
 
+// The tile form also for one, two and six columns on large grids whose tiles of 128 radii fill their rounds
+// over the resident CTAs: there it streams W at 5.5 - 7 TB/s, the row form at 4.6 - 6.3 (one column, many
+// rounds of short blocks), 3.8 - 5.5 (two, plain FMAs) and 4.8 - 5.5 (six, padded to eight).  Row -> tile
+// form, a step in the graph: N_r 2000, N_l 17, one column 267 -> 188 us; 1000/33/1 139 -> 107; 1000/97/2
+// 352 -> 292; 1000/33/6 153 -> 142.  Below 640 radii (much of W or of a round in L2, latency) the row form's
+// step is the faster one (250/145/1 14 %, 350/129/2 16 %), in part-empty rounds too (600/65/1 90 -> 73 us alone).
+static bool radial_tiles(int n_cols, int n_r, int n_l) {
+  if (n_cols > RF_MAX_COLS) return true;
+  if (n_r < 640 || !(n_cols <= 2 || n_cols == 6)) return false;
+  const long tiles = (long)((n_r + RAD_TI - 1) / RAD_TI) * n_l, resident = 2 * g_radial_sms;
+  const double fill = n_cols == 2 ? 0.58 : 0.77;    // of the rounds, by rows of W
+  return (double)n_r * n_l >= fill * RAD_TI * resident * ((tiles + resident - 1) / resident);
+}
+
+template <int TC>
+static void launch_radial_tiles(const GroupArgs& g, const double2* W, const double2* xin, double2* xout, cudaStream_t s) {
+  const int tiles = ((g.n_r + RAD_TI - 1) / RAD_TI) * ((g.n_cols + TC - 1) / TC) * g.n_l;
+  k_radial_fp64<TC><<<std::min(tiles, 2 * g_radial_sms), RAD_THREADS, radial_fp64_smem<TC>(), s>>>(g.n_r, g.n_cols, g.n_l, W, xin,
+                                                                                               xout, g.status);
+}
+
 void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin, double2* xout, cudaStream_t s) {
   const int nc = g.n_cols;
-  if (nc <= RF_MAX_COLS) {
-    const int blocks = g.n_l * ((g.n_r + 31) / 32);
-    const int l_keep = (int)(RF_KEEP / (sizeof(double2) * g.n_r * g.n_r));
-    // eight warps a block until four blocks an SM are there, then four (fewer k slices to start and
-    // to add: 138 -> 133 us at 600/97/9; below, the smaller blocks leave the SMs emptier)
-    const bool wide = blocks < 4 * g_radial_sms;
+  if (radial_tiles(nc, g.n_r, g.n_l)) {
+    if (nc == 1) launch_radial_tiles<1>(g, W, xin, xout, s);
+    else if (nc == 2) launch_radial_tiles<2>(g, W, xin, xout, s);
+    else if (nc <= 6) launch_radial_tiles<6>(g, W, xin, xout, s);
+    else if (nc <= 12) launch_radial_tiles<12>(g, W, xin, xout, s);
+    else launch_radial_tiles<16>(g, W, xin, xout, s);
+    return;
+  }
+  const int blocks = g.n_l * ((g.n_r + 31) / 32);
+  const int l_keep = (int)(RF_KEEP / (sizeof(double2) * g.n_r * g.n_r));
+  // eight warps a block until four blocks an SM are there, then four (fewer k slices to start and
+  // to add: 138 -> 133 us at 600/97/9; below, the smaller blocks leave the SMs emptier)
+  const bool wide = blocks < 4 * g_radial_sms;
 #define GGB_RF_CASE(C)                                                                       \
   case C:                                                                                    \
     if (wide) k_radial_fp64_rows<C, 8><<<blocks, 256, 0, s>>>(g.n_r, l_keep, W, xin, xout);  \
     else k_radial_fp64_rows<C, 4><<<blocks, 128, 0, s>>>(g.n_r, l_keep, W, xin, xout);       \
     break;
-    switch (nc) {
-      GGB_RF_CASE(1) GGB_RF_CASE(2) GGB_RF_CASE(3) GGB_RF_CASE(4) GGB_RF_CASE(5)
-      GGB_RF_CASE(6) GGB_RF_CASE(7) GGB_RF_CASE(8) GGB_RF_CASE(9)
-      default: break;
-    }
-#undef GGB_RF_CASE
-    return;
+  switch (nc) {
+    GGB_RF_CASE(1) GGB_RF_CASE(2) GGB_RF_CASE(3) GGB_RF_CASE(4) GGB_RF_CASE(5)
+    GGB_RF_CASE(6) GGB_RF_CASE(7) GGB_RF_CASE(8) GGB_RF_CASE(9)
+    default: break;
   }
-  const int tc = nc <= 12 ? 12 : 16;
-  const int tiles = ((g.n_r + RAD_TI - 1) / RAD_TI) * ((nc + tc - 1) / tc) * g.n_l;
-  const int ctas = std::min(tiles, 2 * g_radial_sms);
-  if (tc == 12)
-    k_radial_fp64<12><<<ctas, RAD_THREADS, radial_fp64_smem<12>(), s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status);
-  else
-    k_radial_fp64<16><<<ctas, RAD_THREADS, radial_fp64_smem<16>(), s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status);
+#undef GGB_RF_CASE
+}
+
+template <int TC>
+static cudaError_t configure_radial_tiles() {
+  return cudaFuncSetAttribute((const void*)k_radial_fp64<TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)radial_fp64_smem<TC>());
 }
 
 static cudaError_t configure_radial_fp64() {
@@ -731,12 +756,12 @@ static cudaError_t configure_radial_fp64() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&g_radial_sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute((const void*)k_radial_fp64<12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)radial_fp64_smem<12>());
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute((const void*)k_radial_fp64<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)radial_fp64_smem<16>());
+  if (e == cudaSuccess) e = configure_radial_tiles<1>();
+  if (e == cudaSuccess) e = configure_radial_tiles<2>();
+  if (e == cudaSuccess) e = configure_radial_tiles<6>();
+  if (e == cudaSuccess) e = configure_radial_tiles<12>();
+  if (e == cudaSuccess) e = configure_radial_tiles<16>();
+  return e;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -9,6 +9,7 @@ import dataclasses
 import numpy as np
 import pytest
 
+from ggbtddft_b200 import inputs as I
 from ggbtddft_b200 import problems as P
 from ggbtddft_b200.engine import TimePropagation, load_library
 
@@ -35,6 +36,27 @@ def test_fp64_radial_product_at_every_column_count(n_r, cols):
     for r, g in zip(runs, got):
         want = np.einsum("lba,lkb->lka", base.W, r.x0)
         assert np.linalg.norm(g - want) < TOL * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n_r,n_l", [(650, 45), (1001, 33)])
+def test_fp64_radial_product_of_few_columns_on_large_grids(n_r, n_l):
+    """One, two and six columns where the tiles of 128 radii fill the GPU (the tile form's own column
+    counts), the last tile and k chunk part full, and three, which stay on the row form."""
+    rng = np.random.default_rng(n_r)
+    grid, ang = I.make_grid(n_r, 0.5 * n_r, I.zeta_physical_to_ref(0.5, 0.5 * n_r)), I.angular_eigensystems(n_l, 1)
+    w = rng.standard_normal((n_l, n_r, n_r, 2)).view(np.complex128)[..., 0] / np.sqrt(2.0 * n_r)
+    for cols in (1, 2, 3, 6):
+        x = rng.standard_normal((n_l, cols, n_r)) + 1j * rng.standard_normal((n_l, cols, n_r))
+        m = np.zeros(cols, np.int32)
+        run = P.RunInputs(grid=grid, n_l=n_l, dt=0.02, W=w, V={c: ang[c][0] for c in I.COUPLINGS},
+                          D={c: ang[c][1] for c in I.COUPLINGS}, x0=x / np.linalg.norm(x), l_active=m, m_active=m, occ=m + 1,
+                          rho_frozen=np.zeros(n_r), E=np.zeros(1), use_hartree=0, angular="theta")
+        tp = TimePropagation([run], precision="fp64")
+        tp.step(1)
+        got = tp.orbitals(0)
+        tp.close()
+        want = np.matmul(run.x0, w)
+        assert np.linalg.norm(got - want) < TOL * np.linalg.norm(want)
 
 
 @pytest.mark.parametrize("n_l,n_orb,n_r", [(2, 1, 1), (5, 2, 127), (9, 3, 128), (17, 1, 129), (33, 4, 600)])
