@@ -25,22 +25,27 @@ constexpr int NA_MAX_NL = 256;
 // Norm partials (dd), one per (orbital, l): n_orb * N_l <= NA_MAX_PARTIALS (1 MiB).
 static __device__ __align__(256) double2 g_norm_scratch[NA_MAX_PARTIALS];
 
-// One block per (l, orbital) row.  The rows l - 1, l and l + 1 of the orbital come straight from L2
-// (each is read three times: 25 MB of L2 traffic for nine orbitals on 600 radii, 97 l), a thread
-// sums its radii in double-double, and one reduction over the block ends the row: no partial sums
-// per tile of radii, no second pass over them, and one reduction per row where the tile form
-// (a warp reduction of every row for every 32 radii) made ceil(N_r / 32).  128 threads: a row of
-// 600 radii is five loads per thread, all rows of a call are resident at once.  Bound by the latency
-// of one load, the five sums and the reduction; N_r 600, N_l 97, nine orbitals: 12.3 us a
-// call with the norm kernel, 44.7 us as tiles and a reduction kernel.
+// T threads per (l, orbital) row, NA_THREADS / T rows a block.  The rows l - 1, l and l + 1 of the orbital come
+// straight from L2 (each is read three times: 25 MB of L2 traffic for nine orbitals on 600 radii, 97 l), a
+// thread sums its radii in double-double, and one reduction over the row's threads ends it: no partial sums
+// per tile of radii, no second pass over them, and one reduction per row where the tile form (a warp
+// reduction of every row for every 32 radii) made ceil(N_r / 32).  T = 128: a row of 600 radii is five loads
+// per thread, all rows of a call are resident at once; bound by the latency of one load, the five sums
+// and the reduction (N_r 600, N_l 97, nine orbitals: 12.3 us a call with the norm kernel, 44.7 us as tiles and
+// a reduction kernel).  T = 32 up to 128 radii, where the reductions are the work: 65536 rows of 32 radii
+// 60 us (128 threads: 189; tiles: 119), 25854 of 31 radii 27 (78; 43); a few hundred rows take the 6.5 us of
+// the launches either way.
 constexpr int NA_THREADS = 128;
 
+template <int T>
 __global__ void __launch_bounds__(NA_THREADS)
 k_obs_rows(const double2* __restrict__ x, const double* __restrict__ r, const double* __restrict__ coef,
            const int* __restrict__ m_of, int n_l, int n_orb, int n_r, double2* __restrict__ dip,
            double2* __restrict__ acc, double2* __restrict__ norm_part) {
   asm volatile("griddepcontrol.launch_dependents;");
-  const int l = blockIdx.x / n_orb, k = blockIdx.x - l * n_orb;
+  const int row_id = blockIdx.x * (NA_THREADS / T) + threadIdx.x / T, tid = threadIdx.x % T;
+  if (T < NA_THREADS && row_id >= n_l * n_orb) return;   // whole warps
+  const int l = row_id / n_orb, k = row_id - l * n_orb;
   int m = m_of[k];
   if (m < 0 || m > n_l) m = n_l;   // an invalid m contributes nothing (no l satisfies l >= m)
   // dipole (re, im), acceleration (re, im), norm
@@ -54,7 +59,7 @@ k_obs_rows(const double2* __restrict__ x, const double* __restrict__ r, const do
     const double c_d = down ? coef[((size_t)CF_CD * NA_MAX_NL + m) * NA_MAX_NL + l] : 0.0;
     const size_t ls = (size_t)n_orb * n_r;
     const double2* row = x + (size_t)l * ls + (size_t)k * n_r;
-    for (int i = threadIdx.x; i < n_r; i += NA_THREADS) {
+    for (int i = tid; i < n_r; i += T) {
       const double2 xl = row[i];
       const double2 xu = up ? row[ls + i] : make_double2(0.0, 0.0);
       const double2 xd = down ? (row - ls)[i] : make_double2(0.0, 0.0);
@@ -69,24 +74,33 @@ k_obs_rows(const double2* __restrict__ x, const double* __restrict__ r, const do
       s[4] = dd_add(s[4], dd{xl.x * xl.x + xl.y * xl.y, 0.0});
     }
   }
-  __shared__ dd part[NA_THREADS / 32][5];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
     for (int q = 0; q < 5; ++q)
       s[q] = dd_add(s[q], dd{__shfl_xor_sync(0xffffffffu, s[q].hi, o), __shfl_xor_sync(0xffffffffu, s[q].lo, o)});
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int q = 0; q < 5; ++q) part[threadIdx.x >> 5][q] = s[q];
-  __syncthreads();
-  if (threadIdx.x < 5) {
-    dd t = part[0][threadIdx.x];
-#pragma unroll
-    for (int w = 1; w < NA_THREADS / 32; ++w) t = dd_add(t, part[w][threadIdx.x]);
-    const size_t o = (size_t)l * n_orb + k;
-    if (threadIdx.x < 2) reinterpret_cast<double*>(dip + o)[threadIdx.x] = t.hi + t.lo;
-    else if (threadIdx.x < 4) reinterpret_cast<double*>(acc + o)[threadIdx.x - 2] = t.hi + t.lo;
+  const size_t o = (size_t)l * n_orb + k;
+  auto store = [&](int q, dd t) {
+    if (q < 2) reinterpret_cast<double*>(dip + o)[q] = t.hi + t.lo;
+    else if (q < 4) reinterpret_cast<double*>(acc + o)[q - 2] = t.hi + t.lo;
     else norm_part[(size_t)k * n_l + l] = make_double2(t.hi, t.lo);
+  };
+  if constexpr (T == 32) {
+    if (tid == 0)
+#pragma unroll
+      for (int q = 0; q < 5; ++q) store(q, s[q]);
+  } else {
+    __shared__ dd part[T / 32][5];
+    if ((tid & 31) == 0)
+#pragma unroll
+      for (int q = 0; q < 5; ++q) part[tid >> 5][q] = s[q];
+    __syncthreads();
+    if (tid < 5) {
+      dd t = part[0][tid];
+#pragma unroll
+      for (int w = 1; w < T / 32; ++w) t = dd_add(t, part[w][tid]);
+      store(tid, t);
+    }
   }
 }
 
@@ -161,8 +175,14 @@ extern "C" int ggb_observables_noalloc(const double* x, const double* r, const i
   if (rc) return rc;
   const NoallocDevice& d = g_dev[dev];
   cudaStream_t s = (cudaStream_t)stream;
-  k_obs_rows<<<n_l * n_orb, NA_THREADS, 0, s>>>(reinterpret_cast<const double2*>(x), r, d.coef, m, n_l, n_orb, n_r,
-                                                 reinterpret_cast<double2*>(dip), reinterpret_cast<double2*>(acc), d.norm);
+  const int rows = n_l * n_orb;
+  const double2* xs = reinterpret_cast<const double2*>(x);
+  double2 *ds = reinterpret_cast<double2*>(dip), *as = reinterpret_cast<double2*>(acc);
+  if (n_r <= NA_THREADS)
+    k_obs_rows<32><<<(rows + NA_THREADS / 32 - 1) / (NA_THREADS / 32), NA_THREADS, 0, s>>>(xs, r, d.coef, m, n_l, n_orb, n_r, ds, as,
+                                                                                           d.norm);
+  else
+    k_obs_rows<NA_THREADS><<<rows, NA_THREADS, 0, s>>>(xs, r, d.coef, m, n_l, n_orb, n_r, ds, as, d.norm);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute after{};
   after.id = cudaLaunchAttributeProgrammaticStreamSerialization;

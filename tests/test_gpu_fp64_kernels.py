@@ -92,6 +92,12 @@ def test_observables_noalloc_at_the_edges(n_l, n_orb, n_r):
     assert np.allclose(norm.cpu().numpy(), (np.abs(x) ** 2).sum(axis=(0, 2)), rtol=TOL, atol=0)
 
 
+@pytest.mark.parametrize("n_l,n_orb,n_r", [(7, 3, 3), (3, 2, 31), (129, 1, 32), (31, 7, 33)])
+def test_observables_noalloc_rows_that_do_not_fill_a_block(n_l, n_orb, n_r):
+    """Several short rows a block, the last block part full."""
+    test_observables_noalloc_at_the_edges(n_l, n_orb, n_r)
+
+
 @pytest.mark.parametrize("n_r,n_l,n_har", [(9, 8, 5), (13, 9, 17), (37, 33, 65), (45, 40, 33), (66, 36, 71)])
 def test_fp64_multipole_kernels_at_their_edges(n_r, n_l, n_har):
     """The theta form's exact multipoles at radii that do not fill a block's four, nodes and multipoles
