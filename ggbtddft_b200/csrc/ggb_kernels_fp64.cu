@@ -297,6 +297,179 @@ k_angular_fp64(GroupArgs g, int half, const double2* __restrict__ xin, double2* 
   }
 }
 
+// The same half-step for groups of many tiles: blocks of four warps on 16 radii, so that several share an SM
+// and one's products run under another's phases and waits (with eight row groups a block's sixteen warps wait
+// for one another three times per product, and one or two blocks fill an SM).  The tile is held twice, a
+// product reads one copy and writes the other: one barrier per product.  A warp takes pairs of 8-channel
+// tiles one after the other over all 32 columns, its S fragments AS_KU pairs of k steps ahead, and the
+// phases are applied to its accumulators.  Bound by the FP64 pipe, which the products share with the phases'
+// sines: 575 radii, N_l 70, 120 columns, five products 450 us, 15 TFLOP/s of products alone.
+constexpr int AS_WARPS = 4, AS_P = 16, AS_LD = 2 * AS_P + 8, AS_NT = 2 * AS_P / 8, AS_KU = 2;
+__global__ void __launch_bounds__(AS_WARPS * 32)
+k_angular_fp64_small(GroupArgs g, int half, const double2* __restrict__ xin, double2* xout, int do_den) {
+  extern __shared__ __align__(16) double smd[];
+  __shared__ double s_rE[AS_P], s_v1[AS_P], s_v2[AS_P], s_v3[AS_P], s_sb[AS_P];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gid = lane >> 2, q = lane & 3;
+  const int n_l = g.n_l, n8 = (n_l + 7) / 8;
+  const int tilesN = (g.n_r + AS_P - 1) / AS_P;
+  const int col = blockIdx.x / tilesN;
+  const int r0 = (blockIdx.x - col * tilesN) * AS_P;
+  const int m = g.col_m[col];
+  const Chain& ch = g.chain[half];
+  double* xs = smd;
+  double* ys = smd + (size_t)8 * n8 * AS_LD;
+  const RunDev run = g.runs[g.col_run[col]];
+  int step = *g.step;
+  if (step >= run.n_t) step = run.n_t - 1;  // overflow is flagged by k_finalize
+  for (int i = tid; i < 8 * n8 * AS_P; i += AS_WARPS * 32) {
+    const int l = i / AS_P, p = i - l * AS_P, r = r0 + p;
+    const double2 v = (l < n_l && r < g.n_r) ? xin[((size_t)l * g.n_cols + col) * g.n_r + r] : make_double2(0.0, 0.0);
+    *reinterpret_cast<double2*>(xs + (size_t)l * AS_LD + 2 * p) = v;
+    if (l >= n_l) *reinterpret_cast<double2*>(ys + (size_t)l * AS_LD + 2 * p) = make_double2(0.0, 0.0);
+  }
+  if (tid < AS_P) {
+    const int r = r0 + tid;
+    const bool rv = r < g.n_r;
+    const int rc = rv ? r : 0;
+    const double rr = rv ? g.r[r] : 1.0;
+    double v1 = 0.0, v2 = 0.0, v3 = 0.0, sbase = 0.0;
+    if (g.hartree_on) {
+      v1 = run.v[1 * g.n_r + rc];
+      v2 = run.v[2 * g.n_r + rc];
+      v3 = run.v[3 * g.n_r + rc];
+      sbase = run.v[rc] - run.v0[rc] + run.vexc[rc] - run.vexc0[rc];
+    }
+    s_rE[tid] = rr * run.E[step];
+    s_v1[tid] = v1;
+    s_v2[tid] = v2;
+    s_v3[tid] = v3;
+    s_sb[tid] = sbase;
+  }
+  const double hdt = 0.5 * g.dt;
+  const double* pco = g.coef + ((size_t)CF_P * g.n_m + m) * n_l;
+  __syncthreads();
+  if (ch.pre_s) {
+    for (int i = tid; i < n_l * AS_P; i += AS_WARPS * 32) {
+      const int l = i / AS_P, p = i - l * AS_P;
+      double eta = s_sb[p] + pco[l] * s_v2[p];
+      eta *= hdt;
+      double2* x = reinterpret_cast<double2*>(xs + (size_t)l * AS_LD + 2 * p);
+      *x = cmul_conj_phase(*x, eta);
+    }
+    __syncthreads();
+  }
+  const double2* Sm = reinterpret_cast<const double2*>(g.frag) + (size_t)m * n8 * n8 * 32 + lane;
+  const size_t mat_stride = (size_t)g.n_m * n8 * n8 * 32;
+  for (int o = 0; o < ch.n_ops; ++o) {
+    const ChainOp op = ch.ops[o];
+    const double2* S = Sm + op.mat * mat_stride;
+    const bool last = (o == ch.n_ops - 1);
+    const double* Dv = g.dph + ((size_t)op.coupling * g.n_m + m) * g.ldS;
+    for (int pr = warp; 2 * pr < n8; pr += AS_WARPS) {
+      double acc[2][AS_NT][2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int nt = 0; nt < AS_NT; ++nt) acc[t][nt][0] = acc[t][nt][1] = 0.0;
+      double2 fa[AS_KU][2], fn[AS_KU][2];
+      auto load_a = [&](int kp0, double2 (&dst)[AS_KU][2]) {
+#pragma unroll
+        for (int u = 0; u < AS_KU; ++u)
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            dst[u][t] = kp0 + u < n8 && 2 * pr + t < n8 ? __ldg(S + ((size_t)(2 * pr + t) * n8 + kp0 + u) * 32) : make_double2(0.0, 0.0);
+      };
+      load_a(0, fa);
+      for (int kp0 = 0; kp0 < n8; kp0 += AS_KU) {
+        load_a(kp0 + AS_KU, fn);
+#pragma unroll
+        for (int u = 0; u < AS_KU; ++u) {
+          if (kp0 + u < n8) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const double* xr = xs + (size_t)((kp0 + u) * 8 + 4 * e + q) * AS_LD + gid;
+              double fb[AS_NT];
+#pragma unroll
+              for (int nt = 0; nt < AS_NT; ++nt) fb[nt] = xr[nt * 8];
+#pragma unroll
+              for (int nt = 0; nt < AS_NT; ++nt) {
+                mma_f64_8x8x4(acc[0][nt][0], acc[0][nt][1], e ? fa[u][0].y : fa[u][0].x, fb[nt]);
+                mma_f64_8x8x4(acc[1][nt][0], acc[1][nt][1], e ? fa[u][1].y : fa[u][1].x, fb[nt]);
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < AS_KU; ++u) { fa[u][0] = fn[u][0]; fa[u][1] = fn[u][1]; }
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int j = pr * 16 + 8 * t + gid;
+        if (j >= n_l) continue;
+        const double dj = Dv[j];
+#pragma unroll
+        for (int nt = 0; nt < AS_NT; ++nt) {
+          const int p = 4 * nt + q;
+          double2 y = make_double2(acc[t][nt][0], acc[t][nt][1]);
+          // the phases of the kernel above
+          if (op.phase == PH_THETA && j >= m) {
+            double eta = (s_rE[p] + s_v1[p]) * dj + s_v2[p] * legendre_p2(dj) + s_v3[p] * legendre_p3(dj) + s_sb[p];
+            if (g.theta_tab && r0 + p < g.n_r) eta += run.htab[((size_t)m * n_l + j) * g.n_r + r0 + p];
+            eta *= hdt;
+            y = cmul_conj_phase(y, eta);
+          } else if (op.phase != PH_NONE && j >= m) {
+            double eta;
+            if (op.phase == PH_P) eta = g.p_hartree ? (s_rE[p] + s_v1[p]) : s_rE[p];
+            else if (op.phase == PH_D) eta = s_v2[p];
+            else eta = s_v3[p];   // FP and FF
+            eta *= hdt * dj;
+            y = cmul_conj_phase(y, eta);
+          }
+          if (last && ch.post_s) {
+            double eta = s_sb[p] + pco[j] * s_v2[p];
+            eta *= hdt;
+            y = cmul_conj_phase(y, eta);
+          }
+          *reinterpret_cast<double2*>(ys + (size_t)j * AS_LD + 2 * p) = y;
+        }
+      }
+    }
+    __syncthreads();
+    double* t = xs; xs = ys; ys = t;
+  }
+  const double2* x2 = reinterpret_cast<const double2*>(xs);
+  if (xout)
+    for (int i = tid; i < n_l * AS_P; i += AS_WARPS * 32) {
+      const int l = i / AS_P, p = i - l * AS_P, r = r0 + p;
+      if (r < g.n_r) xout[((size_t)l * g.n_cols + col) * g.n_r + r] = x2[(size_t)l * (AS_LD / 2) + p];
+    }
+  if (do_den) {
+    // density multipoles as above, the groups' partials in the free copy of the tile
+    const int n_den = g.n_den > 0 ? g.n_den : 1;
+    const int n_sub = g.den_groups > 0 ? g.den_groups : AS_WARPS * 32 / AS_P;
+    const int sub = tid / AS_P, p = tid - sub * AS_P;
+    double d[N_DEN] = {0.0, 0.0, 0.0, 0.0};
+    if (sub < n_sub) {
+      if (g.den_groups > 0 || n_l < m + 7) {
+        density_partials<double2, AS_LD / 2>(n_den, m, n_l, x2, p, g.coef + (size_t)m * n_l, sub, n_sub, d, g.n_m * n_l);
+      } else {
+        const int per = (n_l - m + n_sub - 1) / n_sub, l0 = m + sub * per;
+        density_window<AS_LD / 2>(n_den, n_l, x2 + p, g.coef + (size_t)m * n_l, (size_t)g.n_m * n_l, l0, min(n_l, l0 + per), d);
+      }
+#pragma unroll
+      for (int L = 0; L < N_DEN; ++L) ys[(sub * N_DEN + L) * AS_P + p] = d[L];
+    }
+    __syncthreads();
+    for (int i = tid; i < n_den * AS_P; i += AS_WARPS * 32) {
+      const int L = i / AS_P, pp = i - L * AS_P, rl = r0 + pp;
+      double sum = 0.0;
+      for (int w = 0; w < n_sub; ++w) sum += ys[(w * N_DEN + L) * AS_P + pp];
+      if (rl < g.n_r) g.dens[((size_t)col * N_DEN + L) * g.n_r + rl] = sum;
+    }
+  }
+}
+
 static int g_angular_sms = 0;
 static constexpr int ANGULAR_POINTS[] = {4, 8, 16, 24, 32, 40};
 
@@ -318,8 +491,17 @@ size_t angular_smem_fp64(int n_l) {
   return most;
 }
 
+static size_t angular_small_smem(int n_l) { return 2 * (size_t)angular_rows(n_l) * AS_LD * sizeof(double); }
+
 // Radii per block: the least rounds over the SMs x (radii + the time of a block that does not depend
-// on them, about that of 12 radii).
+// on them, about that of 12 radii).  0: the four-warp blocks, by the same measure: four of them share an SM
+// (three above 88 channels), and a round of 148 x 4 takes as long as 62 of those units (80 below 30
+// channels).  They are the faster ones from about 2.5 tiles of 16 radii per SM on, where the last round is
+// not nearly empty; eight-warp form -> this one, both halves: the five products of the coupling chain at
+// N_r 253, N_l 49, 24 columns 97 -> 76 us, 575/70/120 1332 -> 927, 425/35/18 87 -> 64; the theta form at
+// 225/30/78 62 -> 46.  Few tiles: 253/49/3 28 against 54 us, 600/97/9 66 against 82.  From 105 channels on
+// two blocks fit an SM or fewer and the eight-warp form is the better one (300/220/9 128 against 278 us), at
+// 9 channels too (the blocks are all set-up).
 static int angular_points(const GroupArgs& g) {
   int best = 4;
   long best_cost = -1;
@@ -331,6 +513,10 @@ static int angular_points(const GroupArgs& g) {
       best_cost = cost;
       best = p;
     }
+  }
+  if (g.n_l >= 17 && g.n_l <= 104) {
+    const long tiles = (long)g.n_cols * ((g.n_r + AS_P - 1) / AS_P), resident = (long)g_angular_sms * (g.n_l <= 88 ? 4 : 3);
+    if ((tiles + resident - 1) / resident * (g.n_l < 30 ? 80 : 62) < best_cost) return 0;
   }
   return best;
 }
@@ -344,6 +530,10 @@ static void launch_angular_tile(const GroupArgs& g, int half, const double2* xin
 template <int R>
 static void launch_angular_rows(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
   switch (angular_points(g)) {
+    case 0:
+      k_angular_fp64_small<<<g.n_cols * ((g.n_r + AS_P - 1) / AS_P), AS_WARPS * 32, angular_small_smem(g.n_l), s>>>(g, half, xin, xout,
+                                                                                                                 do_den);
+      break;
     case 4: launch_angular_tile<1, 1, R>(g, half, xin, xout, do_den, s); break;
     case 8: launch_angular_tile<1, 2, R>(g, half, xin, xout, do_den, s); break;
     case 16: launch_angular_tile<2, 2, R>(g, half, xin, xout, do_den, s); break;
@@ -1111,6 +1301,8 @@ cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max) {
     case 2: e = configure_angular_rows<2>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
     case 1: e = configure_angular_rows<1>(optin); if (e != cudaSuccess) return e;
   }
+  e = set_max_dynamic_smem((const void*)k_angular_fp64_small, optin);
+  if (e != cudaSuccess) return e;
   e = configure_radial_fp64();
   if (e != cudaSuccess) return e;
   e = configure_theta(optin);

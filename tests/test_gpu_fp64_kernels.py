@@ -158,3 +158,11 @@ def test_fp64_angular_tiles_at_their_edges(n_r, n_l, angular):
         assert st == 0, msg
         assert rel_err(x, ref["x"]) < 1e-10
         assert rel_err(pot["v"], ref["v"][:4]) < 1e-10
+
+
+@pytest.mark.parametrize("n_r,n_l,angular", [(90, 17, "reference"), (90, 24, "theta"), (50, 31, "reference"), (51, 88, "theta"),
+                                             (49, 89, "reference"), (50, 104, "reference")])
+def test_fp64_angular_tiles_of_many_columns(n_r, n_l, angular):
+    """Sizes at which 90 columns take the four-warp blocks of 16 radii (one column the larger ones): odd
+    numbers of 8-channel tiles, part-full radii, two, three and four blocks an SM."""
+    test_fp64_angular_tiles_at_their_edges(n_r, n_l, angular)
