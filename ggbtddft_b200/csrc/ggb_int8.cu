@@ -569,25 +569,6 @@ template <int V>
 struct I8c {
   static constexpr int value = V;
 };
-// end of the round that starts at tile i
-template <int K_ATOMS>
-__device__ __forceinline__ int a8_round_end(int one_round, int i) {
-  return K_ATOMS == 2 && i > 0 && one_round ? 4 : i + 1;
-}
-// slice plane pa of tiles [i0, i1) into a stage, one after the other
-template <int K_ATOMS>
-__device__ __forceinline__ void a8_load_round(StGeom geo, const int8_t* mat, int i0, int i1, int pa, uint8_t* stage, uint64_t* bar) {
-  uint32_t bytes = 0;
-  for (int i = i0; i < i1; ++i) bytes += geo.rows(i / K_ATOMS) * geo.pitch(i % K_ATOMS);
-  mbar_expect_tx(bar, bytes);
-  for (int i = i0; i < i1; ++i) {
-    const int mt = i / K_ATOMS, ka = i % K_ATOMS;
-    const uint32_t plane = geo.rows(mt) * geo.pitch(ka);
-    bulk_g2s(stage, mat + geo.tile(mt, ka) + pa * plane, plane, bar);
-    stage += plane;
-  }
-}
-
 // One CTA per (orbital column, NP radii): NP = 32 for N_l <= 128 (one M tile of 128 channels),
 // NP = 16 for N_l <= 256 (two M tiles), so that every CTA holds 256 TMEM columns and two CTAs share
 // an SM (one CTA's epilogue overlaps the other's products and loads).
@@ -710,10 +691,13 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
   // the first S^T slice planes are on their way while the operand is filled
   const int mat0 = ch.ops[o0].mat + (step_raw & (t.n_var - 1)) * t.n_mats;   // this step's variant
   if (threadIdx.x == 0) {
+    const uint32_t plane = (uint32_t)(t.geo.rows(0) * t.geo.pitch(0));
+    const int8_t* src = t.St + ((size_t)mat0 * g.n_m + m) * t.geo.bytes();
 #pragma unroll
-    for (int pa = 0; pa < I8_SLICES; ++pa)
-      a8_load_round<K_ATOMS>(t.geo, t.St + ((size_t)mat0 * g.n_m + m) * t.geo.bytes(), 0, a8_round_end<K_ATOMS>(t.one_round, 0), pa,
-                             sst + pa * A8_A_TILE, &full_bar[pa]);
+    for (int pa = 0; pa < I8_SLICES; ++pa) {
+      mbar_expect_tx(&full_bar[pa], plane);
+      bulk_g2s(sst + pa * A8_A_TILE, src + pa * plane, plane, &full_bar[pa]);
+    }
   }
 
   // operand: phases of the tile in registers (second half: the l-diagonal S phase; basis reuse: the
@@ -792,21 +776,49 @@ k_angular_i8(GroupArgs g, Ang8Args t, const double2* xin, double2* xout) {
     if (lane == 0) {
       int it = 0;
       bool ok = true;
+      // per tile: bytes of a slice plane and offset of the first one.  Worked out here and the rounds unrolled:
+      // this thread shares its SM sub-partition with busy epilogue warps, so what it does per refill is
+      // exposed between the rounds (as a loop over tiles with its index arithmetic: the halves of the coupling
+      // chain at N_r 300, 30 columns 151 + 158 us at N_l 161 and 186 + 199 at 220; so: 131 + 140 and 158 + 171)
+      uint32_t plane[K_ATOMS * K_ATOMS], off[K_ATOMS * K_ATOMS];
+#pragma unroll
+      for (int i = 0; i < K_ATOMS * K_ATOMS; ++i) {
+        plane[i] = (uint32_t)(t.geo.rows(i / K_ATOMS) * t.geo.pitch(i % K_ATOMS));
+        off[i] = (uint32_t)t.geo.tile(i / K_ATOMS, i % K_ATOMS);
+      }
+      const size_t mat_bytes = t.geo.bytes(), m_stride = mat_bytes * g.n_m;
+      const int8_t* mats = t.St + (size_t)((step_raw & (t.n_var - 1)) * t.n_mats) * m_stride + m * mat_bytes;   // this step's variant
       for (int o = o0; o < n_ops && ok; ++o) {
-        const int mat = ch.ops[o].mat + (step_raw & (t.n_var - 1)) * t.n_mats;   // this step's variant
-        const int8_t* src = t.St + ((size_t)mat * g.n_m + m) * t.geo.bytes();
+        const int8_t* src = mats + ch.ops[o].mat * m_stride;
         // stage pa takes slice plane pa; the ring turns once per round
-        for (int i0 = 0, i1; i0 < K_ATOMS * K_ATOMS && ok; i0 = i1) {
-          i1 = a8_round_end<K_ATOMS>(t.one_round, i0);
+        auto load_round = [&](auto I0, auto I1) -> bool {
+          uint32_t bytes = 0;
+#pragma unroll
+          for (int i = decltype(I0)::value; i < decltype(I1)::value; ++i) bytes += plane[i];
           const int round = it / I8_SLICES;
+          if (round == 0) {                    // issued before the fill
+            it += I8_SLICES;
+            return true;
+          }
 #pragma unroll
           for (int pa = 0; pa < I8_SLICES; ++pa, ++it) {
-            if (round == 0) continue;          // issued before the fill
-            if (!mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) {
-              ok = false;
-              break;
+            if (!mbar_wait(&empty_bar[pa], (round & 1) ^ 1, abort_p)) return false;
+            mbar_expect_tx(&full_bar[pa], bytes);
+            uint8_t* stage = sst + pa * A8_A_TILE;
+#pragma unroll
+            for (int i = decltype(I0)::value; i < decltype(I1)::value; ++i) {
+              bulk_g2s(stage, src + off[i] + pa * plane[i], plane[i], &full_bar[pa]);
+              stage += plane[i];
             }
-            a8_load_round<K_ATOMS>(t.geo, src, i0, i1, pa, sst + pa * A8_A_TILE, &full_bar[pa]);
+          }
+          return true;
+        };
+        ok = load_round(I8c<0>(), I8c<1>());
+        if constexpr (K_ATOMS == 2) {
+          if (t.one_round) {
+            ok = ok && load_round(I8c<1>(), I8c<4>());
+          } else {
+            ok = ok && load_round(I8c<1>(), I8c<2>()) && load_round(I8c<2>(), I8c<3>()) && load_round(I8c<3>(), I8c<4>());
           }
         }
       }
