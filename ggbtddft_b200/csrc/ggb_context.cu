@@ -402,7 +402,8 @@ static int prepare(ggb_ctx* ctx) {
     int rc;
     if ((rc = dalloc(ctx, &g.mats_d, mats.size()))) return rc;
     CK(cudaMemcpy(g.mats_d, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
-    if (ctx->dims.precision != GGB_SPLIT_BF16) {
+    // (the int8 form's own chain takes S^T slices; its initial density runs an empty chain)
+    if (ctx->dims.precision == GGB_FP64 || (ctx->dims.precision == GGB_SPLIT_INT8 && g.mixed.angular_fp64)) {
       // FP64 MMA fragments: lane (gid, q) of row tile rt holds S[l][8 rt + gid] at l = 8 kp + 4 e + q,
       // e = 0, 1, of k-step pair kp; rows l < m and beyond N_l are zero
       const int n8 = (n_l + 7) / 8;
