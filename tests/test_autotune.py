@@ -55,3 +55,17 @@ def test_a_corrupt_cache_is_ignored(tmp_path):
     p = tmp_path / "tune.json"
     p.write_text("{not json")
     assert AT.load_cache(str(p)) == {}
+
+
+def test_tunings_of_the_kernel_before_the_staged_operands_are_not_reused(tmp_path):
+    """The radial kernel whose stages were tensor-copy boxes reported version 0.2: what a user's cache holds
+    from it does not override the shipped tunings, which carry the present version."""
+    run = SimpleNamespace(n_r=600, n_l=97, n_orb=9)
+    old = AT.cache_key(600, 96, 90, "NVIDIA B200", "ggbtddft-b200 0.2 (sm_100a)")
+    path = str(tmp_path / "tune.json")
+    AT.save_cache(path, {old: dict(bn=16, stages=3, ms={})})
+    shipped = AT.load_cache(AT.PACKAGED_CACHE)
+    assert all(f"|{AT.library_version()}|" in k for k in shipped)
+    want = shipped[AT.cache_key(600, 96, 90, "NVIDIA B200")]
+    got = AT.tuning_for([run] * 10, [list(range(10))], cache_file=path, device_name="NVIDIA B200", timer=None)
+    assert got == {0: (want["bn"], want["stages"])} != {0: (16, 3)}
