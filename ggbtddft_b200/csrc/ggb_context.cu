@@ -55,6 +55,7 @@ struct GroupHost {
   int* step_d = nullptr;
   double* fin_scr_d = nullptr;
   bool needs_init = true;
+  bool xc_stale = false;         // another grid was set under a density that no step recomputes
   GroupArgs args{};
   ThetaArgs theta_args{};        // theta form with n_har > 4 (ggb_theta.cu)
   cudaStream_t branch = nullptr; // its second branch of a step, forked from and joined to the group's stream
@@ -569,6 +570,7 @@ static int launch_init(ggb_ctx* ctx, GroupHost& g, cudaStream_t s) {
   if (a.theta_tab) launch_theta_potentials(a, g.theta_args, g.x_d, s);
   CK(cudaGetLastError());
   g.needs_init = false;
+  g.xc_stale = false;
   return GGB_OK;
 }
 
@@ -689,6 +691,7 @@ int ggb_set_grid(ggb_ctx* ctx, int group, const double* r, const double* drdx, c
   CK(cudaMemcpy(g.drdx_d, drdx, n_r * sizeof(double), cudaMemcpyDefault));
   CK(cudaMemcpy(g.P_d, P, n_r * sizeof(double), cudaMemcpyDefault));
   g.grid_set = true;
+  g.xc_stale = ctx->prepared && g.args.n_den == 0;
   return GGB_OK;
 }
 
@@ -805,9 +808,15 @@ int ggb_step(ggb_ctx* ctx, int n_steps, void* stream) {
   if (!was_prepared && ctx->dims.precision == GGB_SPLIT_BF16)
     for (GroupHost& g : ctx->groups)
       if ((rc = mixed_load_orbitals(g.mixed, g.args, g.x_d))) return fail(ctx, rc, "orbital conversion failed");
-  for (GroupHost& g : ctx->groups)
-    if (g.needs_init)
+  for (GroupHost& g : ctx->groups) {
+    if (g.needs_init) {
       if ((rc = launch_init(ctx, g, s))) return rc;
+    } else if (g.xc_stale && n_steps > 0) {
+      launch_finalize(g.args, obs_source(ctx, g), 3, s);
+      CK(cudaGetLastError());
+      g.xc_stale = false;
+    }
+  }
   if (!ctx->graph_exec) {
     // capture once, on the first call, so that later calls only replay
     for (const GroupHost& g : ctx->groups)

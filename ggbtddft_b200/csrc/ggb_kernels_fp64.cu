@@ -1062,15 +1062,15 @@ __device__ __forceinline__ void observe_row(const GroupArgs& g, const double2* x
 }
 
 // exchange blocks per run: one radius per thread; without Hartree the density is the frozen one, and
-// the potential stays what mode 0 wrote
+// the potential stays what mode 0 wrote, until another grid is set (mode 3)
 __host__ __device__ inline int fin_xc_blocks(const GroupArgs& g, int mode) {
-  return (g.n_den > 0 || mode == 0) ? (g.n_r + FIN_THREADS - 1) / FIN_THREADS : 0;
+  return (g.n_den > 0 || mode == 0 || mode == 3) ? (g.n_r + FIN_THREADS - 1) / FIN_THREADS : 0;
 }
 
 // Blocks: for each run of the group, n_den Hartree blocks (L = 0..n_den-1), the exchange blocks and
 // g.fin_ob observables blocks.  mode 0 = initial potentials (no observables,
 // no step increment), mode 1 = end of step, mode 2 = end of step without the step increment and the
-// watchdog checks (the per-phase timing).
+// watchdog checks (the per-phase timing), mode 3 = the exchange potential alone (without Hartree).
 //
 // Observables: one warp per row (l, orbital) of the run.  ROWS (the FP64 angular kernel): from the
 // orbitals, straight from L2 where those of a run still are (the angular kernel's tiles summed them
@@ -1110,7 +1110,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize(GroupArgs g, const dou
 
   if (obs_block && mode != 0 && step >= run.n_t) {
     if (mode == 1 && ob == 0 && tid == 0) atomicOr(g.status, ST_STEP_OVERFLOW);
-  } else if (obs_block) {
+  } else if (obs_block && mode != 3) {
     const int n_orb = run.n_orb;
     double2* scr = reinterpret_cast<double2*>(g.fin_scr);     // [col][N_l + 1][5]; row N_l: the norm
     const int rows = n_l * n_orb + (ROWS ? 0 : n_orb);
