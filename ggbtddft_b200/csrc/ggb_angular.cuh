@@ -1,6 +1,6 @@
-// Epilogue helpers shared by the angular kernels of both forms: density multipoles and
-// dipole/acceleration partial sums of one orbital column over one tile of radii.  The shared-memory
-// orbitals may be complex128 (FP64 form) or complex64 (split form); products and sums are FP64.
+// Epilogue helpers of the angular kernels: density multipoles of one orbital column over one tile of radii
+// (every form) and its dipole/acceleration partial sums (BF16 form).  The shared-memory orbitals may be
+// complex128 (FP64 and int8 forms) or complex64 (BF16 form); products and sums are FP64.
 #pragma once
 #include "ggb_internal.cuh"
 
@@ -71,7 +71,6 @@ __device__ double density_multipole(int L, int m, int n_l, const C* xs, int lane
   return d;
 }
 
-// compensated sum over aligned segments of `seg` lanes (seg = 32: the whole warp)
 // The seven coefficient rows of one m (CF_CU .. CF_F3 order), contiguous: rows[c * n_l + l].
 // Density multipoles L = 0 .. n_den-1 of one orbital at the radius of this lane: the same terms and
 // literal l ranges as density_multipole, but every l loop is strided over the n_warps warps, and
@@ -122,50 +121,27 @@ __device__ void density_partials(int n_den, int m, int n_l, const C* xs, int lan
   }
 }
 
-__device__ __forceinline__ dd warp_sum_dd(double v, int seg = 32) {
+__device__ __forceinline__ dd warp_sum_dd(double v) {
   dd a{v, 0.0};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    if (o < seg) {
-      const dd b{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-      a = dd_add(a, b);
-    }
-  }
+  for (int o = 16; o > 0; o >>= 1)
+    a = dd_add(a, dd{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
   return a;
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Dipole and acceleration partial sums for every l of one column over the radii r0 + lane held by
-// a lane group -- a warp, or half of one with seg = 16, the halves on different l
-// (dipoleMoment.cuh:19-43 / dipoleAcceleration.cuh:17-41 followed by cublasZdotc): one
-// partial per g.obs_seg consecutive radii (32 or 16), index (r0 + lane) / g.obs_seg.  Lanes from
-// n_valid on hold no radius.
-// COMPENSATED: double-double sums (the FP64 form, held to 1e-10 of the reference); otherwise plain
-// FP64 sums (the split forms, whose own error is far larger than FP64 summation error).
-// cu_row, cd_row: the c_u and c_d rows of this m when the caller has staged them (e.g. in shared
-// memory); by default they are read from the group's table.
-template <class C, int STRIDE = TR, bool COMPENSATED = true>
-__device__ void observables_tile(const GroupArgs& g, const C* xs, int col, int m, int r0, int lane,
-                                 int warp, int n_warps, double rr, double fr2, int n_valid = TR,
-                                 const double* cu_row = nullptr, const double* cd_row = nullptr) {
+// Dipole and acceleration partial sums for every l of one column over the 32 radii r0 + lane of a warp
+// (dipoleMoment.cuh:19-43 / dipoleAcceleration.cuh:17-41 followed by cublasZdotc), in double-double: one
+// partial per 32 consecutive radii (BF16 form; the FP64 form takes the sums from the orbitals, the int8 form
+// has its own).
+template <class C, int STRIDE = TR>
+__device__ void observables_tile(const GroupArgs& g, const C* xs, int col, int m, int r0, int lane, int warp, int n_warps,
+                                 double rr, double fr2) {
   const int n_l = g.n_l;
-  const int seg = g.obs_seg;
-  const bool lv = lane < n_valid;
-  const double* cu = cu_row ? cu_row : g.coef + ((size_t)CF_CU * g.n_m + m) * n_l;
-  const double* cd = cd_row ? cd_row : g.coef + ((size_t)CF_CD * g.n_m + m) * n_l;
-  // every lane runs the same number of iterations (the shuffles below span the whole warp, whose
-  // lane groups may hold different l)
-  const int iters = (n_l + n_warps - 1) / n_warps;
-  for (int it = 0; it < iters; ++it) {
-    const int l = warp + it * n_warps;
-    const bool lok = l < n_l;
+  const double* cu = g.coef + ((size_t)CF_CU * g.n_m + m) * n_l;
+  const double* cd = g.coef + ((size_t)CF_CD * g.n_m + m) * n_l;
+  for (int l = warp; l < n_l; l += n_warps) {
     double4 out = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (lok && l >= m && lv) {
+    if (l >= m) {
       const double2 xl = to_d2(xs[l * STRIDE + lane]);
       const double2 xu = (l + 1 < n_l) ? to_d2(xs[(l + 1) * STRIDE + lane]) : make_double2(0.0, 0.0);
       const double2 xd = (l >= 1) ? to_d2(xs[(l - 1) * STRIDE + lane]) : make_double2(0.0, 0.0);
@@ -187,28 +163,13 @@ __device__ void observables_tile(const GroupArgs& g, const C* xs, int col, int m
       out.z = xl.x * z2.x + xl.y * z2.y;
       out.w = xl.x * z2.y - xl.y * z2.x;
     }
-    // compensated (double-double) reduction over the tile's radii
-    dd sx, sy, sz, sw;
-    if (COMPENSATED) {
-      sx = warp_sum_dd(out.x, seg); sy = warp_sum_dd(out.y, seg);
-      sz = warp_sum_dd(out.z, seg); sw = warp_sum_dd(out.w, seg);
-    } else {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        if (o < seg) {
-          out.x += __shfl_xor_sync(0xffffffffu, out.x, o); out.y += __shfl_xor_sync(0xffffffffu, out.y, o);
-          out.z += __shfl_xor_sync(0xffffffffu, out.z, o); out.w += __shfl_xor_sync(0xffffffffu, out.w, o);
-        }
-      }
-      sx = dd{out.x, 0.0}; sy = dd{out.y, 0.0}; sz = dd{out.z, 0.0}; sw = dd{out.w, 0.0};
-    }
-    if (lok && lv && (lane & (seg - 1)) == 0) {
-      double4* o = g.obs + 2 * (((size_t)col * n_l + l) * g.n_tiles + (r0 + lane) / seg);
+    const dd sx = warp_sum_dd(out.x), sy = warp_sum_dd(out.y), sz = warp_sum_dd(out.z), sw = warp_sum_dd(out.w);
+    if (lane == 0) {
+      double4* o = g.obs + 2 * (((size_t)col * n_l + l) * g.n_tiles + r0 / TR);
       o[0] = make_double4(sx.hi, sy.hi, sz.hi, sw.hi);
       o[1] = make_double4(sx.lo, sy.lo, sz.lo, sw.lo);
     }
   }
 }
-
 
 }  // namespace ggb

@@ -130,10 +130,10 @@ __global__ void k_w_rowmax(const double2* __restrict__ W, int* __restrict__ wexp
 // 32-byte swizzle already applied (the two 16-byte halves of a row change places in rows 4 .. 7 of every
 // eight), so that a stage is one contiguous copy.  The last tiles are only as high as the matrix needs:
 // N_r rounded up to 8 rows of W (the product's further rows are what follows in the buffer, never
-// read from the accumulators), the orbital columns rounded up to 16 (the MMAs' N follows).  As a [rows][k] matrix a stage was a TMA box of 32-byte
-// rows, 1024 and more of them, which paced
-// the copies: 69 -> 53 us for one argon run (N_r 600, N_l 97: 302 MB of W, 5.7 TB/s), 176 -> 155 us for
-// ten, 990 -> 859 us for 21 at N_r 1000, N_l 161.
+// read from the accumulators), the orbital columns rounded up to 16 (the MMAs' N follows).  As a [rows][k]
+// matrix a stage was a TMA box of 32-byte rows, 1024 and more of them, which paced the copies: 69 -> 53 us for
+// one argon run (N_r 600, N_l 97: 283 MB of W, 5.3 TB/s), 176 -> 155 us for ten (123 with the trimmed tiles
+// and 32 columns a tile), 990 -> 859 us for 21 at N_r 1000, N_l 161.
 __host__ __device__ __forceinline__ uint32_t r8_row_off(int row, int k) {
   return (uint32_t)(row * 32 + ((((k >> 4) & 1) ^ ((row >> 2) & 1)) << 4) + (k & 15));
 }

@@ -21,7 +21,7 @@ namespace ggb {
 
 constexpr int TR = 32;            // radii per angular tile (one warp-width, coalesced along r)
 constexpr int ANG_WARPS = 8;      // warps per angular CTA
-constexpr int MAX_NL = 220;       // largest N_l: two [N_l][32] complex128 tiles fit in 227 KB of shared memory
+constexpr int MAX_NL = 220;       // largest N_l: the int8 fill's two rounds of l quads, a theta node per four threads of a block
 constexpr int MAX_NR = 8192;      // largest N_r: three [N_r] FP64 rows of the potentials kernel
 constexpr int FIN_OB = 148;        // observables blocks per run in k_finalize, at most (8 rows (l, orbital) each)
 constexpr int N_DEN = 4;          // density multipoles carried per column (L = 0..3)
@@ -87,8 +87,8 @@ struct GroupArgs {
   int per_l;
   double dt;
   double n_g_fac;   // N_g (N_g + 1) / 2
-  double norm_tol;
-  int obs_seg;      // radii per observables partial sum (32; 16 for the int8 form when N_l > 128)  // relative growth of an orbital norm above its initial value that raises ST_NORM_GROWTH
+  double norm_tol;  // relative growth of an orbital norm above its initial value that raises ST_NORM_GROWTH
+  int obs_seg;      // radii per observables partial sum (32; 16 for the int8 form when N_l > 128)
   int obs_parts;    // entries of g.obs per partial: 1, or 2 (high and low parts)
   const double* r;
   const double* drdx;

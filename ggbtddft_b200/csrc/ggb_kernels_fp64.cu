@@ -8,14 +8,16 @@
 //                  h_couplingFF/FP/D/P (couplingP.cuh:108-125, couplingD.cuh, couplingF.cuh) and
 //                  h_couplingS (couplingS.cuh:43-57).  The second half also produces the
 //                  density-multipole partial sums of the new orbitals
-//                  (hartreePotentialDensity.cuh:1-181).
+//                  (hartreePotentialDensity.cuh:1-181).  k_angular_fp64_small: the same for groups of
+//                  many tiles and up to 104 channels, in smaller blocks.
 //  k_radial_fp64   x_l <- A_l x_l for every l with A_l(a,b) = W[l][b][a]: the batched ZGEMM of
 //                  h_propagationH0 (h_timePropagation.cuh:1-30), out of place.  More than nine
-//                  columns: persistent, two CTAs per SM; a producer warp streams the W rows and x
+//                  columns, and large grids of one, two and six (radial_tiles): persistent, two CTAs
+//                  per SM; a producer warp streams the W rows and x
 //                  segments of each 16-wide k chunk into a 3-stage shared-memory ring with
 //                  cp.async.bulk (mbarrier transaction counts), so that ~200 KB per SM are in flight
 //                  whatever the occupancy; four consumer warps run the product on the FP64 tensor
-//                  cores.  Up to nine columns (one run): k_radial_fp64_rows.
+//                  cores.  Else, up to nine columns (one run): k_radial_fp64_rows.
 //  k_finalize      per run: observables of the step from the partials, density multipoles
 //                  (occupation-weighted sum over orbitals), Hartree potentials by compensated
 //                  prefix scans (h_calculateHartreePotential.cuh:1-136), LDA exchange
@@ -743,7 +745,8 @@ __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, boo
 
 // The first RF_KEEP bytes of W stay in L2 from step to step (normal priority), the rest streams
 // through it (evict first), so that W does not push itself out of L2 before it comes round again.
-// The helium step (166 MB of W) takes 156.9 us with none kept, 154.6 with 48 MB, 166.5 with 96 MB.
+// The helium step (166 MB of W) takes 70.2 us with none kept, 66.7 with 48 MB, 74.6 with 96 MB; one argon
+// run's (559 MB) 212.9, 205.8 and 219.3.
 constexpr size_t RF_KEEP = 48u << 20;
 
 template <int TC, int RF_WARPS, bool KEEP>

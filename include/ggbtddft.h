@@ -73,8 +73,7 @@ enum {
 /* A grid group: runs that share the radial grid, N_l and the radial propagators W_l. */
 typedef struct ggb_group_desc {
   int n_r;      /* radial points N_r (any value >= 2; no multiple-of-32 restriction)       */
-  int n_l;      /* angular momenta N_l = l_max + 1 (2 .. 220 in every form: two [N_l][32]
-                   complex128 tiles of the FP64 angular kernel fit in shared memory)           */
+  int n_l;      /* angular momenta N_l = l_max + 1 (2 .. 220 in every form)                    */
   int n_m;      /* number of azimuthal blocks N_m (m = 0 .. n_m-1)                          */
 } ggb_group_desc;
 
@@ -118,7 +117,8 @@ int ggb_set_radial_propagators(ggb_ctx* ctx, int group, const double* W);
 int ggb_set_angular(ggb_ctx* ctx, int group, int coupling, int m, const double* V, const double* D);
 
 /* Initial orbitals x[l][kso][r] (complex128), and l, m, occupation per orbital, frozen density
-   (h_initialiseTDKSOSet.cuh:19-107).  Resets the run's step counter and observables. */
+   (h_initialiseTDKSOSet.cuh:19-107).  Resets the run's step counter and observables.  Host arrays are
+   read after the work queued before the call on the legacy stream and the blocking ones. */
 int ggb_set_orbitals(ggb_ctx* ctx, int run, const double* x, const int* l, const int* m,
                      const int* occ, const double* rho_frozen);
 
