@@ -401,26 +401,23 @@ static int prepare(ggb_ctx* ctx) {
     build_chain(g, rev, 1, k + 1, c1, mats);
     c2.n_ops = 0;
     int rc;
-    if ((rc = dalloc(ctx, &g.mats_d, mats.size()))) return rc;
-    CK(cudaMemcpy(g.mats_d, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (ctx->dims.precision != GGB_FP64) {
+      if ((rc = dalloc(ctx, &g.mats_d, mats.size()))) return rc;
+      CK(cudaMemcpy(g.mats_d, mats.data(), mats.size() * sizeof(double), cudaMemcpyHostToDevice));
+    }
     // (the int8 form's own chain takes S^T slices; its initial density runs an empty chain)
     if (ctx->dims.precision == GGB_FP64 || (ctx->dims.precision == GGB_SPLIT_INT8 && g.mixed.angular_fp64)) {
       // FP64 MMA fragments: lane (gid, q) of row tile rt holds S[l][8 rt + gid] at l = 8 kp + 4 e + q,
-      // e = 0, 1, of k-step pair kp; rows l < m and beyond N_l are zero
+      // e = 0, 1, of k-step pair kp; rows l < m and beyond N_l are zero.  Filled row by row of S (element by
+      // element of the fragments, 0.7 ms of a context's first step at N_l 97, two m)
       const int n8 = (n_l + 7) / 8;
       std::vector<double> frag((size_t)n_mats * n_m * n8 * n8 * 64, 0.0);
-      size_t o = 0;
-      for (int mm = 0; mm < n_mats * n_m; ++mm) {
-        const double* S = mats.data() + (size_t)mm * n_l * ldS;
-        const int m = mm % n_m;
-        for (int rt = 0; rt < n8; ++rt)
-          for (int kp = 0; kp < n8; ++kp)
-            for (int lane = 0; lane < 32; ++lane)
-              for (int e = 0; e < 2; ++e, ++o) {
-                const int j = 8 * rt + lane / 4, l = 8 * kp + 4 * e + lane % 4;
-                if (j < n_l && l < n_l && l >= m) frag[o] = S[(size_t)l * ldS + j];
-              }
-      }
+      for (int mm = 0; mm < n_mats * n_m; ++mm)
+        for (int l = mm % n_m; l < n_l; ++l) {
+          const double* row = mats.data() + ((size_t)mm * n_l + l) * ldS;
+          double* f = frag.data() + ((size_t)mm * n8 * n8 + l / 8) * 64 + (l % 4) * 2 + (l / 4) % 2;
+          for (int j = 0; j < n_l; ++j) f[(size_t)(j / 8) * n8 * 64 + (j % 8) * 8] = row[j];
+        }
       if ((rc = dalloc(ctx, &g.frag_d, frag.size()))) return rc;
       CK(cudaMemcpy(g.frag_d, frag.data(), frag.size() * sizeof(double), cudaMemcpyHostToDevice));
     }

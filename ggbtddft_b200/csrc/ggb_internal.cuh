@@ -6,8 +6,10 @@
 //            d_x[l][kso*N_r + r] (main.cu:356-369) without the pointer-array indirection.
 //   W        radial propagators, FP64 form: double2 [N_l][N_r][N_r] = propagatorL%03d.bin.
 //   mats     angular chain matrices, [n_mats][N_m][N_l][ldS] doubles, stored so that the kernel's
-//            product is y[j] = sum_l S[l][j] x[l]  (S = A^T of the left multiplier A).
-//   frag     the same matrices as FP64 MMA fragments, [n_mats][N_m][row tile][k-step pair][lane][2].
+//            product is y[j] = sum_l S[l][j] x[l]  (S = A^T of the left multiplier A).  Split forms, which
+//            build their operands from them.
+//   frag     the same matrices as FP64 MMA fragments, [n_mats][N_m][row tile][k-step pair][lane][2].  FP64
+//            form, and the int8 form with FP64 angular products.
 //   dph      angular eigenvalues D[c][m][j], [4][N_m][ldS].
 //   coef     angular coefficient tables [COEF_N][N_m][N_l] (cu, cd, p, qu, qd, p3lm, f3lm).
 //   dens     density partials per column [n_cols][4][N_r] (not yet occupation weighted).
