@@ -480,6 +480,8 @@ static int prepare(ggb_ctx* ctx) {
     a.den_groups = ctx->dims.precision == GGB_SPLIT_INT8 ? 128 / g.obs_seg : 0;
     a.chain[0] = c0; a.chain[1] = c1;
     a.chain[2] = c2;
+    // (the int8 form's initial density runs on the FP64 angular kernel)
+    CK(configure_group_fp64(a, ctx->dims.precision == GGB_FP64, ctx->dims.precision != GGB_SPLIT_BF16, obs_source(ctx, g) != nullptr));
     if (ctx->dims.precision != GGB_FP64) {
       if ((rc = mixed_prepare(g.mixed, a, g.W_d, g.x_d, g.y_d, ctx->dims.precision, ctx->err))) return rc;
     }

@@ -1307,14 +1307,17 @@ int int8_prepare(MixedGroup& mg, GroupArgs& a, const double2* W_fp64, int n_mats
     case 32: I8_CK(set_max_dynamic_smem((const void*)k_radial_i8<32>, optin)); q.smem = r8_smem<32>(q.stages); break;
     default: I8_CK(set_max_dynamic_smem((const void*)k_radial_i8<64>, optin)); q.smem = r8_smem<64>(q.stages); break;
   }
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<32, false, false>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<32, true, false>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<16, false, false>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<16, true, false>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<32, false, true>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<32, true, true>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<16, false, true>, optin));
-  I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<16, true, true>, optin));
+  // the two halves that this group launches (a kernel's first mention in a process loads it)
+#define GGB_A8(NP, TH)                                                              \
+  do {                                                                              \
+    I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<NP, false, TH>, optin));   \
+    I8_CK(set_max_dynamic_smem((const void*)k_angular_i8<NP, true, TH>, optin));    \
+  } while (0)
+  if (!mg.angular_fp64) {
+    if (q.np == 32) { if (a.theta) GGB_A8(32, true); else GGB_A8(32, false); }
+    else { if (a.theta) GGB_A8(16, true); else GGB_A8(16, false); }
+  }
+#undef GGB_A8
   I8_CK(cudaDeviceSynchronize());
   return GGB_OK;
 }

@@ -181,6 +181,8 @@ void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin
 void launch_finalize(const GroupArgs& g, const double2* x, int mode, cudaStream_t s);
 size_t angular_smem_fp64(int n_l);
 cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max);
+// shared memory of the kernels that this group launches; obs_rows: k_finalize takes the orbitals
+cudaError_t configure_group_fp64(const GroupArgs& g, bool radial, bool angular, bool obs_rows);
 cudaError_t set_max_dynamic_smem(const void* fn, int optin);
 
 }  // namespace ggb

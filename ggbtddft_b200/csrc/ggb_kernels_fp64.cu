@@ -523,48 +523,43 @@ static int angular_points(const GroupArgs& g) {
   return best;
 }
 
+// The kernel that a group's half-steps run on.
+struct AngularLaunch {
+  void (*fn)(GroupArgs, int, const double2*, double2*, int);
+  int points, threads;
+  size_t smem;
+};
 template <int NT, int WN, int R>
-static void launch_angular_tile(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
+static AngularLaunch angular_tile(int n_l) {
   constexpr int P = 4 * NT * WN;
-  const int tiles = g.n_cols * ((g.n_r + P - 1) / P);
-  k_angular_fp64<NT, WN, R><<<tiles, AM_ROW_GROUPS * WN * 32, angular_smem_points(g.n_l, P), s>>>(g, half, xin, xout, do_den);
+  return {k_angular_fp64<NT, WN, R>, P, AM_ROW_GROUPS * WN * 32, angular_smem_points(n_l, P)};
 }
 template <int R>
-static void launch_angular_rows(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
-  switch (angular_points(g)) {
-    case 0:
-      k_angular_fp64_small<<<g.n_cols * ((g.n_r + AS_P - 1) / AS_P), AS_WARPS * 32, angular_small_smem(g.n_l), s>>>(g, half, xin, xout,
-                                                                                                                 do_den);
-      break;
-    case 4: launch_angular_tile<1, 1, R>(g, half, xin, xout, do_den, s); break;
-    case 8: launch_angular_tile<1, 2, R>(g, half, xin, xout, do_den, s); break;
-    case 16: launch_angular_tile<2, 2, R>(g, half, xin, xout, do_den, s); break;
-    case 24: launch_angular_tile<3, 2, R>(g, half, xin, xout, do_den, s); break;
-    case 32: if constexpr (R <= 3) launch_angular_tile<4, 2, R>(g, half, xin, xout, do_den, s); break;
-    default: if constexpr (R <= 2) launch_angular_tile<5, 2, R>(g, half, xin, xout, do_den, s); break;
+static AngularLaunch angular_launch_rows(int n_l, int points) {
+  switch (points) {
+    case 4: return angular_tile<1, 1, R>(n_l);
+    case 8: return angular_tile<1, 2, R>(n_l);
+    case 16: return angular_tile<2, 2, R>(n_l);
+    case 32: if constexpr (R <= 3) return angular_tile<4, 2, R>(n_l); break;
+    case 40: if constexpr (R <= 2) return angular_tile<5, 2, R>(n_l); break;
+    default: break;
+  }
+  return angular_tile<3, 2, R>(n_l);
+}
+static AngularLaunch angular_launch(const GroupArgs& g) {
+  const int points = angular_points(g);
+  if (points == 0) return {k_angular_fp64_small, AS_P, AS_WARPS * 32, angular_small_smem(g.n_l)};
+  switch (((g.n_l + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS) {
+    case 1: return angular_launch_rows<1>(g.n_l, points);
+    case 2: return angular_launch_rows<2>(g.n_l, points);
+    case 3: return angular_launch_rows<3>(g.n_l, points);
+    default: return angular_launch_rows<4>(g.n_l, points);
   }
 }
 
 void launch_angular_fp64(const GroupArgs& g, int half, const double2* xin, double2* xout, int do_den, cudaStream_t s) {
-  switch (((g.n_l + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS) {
-    case 1: launch_angular_rows<1>(g, half, xin, xout, do_den, s); break;
-    case 2: launch_angular_rows<2>(g, half, xin, xout, do_den, s); break;
-    case 3: launch_angular_rows<3>(g, half, xin, xout, do_den, s); break;
-    default: launch_angular_rows<4>(g, half, xin, xout, do_den, s); break;
-  }
-}
-
-template <int R>
-static cudaError_t configure_angular_rows(int optin) {
-  cudaError_t e = set_max_dynamic_smem((const void*)k_angular_fp64<1, 1, R>, optin);
-  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<1, 2, R>, optin);
-  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<2, 2, R>, optin);
-  if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<3, 2, R>, optin);
-  if constexpr (R <= 3)
-    if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<4, 2, R>, optin);
-  if constexpr (R <= 2)
-    if (e == cudaSuccess) e = set_max_dynamic_smem((const void*)k_angular_fp64<5, 2, R>, optin);
-  return e;
+  const AngularLaunch k = angular_launch(g);
+  k.fn<<<g.n_cols * ((g.n_r + k.points - 1) / k.points), k.threads, k.smem, s>>>(g, half, xin, xout, do_den);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -903,21 +898,24 @@ static bool radial_tiles(int n_cols, int n_r, int n_l) {
   return (double)n_r * n_l >= fill * RAD_TI * resident * ((tiles + resident - 1) / resident);
 }
 
+struct RadialTile {
+  void (*fn)(int, int, int, const double2*, const double2*, double2*, unsigned*);
+  int cols;
+  size_t smem;
+};
 template <int TC>
-static void launch_radial_tiles(const GroupArgs& g, const double2* W, const double2* xin, double2* xout, cudaStream_t s) {
-  const int tiles = ((g.n_r + RAD_TI - 1) / RAD_TI) * ((g.n_cols + TC - 1) / TC) * g.n_l;
-  k_radial_fp64<TC><<<std::min(tiles, 2 * g_radial_sms), RAD_THREADS, radial_fp64_smem<TC>(), s>>>(g.n_r, g.n_cols, g.n_l, W, xin,
-                                                                                               xout, g.status);
+static RadialTile radial_tile() { return {k_radial_fp64<TC>, TC, radial_fp64_smem<TC>()}; }
+static RadialTile radial_tile_of(int n_cols) {
+  return n_cols == 1 ? radial_tile<1>() : n_cols == 2 ? radial_tile<2>() : n_cols <= 6 ? radial_tile<6>()
+       : n_cols <= 12 ? radial_tile<12>() : radial_tile<16>();
 }
 
 void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin, double2* xout, cudaStream_t s) {
   const int nc = g.n_cols;
   if (radial_tiles(nc, g.n_r, g.n_l)) {
-    if (nc == 1) launch_radial_tiles<1>(g, W, xin, xout, s);
-    else if (nc == 2) launch_radial_tiles<2>(g, W, xin, xout, s);
-    else if (nc <= 6) launch_radial_tiles<6>(g, W, xin, xout, s);
-    else if (nc <= 12) launch_radial_tiles<12>(g, W, xin, xout, s);
-    else launch_radial_tiles<16>(g, W, xin, xout, s);
+    const RadialTile k = radial_tile_of(nc);
+    const int tiles = ((g.n_r + RAD_TI - 1) / RAD_TI) * ((nc + k.cols - 1) / k.cols) * g.n_l;
+    k.fn<<<std::min(tiles, 2 * g_radial_sms), RAD_THREADS, k.smem, s>>>(g.n_r, nc, g.n_l, W, xin, xout, g.status);
     return;
   }
   const int blocks = g.n_l * ((g.n_r + 31) / 32);
@@ -936,25 +934,6 @@ void launch_radial_fp64(const GroupArgs& g, const double2* W, const double2* xin
     default: break;
   }
 #undef GGB_RF_CASE
-}
-
-template <int TC>
-static cudaError_t configure_radial_tiles() {
-  return cudaFuncSetAttribute((const void*)k_radial_fp64<TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)radial_fp64_smem<TC>());
-}
-
-static cudaError_t configure_radial_fp64() {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&g_radial_sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = configure_radial_tiles<1>();
-  if (e == cudaSuccess) e = configure_radial_tiles<2>();
-  if (e == cudaSuccess) e = configure_radial_tiles<6>();
-  if (e == cudaSuccess) e = configure_radial_tiles<12>();
-  if (e == cudaSuccess) e = configure_radial_tiles<16>();
-  return e;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1287,32 +1266,31 @@ cudaError_t set_max_dynamic_smem(const void* fn, int optin) {
 }
 
 cudaError_t configure_kernels_fp64(int n_l_max, int n_r_max) {
-  // The attribute is global per function: set it to the device's opt-in maximum once, so that
-  // contexts of different sizes can coexist.  Callers check their own sizes against it.
-  int dev = 0, optin = 0;
+  int dev = 0, optin = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   if (angular_smem_fp64(n_l_max) > (size_t)optin || 3 * (size_t)n_r_max * sizeof(double) > (size_t)optin)
     return cudaErrorInvalidValue;
-  e = cudaDeviceGetAttribute(&g_angular_sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  switch (((n_l_max + 7) / 8 + AM_ROW_GROUPS - 1) / AM_ROW_GROUPS) {   // groups of fewer row tiles too
-    default: e = configure_angular_rows<4>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
-    case 3: e = configure_angular_rows<3>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
-    case 2: e = configure_angular_rows<2>(optin); if (e != cudaSuccess) return e; [[fallthrough]];
-    case 1: e = configure_angular_rows<1>(optin); if (e != cudaSuccess) return e;
-  }
-  e = set_max_dynamic_smem((const void*)k_angular_fp64_small, optin);
-  if (e != cudaSuccess) return e;
-  e = configure_radial_fp64();
-  if (e != cudaSuccess) return e;
-  e = configure_theta(optin);
-  if (e != cudaSuccess) return e;
-  e = set_max_dynamic_smem((const void*)k_finalize<true>, optin);
-  if (e != cudaSuccess) return e;
-  return set_max_dynamic_smem((const void*)k_finalize<false>, optin);
+  g_angular_sms = g_radial_sms = sms;
+  return cudaSuccess;
+}
+
+// The attribute is global per function: set to the device's opt-in maximum, so that contexts of different
+// sizes can coexist.  Callers check their own sizes against it.  Only for the kernels that the group
+// launches: the first mention of a kernel in a process loads it (all of this file's forms: 3 ms of the first
+// context of 33 channels, more with more).
+cudaError_t configure_group_fp64(const GroupArgs& g, bool radial, bool angular, bool obs_rows) {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess && angular) e = set_max_dynamic_smem((const void*)angular_launch(g).fn, optin);
+  if (e == cudaSuccess && radial && radial_tiles(g.n_cols, g.n_r, g.n_l))
+    e = set_max_dynamic_smem((const void*)radial_tile_of(g.n_cols).fn, optin);
+  if (e == cudaSuccess && g.theta_tab) e = configure_theta(optin);
+  if (e == cudaSuccess) e = set_max_dynamic_smem(obs_rows ? (const void*)k_finalize<true> : (const void*)k_finalize<false>, optin);
+  return e;
 }
 
 }  // namespace ggb

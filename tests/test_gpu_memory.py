@@ -55,3 +55,21 @@ def test_fp64_form_holds_the_chain_matrices_in_fragment_order_only():
     held()                            # module loading and the like
     fragments = 2 * 5 * n_m * 28 * 28 * 64 * 8
     assert held() < fragments + (16 << 20)
+
+
+def test_steps_at_radii_that_need_more_shared_memory_than_the_default():
+    """3500 radii: the potentials' rows take 56 KB; each form's kernels are configured by its own groups."""
+    rng = np.random.default_rng(1)
+    base = P.reference_like(40, 4, 2, "Ne3", r_mask=12.0, dt_as=10.0)
+    n_r = 3500
+    grid = I.make_grid(n_r, 0.5 * n_r, I.zeta_physical_to_ref(0.5, 0.5 * n_r))
+    w = np.zeros((4, n_r, n_r), np.complex128)
+    w[:, np.arange(n_r), np.arange(n_r)] = 1.0
+    x = rng.standard_normal((4, 3, n_r)) + 0j
+    x[0, base.m_active == 1] = 0
+    run = dataclasses.replace(base, grid=grid, W=w, x0=x / np.linalg.norm(x), rho_frozen=np.zeros(n_r), angular="theta")
+    for precision in ("fp64", "split_int8"):
+        tp = TimePropagation([run], precision=precision)
+        tp.step(2)
+        assert np.allclose(tp.observables(0)["norm"].sum(axis=0), 1.0, atol=1e-6) and tp.status()[0] == 0
+        tp.close()
